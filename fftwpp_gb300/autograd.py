@@ -126,6 +126,7 @@ class GraphedLossStep:
         if psi.dtype != op.dtype or omega.dtype != op.dtype:
             raise ValueError(f"psi and omega must be {op.dtype} tensors")
         loss_fn = loss_fn or _sum_sq
+        self.op = op        # the graph replays into its plans' staging
         self.psi = psi.detach().requires_grad_(True)
         self.omega = omega.detach().requires_grad_(True)
 
