@@ -151,6 +151,11 @@ def load():
     lib.fgb_fft_radices.argtypes = [sz, ctypes.c_int, ctypes.c_int,
                                     ctypes.c_int, P(ctypes.c_int),
                                     ctypes.c_int]
+    lib.fgb_fused_radices.restype = ctypes.c_int
+    lib.fgb_fused_radices.argtypes = [sz, ctypes.c_int, ctypes.c_int,
+                                      ctypes.c_int, ctypes.c_int,
+                                      P(ctypes.c_int), ctypes.c_int,
+                                      P(ctypes.c_int)]
     lib.fgb_index.restype = sz
     lib.fgb_index.argtypes = [ctypes.c_int, sz, sz, sz, sz, sz, sz, sz]
     lib.fgb_hermitian_symmetrize_x_device.restype = ctypes.c_int

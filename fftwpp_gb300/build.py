@@ -15,15 +15,20 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 BUILD = os.path.join(HERE, "_build")
 LIB = os.path.join(HERE, "lib_fftwpp.so")
-# (source, object, extra flags): kernels.cu is compiled once per precision so
-# the two halves of its template instantiations build in parallel.
-UNITS = [("kernels.cu", "kernels_f64.o", ["-DFGB_ONLY_DOUBLE"]),
-         ("kernels.cu", "kernels_f32.o", ["-DFGB_ONLY_FLOAT"]),
-         ("kernels.cu", "kernels_ff.o", ["-DFGB_ONLY_FF"]),
-         ("engine.cu", "engine.o", []),
-         ("batch.cu", "batch.o", []),
-         ("capi.cu", "capi.o", []),
-         ("noalloc.cu", "noalloc.o", [])]
+# (source, object, extra flags): kernels.cu is compiled once per precision and
+# kernel family so that its template instantiations build in parallel, the
+# longest first.
+UNITS = ([("kernels.cu", f"kernels_{t}_{part}.o",
+           [f"-DFGB_T={t}", f"-DFGB_PART={k}"])
+          for t in ("ff", "float", "double")
+          for k, part in ((2, "herm"), (1, "rows"), (4, "batch"),
+                          (6, "real"), (3, "outer"))
+          if (t, part) != ("ff", "batch")] +
+         [("kernels.cu", "kernels_misc.o", ["-DFGB_T=double", "-DFGB_PART=5"]),
+          ("engine.cu", "engine.o", []),
+          ("batch.cu", "batch.o", []),
+          ("capi.cu", "capi.o", []),
+          ("noalloc.cu", "noalloc.o", [])])
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC",
          "-I", os.path.join(os.path.dirname(HERE), "include")]

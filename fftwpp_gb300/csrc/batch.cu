@@ -29,11 +29,23 @@ static const int THREADS=256;
 
 static size_t elemBytes(int prec) {return prec == PREC_F64 ? 16 : 8;}
 
-static size_t rowNeedB(int prec, long L, long m, int A, int B, int rpc=1,
-                       int direct=0)
+static size_t rowNeedB(int prec, long L, long m, int A, int B)
 {
-  return prec == PREC_F64 ? rowSmem<double>(L,m,A,B,rpc,direct) :
-    rowSmem<float>(L,m,A,B,rpc,direct);
+  return prec == PREC_F64 ? rowSmem<double>(L,m,A,B) :
+    rowSmem<float>(L,m,A,B);
+}
+
+FFTPlanDev fftPlanPublic(long n, int prec, bool oddFirst);   // engine.cu
+FusedFFT fusedRowPlan(long n, int prec, int A, bool herm, bool half,
+                      int nteam, int maxR);
+void fusedRowTables(FusedFFT& p, int prec);
+
+// Shared memory of nteam fused rows of length m at a time.
+static size_t fusedNeedB(int prec, long m, int A, bool half, int nteam)
+{
+  const FusedFFT p=fusedRowPlan(m,prec,A,false,half,nteam,8);
+  return prec == PREC_F64 ? fusedRowSmem<double>(p.n,p.lg,A,nteam) :
+    fusedRowSmem<float>(p.n,p.lg,A,nteam);
 }
 
 static size_t outerNeedB(int prec, long L, long m, int tile)
@@ -46,8 +58,6 @@ static size_t outerNeedB(int prec, long L, long m, int tile)
 }
 
 static double fftCostB(long m) {return m*std::log2((double) std::max(m,2L));}
-
-FFTPlanDev fftPlanPublic(long n, int prec, bool oddFirst);   // engine.cu
 
 // Candidate plans of one problem, cheapest (by the cost model) first.
 // choice > 0: short problem with residue block m = choice;
@@ -321,14 +331,21 @@ void BatchConv::build()
       R.cshift=kind == KIND_CENTERED ? (int) (L/2) : 0;
       R.A=A; R.B=B; R.mult=mult; R.realIO=0; R.rpc=1;
       R.scale=(T) (1.0/(double) (m*q));
-      R.fp=fftPlanPublic(m,prec,prec != PREC_F64);   // in-place rows in FP32
-      R.direct=0;
+      R.direct=q == 1 && L <= m;
+      R.nteam=1;
+      if(R.direct) {
+        R.fz=fusedRowPlan(m,prec,A,false,R.cshift == 0 && 2*L <= m,1,8);
+        fusedRowTables(R.fz,prec);
+        smem=std::max(smem,fusedNeedB(prec,m,A,R.fz.half,1));
+      } else {
+        R.fp=fftPlanPublic(m,prec,prec != PREC_F64); // in-place rows in FP32
+        smem=std::max(smem,rowNeedB(prec,L,m,A,B));
+      }
       R.twN=(const Tw *) twiddles(m*q,prec);
       R.rowStride=L; R.nrows=1;
       for(int a=0; a < A; ++a) R.in[a]=(const cplx<T> *) (offsets[i]*e);
       for(int b=0; b < B; ++b) R.out[b]=(cplx<T> *) (offsets[i]*e);
       P.rel=1|2;
-      smem=std::max(smem,rowNeedB(prec,L,m,A,B));
       small.push_back({q*fftCostB(m)*(A+B),i});
       ++nsmall;
     } else {
@@ -363,19 +380,21 @@ void BatchConv::build()
       // The rows hold one residue of one fold: the direct row variant
       // (no staging, in-place transforms).
       int rpc=1;
-      while(rpc < 8 && rpc < qc &&
-            rowNeedB(prec,m,m,A,B,rpc+1,1) <= budget) ++rpc;
+      while(2*rpc <= 8 && 2*rpc <= qc &&
+            fusedNeedB(prec,m,A,false,2*rpc) <= budget) rpc *= 2;
       RowPlan<T>& R=P.row;
       R.L=(int) m; R.m=(int) m; R.q=1; R.N=(int) m; R.cshift=0;
       R.A=A; R.B=B; R.mult=mult; R.realIO=0; R.rpc=rpc; R.scale=(T) 1;
-      R.fp=fftPlanPublic(m,prec,true);
       R.direct=1;
+      R.nteam=rpc;
+      R.fz=fusedRowPlan(m,prec,A,false,false,rpc,8);
+      fusedRowTables(R.fz,prec);
       R.twN=(const Tw *) twiddles(m,prec);
       R.rowStride=m; R.nrows=qc;
       P.rel=4|8;
       P.nfwd=(int) (ceilquotient(m,tile)*A);
       P.nrows=(int) ceilquotient(qc,rpc);   // row tasks the backward waits for
-      smem=std::max(smem,rowNeedB(prec,m,m,A,B,rpc,1));
+      smem=std::max(smem,fusedNeedB(prec,m,A,false,rpc));
       smem=std::max(smem,outerNeedB(prec,pc,qc,tile));
       lng.push_back({(double) N*std::log2((double) N),i});
       ++nlong;

@@ -1101,6 +1101,24 @@ int fgb_fft_radices(size_t n, int precision, int inplace, int wide,
   return nst;
 }
 
+int fgb_fused_radices(size_t n, int precision, int inputs, int hermitian,
+                      int half, int *radix, int max, int *padding)
+{
+  int r[FGB_FUSED_STAGES+8];
+  const int nst=inputs < 1 || inputs > FGB_MAXA ? -1 :
+    fusedRadices((long) n,precision,inputs,hermitian != 0,half != 0,
+                 precision == PREC_F32 ? 16 : 8,r);
+  if(nst < 0) {
+    setLastError("transform length "+std::to_string(n)+" has no radix plan");
+    return -1;
+  }
+  for(int s=0; s < nst && s < max; ++s) radix[s]=r[s];
+  if(padding)
+    for(int level=0; level < 2; ++level)
+      padding[level]=fusedPadding(r,nst,level);
+  return nst;
+}
+
 // Transformed index (fftBase::index, convolve.h:297-326; fftPadReal::index,
 // convolve.h:956-979).  D0 = n mod D (or D), the remainder block of the
 // residue loop (convolve.cc:701-703); overwrite is not modelled.

@@ -109,27 +109,17 @@ cudaError_t devAlloc(void **p, size_t bytes)
 // ---------------------------------------------------------------------------
 // Twiddle tables.
 
-const void *twiddles(long n, int prec)
+// exp(2 pi i t/n), t < n, from the exact rational angle t/n, reduced to the
+// first octant so that the long double evaluation stays accurate.
+static void unitRoots(long n, std::vector<double>& c, std::vector<double>& s)
 {
-  if(prec == PREC_FF) prec=PREC_F32;        // the same hi+lo float4 table
-  static std::mutex mu;
-  static std::map<std::tuple<int,long,int>,void *> cache;
-  int dev=0;
-  cudaGetDevice(&dev);
-  std::lock_guard<std::mutex> lock(mu);
-  auto key=std::make_tuple(dev,n,prec);
-  auto it=cache.find(key);
-  if(it != cache.end()) return it->second;
-
-  // exp(2 pi i t/n) from the exact rational angle t/n, reduced to the
-  // first octant so that the long double evaluation stays accurate.
-  std::vector<double> c(n), s(n);
+  c.resize(n);
+  s.resize(n);
   const long double pi=3.141592653589793238462643383279502884L;
   for(long t=0; t < n; ++t) {
     // angle = 2 pi t/n; fold by symmetry into [0, pi/4].
-    long tt=t;
     long double sign_c=1, sign_s=1;
-    long u=tt;
+    long u=t;
     // Use 8t vs n comparisons with exact integer arithmetic.
     long double a;
     bool swap=false;
@@ -146,23 +136,51 @@ const void *twiddles(long n, int prec)
     c[t]=(double) (sign_c*cv);
     s[t]=(double) (sign_s*sv);
   }
+}
+
+// A device table of the roots c[e[k]] + i s[e[k]] in the form of prec
+// (double2, or float4 split into hi and lo), NULL if the allocation fails.
+static void *rootTable(const std::vector<double>& c,
+                       const std::vector<double>& s,
+                       const std::vector<long>& e, int prec)
+{
   void *d=NULL;
+  const size_t n=e.size();
   if(prec == PREC_F64) {
     std::vector<double2> h(n);
-    for(long t=0; t < n; ++t) h[t]=make_double2(c[t],s[t]);
+    for(size_t k=0; k < n; ++k) h[k]=make_double2(c[e[k]],s[e[k]]);
     if(devAlloc((void **) &d,n*sizeof(double2)) != cudaSuccess) return NULL;
     cudaMemcpy(d,h.data(),n*sizeof(double2),cudaMemcpyHostToDevice);
   } else {
     std::vector<float4> h(n);
-    for(long t=0; t < n; ++t) {
-      float hx=(float) c[t], hy=(float) s[t];
-      h[t]=make_float4(hx,hy,(float) (c[t]-(double) hx),
-                       (float) (s[t]-(double) hy));
+    for(size_t k=0; k < n; ++k) {
+      const double x=c[e[k]], y=s[e[k]];
+      float hx=(float) x, hy=(float) y;
+      h[k]=make_float4(hx,hy,(float) (x-(double) hx),(float) (y-(double) hy));
     }
     if(devAlloc((void **) &d,n*sizeof(float4)) != cudaSuccess) return NULL;
     cudaMemcpy(d,h.data(),n*sizeof(float4),cudaMemcpyHostToDevice);
   }
-  cache[key]=d;
+  return d;
+}
+
+const void *twiddles(long n, int prec)
+{
+  if(prec == PREC_FF) prec=PREC_F32;        // the same hi+lo float4 table
+  static std::mutex mu;
+  static std::map<std::tuple<int,long,int>,void *> cache;
+  int dev=0;
+  cudaGetDevice(&dev);
+  std::lock_guard<std::mutex> lock(mu);
+  auto key=std::make_tuple(dev,n,prec);
+  auto it=cache.find(key);
+  if(it != cache.end()) return it->second;
+  std::vector<double> c, s;
+  unitRoots(n,c,s);
+  std::vector<long> e(n);
+  for(long t=0; t < n; ++t) e[t]=t;
+  void *d=rootTable(c,s,e,prec);
+  if(d) cache[key]=d;
   return d;
 }
 
@@ -241,9 +259,212 @@ FFTPlanDev fftPlanPublic(long n, int prec, bool oddFirst)
 }
 
 // ---------------------------------------------------------------------------
-// Planning.
+// Plans of the fused transforms (fft_fused.cuh).
 
 static const size_t SMEM_MAX=227*1024;
+
+int fusedRadices(long n, int prec, int A, bool herm, bool half, int maxR,
+                 int *radix)
+{
+  if(n < 1 || !smooth(n)) return -1;
+  int k2=0, odd[24], nodd=0;
+  long r=n;
+  while(r % 2 == 0) {++k2; r /= 2;}
+  for(int f : {7,5,3})
+    while(r % f == 0) {odd[nodd++]=f; r /= f;}
+  auto log2i=[](int v) {
+    int k=0;
+    while((2 << k) <= v) ++k;
+    return k;
+  };
+  // The middle stage holds R values of all A inputs in registers
+  // (fusedMiddle in rowkernels.cuh); float-float has none.
+  const int lim=prec == PREC_FF ? 20 : 20/A;
+  const int lgR=log2i(maxR), lgLast=std::max(1,std::min(lgR,log2i(std::max(2,lim))));
+  auto stages=[&](int k) {
+    return k == 0 ? 0 : k <= lgLast ? 1 : 1+(k-lgLast+lgR-1)/lgR;
+  };
+  // A radix 6 in place of a 3 where the factor 2 it takes saves a stage.
+  const bool six=prec == PREC_F32 && nodd > 0 && odd[nodd-1] == 3 && k2 >= 2 &&
+    stages(k2-1) < stages(k2);
+  if(six) --k2;
+  int nst=0, p2[16], np2=0;
+  // Split 2^k2: the last stage as much as it may take (its radix is the
+  // padding unit), the others evenly, larger first.
+  // A Hermitian first stage holds two butterflies in registers: radix 8 at
+  // most.
+  int k=k2;
+  bool front=false;                        // an even radix first
+  if(herm && prec == PREC_F32 && nodd == 0 && k > 3) {
+    p2[np2++]=3;
+    k -= 3;
+    front=true;
+  }
+  if(k > 0) {
+    const int s=stages(k), last=std::min(lgLast,k);
+    int rest=k-last;
+    for(int i=s-1; i > 0; --i) {
+      const int b=(rest+i-1)/i;
+      p2[np2++]=b;
+      rest -= b;
+    }
+    p2[np2++]=last;
+  }
+  if(half && nodd > 0 && np2 > 1) front=true;
+  int at=0;
+  if(front) radix[nst++]=1 << p2[at++];
+  for(int i=0; i < nodd; ++i)
+    if(!(six && i == nodd-1)) radix[nst++]=odd[i];
+  if(six) radix[nst++]=6;
+  while(at < np2) radix[nst++]=1 << p2[at++];
+  if(nst == 0) radix[nst++]=1;
+  if(np2 == 0 && radix[nst-1] > 3 && radix[nst-1] > lim) radix[nst++]=1;
+  if(nst == 1) {                      // at least two stages
+    const int R=radix[0], f=R == 4 || R == 8 ? 2 : R == 16 ? 4 : 1;
+    radix[0]=f;
+    radix[1]=R/f;
+    nst=2;
+  }
+  return nst <= FGB_FUSED_STAGES ? nst : -1;
+}
+
+// lg of the padding unit: the product of the last radices, at least four
+// (level 0; level k: k stages more), which makes every stage's offsets add
+// up (StageMap); 30 (no padding) where that is not a power of two.
+int fusedPadding(const int *radix, int nst, int level)
+{
+  int u=1, s=nst;
+  while(s > 0 && u < 4) u *= radix[--s];
+  while(s > 0 && level-- > 0) u *= radix[--s];
+  if(u & (u-1)) return 30;
+  int lg=0;
+  while((1 << lg) < u) ++lg;
+  return lg >= 2 ? lg : 30;
+}
+
+// The fused transform of length n whose kernel holds `columns` columns in
+// shared memory at once, padded as far as they fit.
+static FusedFFT fusedPlan(long n, int prec, int A, bool herm, bool half,
+                          int maxR, long columns)
+{
+  int rad[FGB_FUSED_STAGES+8];
+  FusedFFT p;
+  p.n=(int) n;
+  p.nst=fusedRadices(n,prec,A,herm,half,maxR,rad);
+  if(p.nst < 0)
+    throw std::runtime_error("transform length "+std::to_string(n)+
+                             " is not a product of 2, 3, 5 and 7");
+  for(int s=0; s < p.nst; ++s) p.radix[s]=(unsigned char) rad[s];
+  p.half=half && rad[0] % 2 == 0;
+  p.twb=p.twj=NULL;
+  p.pairs=NULL;
+  p.pos=NULL;
+  const size_t e=prec == PREC_F32 ? 8 : 16;
+  for(int level=0; level < 3; ++level) {
+    p.lg=level < 2 ? fusedPadding(rad,p.nst,level) : 30;
+    if(e*columns*fusedSpan((int) n,p.lg) <= SMEM_MAX) break;
+  }
+  return p;
+}
+
+// Twiddle tables of a fused plan (cached for the process): block twiddles
+// W_{R_0..R_s}^{r rev(b)} of the stages s >= 1, inverse twiddles W_{R m}^{r j}
+// of every stage, and the block pairs of real data.
+static void fusedTables(FusedFFT& p, int prec)
+{
+  if(prec == PREC_FF) prec=PREC_F32;
+  static std::mutex mu;
+  struct Tables {void *twb, *twj, *pairs, *pos;};
+  static std::map<std::tuple<int,int,std::string>,Tables> cache;
+  int dev=0;
+  cudaGetDevice(&dev);
+  const auto key=std::make_tuple(dev,prec,std::string((const char *) p.radix,
+                                                      p.nst));
+  std::lock_guard<std::mutex> lock(mu);
+  auto it=cache.find(key);
+  if(it == cache.end()) {
+    const long n=p.n;
+    std::vector<double> c, s;
+    unitRoots(n,c,s);
+    std::vector<long> eb, ej;
+    long nblk=p.radix[0];
+    std::vector<long> rev(p.radix[0]);
+    for(long b=0; b < nblk; ++b) rev[b]=b;
+    std::vector<int4> pairs;
+    for(int st=1; st < p.nst; ++st) {
+      const int R=p.radix[st];
+      for(int r=1; r < R; ++r)
+        for(long b=0; b < nblk; ++b)
+          eb.push_back(r*rev[b]*(n/(nblk*R)) % n);
+      if(st == p.nst-1) {
+        // Partner blocks of the last stage: rev(b) and nblk - rev(b).
+        std::vector<int> at(nblk);
+        for(long b=0; b < nblk; ++b) at[rev[b]]=(int) b;
+        pairs.push_back(make_int4(0,nblk % 2 ? -1 : at[nblk/2],0,0));
+        for(long b=1; b < nblk; ++b) {
+          const long k=rev[b];
+          if(2*k < nblk) pairs.push_back(make_int4((int) b,at[nblk-k],(int) k,
+                                                   0));
+        }
+      }
+      std::vector<long> next(nblk*R);
+      for(long b=0; b < nblk; ++b)
+        for(int r=0; r < R; ++r) next[b*R+r]=rev[b]+nblk*r;
+      rev.swap(next);
+      nblk *= R;
+    }
+    long m=1;
+    for(int st=p.nst-1; st >= 0; --st) {
+      const int R=p.radix[st];
+      for(int r=1; r < R; ++r)
+        for(long j=0; j < m; ++j) ej.push_back(r*j*(n/(R*m)) % n);
+      m *= R;
+    }
+    if(eb.empty()) eb.push_back(0);
+    if(ej.empty()) ej.push_back(0);
+    Tables t;
+    t.twb=rootTable(c,s,eb,prec);
+    t.twj=rootTable(c,s,ej,prec);
+    t.pairs=t.pos=NULL;
+    std::vector<int> pos(n);
+    for(long b=0; b < n; ++b) pos[rev[b]]=(int) b;
+    const size_t pb=pairs.size()*sizeof(int4), nb=n*sizeof(int);
+    if(!t.twb || !t.twj || devAlloc(&t.pairs,pb) != cudaSuccess ||
+       devAlloc(&t.pos,nb) != cudaSuccess) {
+      for(void *q : {t.twb,t.twj,t.pairs,t.pos}) if(q) cudaFree(q);
+      throw std::runtime_error("twiddle table allocation failed");
+    }
+    cudaMemcpy(t.pairs,pairs.data(),pb,cudaMemcpyHostToDevice);
+    cudaMemcpy(t.pos,pos.data(),nb,cudaMemcpyHostToDevice);
+    it=cache.emplace(key,t).first;
+  }
+  p.twb=it->second.twb;
+  p.twj=it->second.twj;
+  p.pairs=(const int4 *) it->second.pairs;
+  p.pos=(const int *) it->second.pos;
+}
+
+// Teams of a fused row launch: one per row where a team keeps at least eight
+// threads, and a divisor of the rows per CTA.
+int rowTeams(int rpc, int threads)
+{
+  int t=1;
+  while(rpc % (2*t) == 0 && threads/(2*t) >= 8) t *= 2;
+  return t;
+}
+
+static int widest(int prec) {return prec == PREC_F32 ? 16 : 8;}
+
+FusedFFT fusedRowPlan(long n, int prec, int A, bool herm, bool half,
+                      int nteam, int maxR)
+{
+  return fusedPlan(n,prec,A,herm,half,maxR,(long) nteam*A);
+}
+
+void fusedRowTables(FusedFFT& p, int prec) {fusedTables(p,prec);}
+
+// ---------------------------------------------------------------------------
+// Planning.
 
 // 16-byte complex elements (FP64 and float-float) or 8-byte ones (FP32).
 static bool wide(int prec) {return prec != PREC_F32;}
@@ -253,16 +474,92 @@ static bool wide(int prec) {return prec != PREC_F32;}
   (prec) == PREC_FF ? F<ff>(__VA_ARGS__) : F<float>(__VA_ARGS__))
 static size_t elem(int prec) {return wide(prec) ? 16 : 8;}
 
-// direct: a row plan with one residue and one fold (RowPlan::direct).
-static size_t rowNeed(int prec, long L, long m, int A, int B, int rpc=1,
-                      int direct=0)
+// Shared memory of a row kernel of several residues or folds.
+static size_t rowNeed(int prec, long L, long m, int A, int B, int rpc=1)
 {
-  return FGB_BY_PREC(prec,rowSmem,L,m,A,B,rpc,direct);
+  return FGB_BY_PREC(prec,rowSmem,L,m,A,B,rpc);
 }
 
-static size_t hermNeed(int prec, long H, long Nh, int A, int rpc=1)
+// Whether a complex row axis takes the fused rows.
+static bool rowDirect(const AxisPlan& a) {return a.q == 1 && a.stored <= a.m;}
+// Only the first half of the padded length holds data.
+static bool halfEmpty(const AxisPlan& a)
 {
-  return FGB_BY_PREC(prec,hermRowSmem,H,Nh,A,rpc);
+  return a.cshift == 0 && 2*a.stored <= a.m;
+}
+
+// Shared memory of the fused rows of length n, rpc per CTA.
+static size_t fusedRowNeed(int prec, long n, int A, bool herm, bool half,
+                           int rpc, int threads)
+{
+  const int teams=rowTeams(rpc,threads);
+  const FusedFFT p=fusedRowPlan(n,prec,A,herm,half,teams,widest(prec));
+  return FGB_BY_PREC(prec,fusedRowSmem,p.n,p.lg,A,teams);
+}
+
+// Shared memory of the innermost axis' row kernel, as planned.
+static size_t innerNeed(const ConvInfo& I, const AxisPlan& a, int rpc,
+                        int threads)
+{
+  if(I.longRow)
+    return fusedRowNeed(I.prec,I.rowM,I.A,false,false,rpc,threads);
+  if(a.kind == KIND_HERMITIAN)
+    return fusedRowNeed(I.prec,a.N/2,I.A,true,false,rpc,threads);
+  if(rowDirect(a))
+    return fusedRowNeed(I.prec,a.m,I.A,false,halfEmpty(a),rpc,threads);
+  return rowNeed(I.prec,a.stored,a.m,I.A,I.B,rpc);
+}
+
+// Whether an outer complex axis takes the fused kernels (one fold: data no
+// longer than a residue block), and its transform on a tile of columns.
+static bool outerFused(const AxisPlan& a)
+{
+  return a.kind != KIND_REAL && a.p == 1;
+}
+
+static FusedFFT outerFFT(const AxisPlan& a, int prec, int tile)
+{
+  return fusedPlan(a.m,prec,1,false,halfEmpty(a),widest(prec),tile);
+}
+
+// The real outer kernels' transform of half the padded length (two blocks of
+// a pair in registers, as two inputs).
+static FusedFFT realFFT(long N, long L, int prec, int tile)
+{
+  return fusedPlan(N/2,prec,2,false,2*L <= N,widest(prec),tile);
+}
+
+static size_t realNeed(const AxisPlan& a, int prec, int tile)
+{
+  const FusedFFT p=realFFT(a.N,a.L,prec,tile);
+  return FGB_BY_PREC(prec,fusedOuterSmem,a.L,p.n,p.lg,tile,1);
+}
+
+static size_t outerFwdNeed(const AxisPlan& a, int prec, int tile)
+{
+  if(a.kind == KIND_REAL) return realNeed(a,prec,tile);
+  if(outerFused(a)) {
+    const FusedFFT p=outerFFT(a,prec,tile);
+    return FGB_BY_PREC(prec,fusedOuterSmem,a.L,p.n,p.lg,tile,1);
+  }
+  return FGB_BY_PREC(prec,outerFwdSmem,a.L,a.m,tile);
+}
+
+static size_t outerBwdNeed(const AxisPlan& a, int prec, int tile)
+{
+  if(a.kind == KIND_REAL) return realNeed(a,prec,tile);
+  if(outerFused(a)) {
+    const FusedFFT p=outerFFT(a,prec,tile);
+    return FGB_BY_PREC(prec,fusedOuterSmem,a.L,p.n,p.lg,tile,(int) a.q);
+  }
+  return FGB_BY_PREC(prec,outerBwdSmem,a.L,a.m,tile,(int) a.q);
+}
+
+// Whether a Hermitian row goes to one CTA or to the long path; the line
+// stays where a ping-pong FP64 transform put it.
+static size_t hermNeed(int prec, long Nh, int A)
+{
+  return elem(prec)*(prec == PREC_F64 ? 2 : 1)*(size_t) padded((int) (Nh*A));
 }
 
 static size_t outerNeed(int prec, long L, long m, int tile)
@@ -288,14 +585,59 @@ static int pickRpc(long n, int A, long nrows, F smem)
   return rpc;
 }
 
-// Estimated arithmetic instructions of a row axis with residue blocks of m
-// points and q residues: transforms, the fold (a complex twiddle per term
-// for residues r > 0) and the post-twiddled accumulation.
-static double rowCost(const AxisPlan& a, long m, long q, int A, int B)
+// Estimated instructions of the fused transforms of one row of n points, A
+// forward and B inverse: FP64 instructions per point of each radix's
+// butterfly (fft_smem.cuh; without twiddles in the first stage, less than
+// half of it where half the input is empty) plus a stage's loads, stores
+// and index arithmetic, which weigh more where the arithmetic is FP32.
+static double fusedCost(long n, int prec, int A, int B, bool herm, bool half)
 {
+  int rad[FGB_FUSED_STAGES+8];
+  const int nst=fusedRadices(n,prec,A,herm,half,prec == PREC_F32 ? 16 : 8,
+                             rad);
+  if(nst < 0) return 1e300;
+  auto with=[](int R) {
+    return R == 1 ? 0.0 : R == 2 ? 3.0 : R == 3 ? 6.0 : R == 4 ? 6.0 :
+      R == 5 ? 10.4 : R == 6 ? 10.4 : R == 7 ? 12.9 : R == 8 ? 9.0 : 12.0;
+  };
+  auto without=[](int R) {
+    return R == 1 ? 0.0 : R == 2 ? 2.0 : R == 3 ? 4.0 : R == 4 ? 4.0 :
+      R == 5 ? 7.2 : R == 6 ? 7.0 : R == 7 ? 9.4 : R == 8 ? 6.5 : 9.5;
+  };
+  const double stage=prec == PREC_F64 ? 1.0 : prec == PREC_FF ? 0.5 : 4.0;
+  double fwd=half && rad[0] % 2 == 0 ? 0.68*without(rad[0]) : without(rad[0]);
+  double inv=without(rad[nst-1])+with(rad[0]);
+  for(int s=1; s < nst; ++s) {
+    fwd += with(rad[s]);
+    if(s < nst-1) inv += with(rad[s]);
+  }
+  return n*(A*fwd+B*inv+(A+B)*nst*stage+6.0);
+}
+
+// Lengths a row of at least M points may be padded to, a third longer at
+// most: fewer or cheaper stages may pay for the points (M = 201: 256 = 8 4 8
+// against 210 = 7 5 3 2).
+static std::vector<long> paddedLengths(long M)
+{
+  std::vector<long> v;
+  for(long n=M; n <= M+M/3+8; ++n)
+    if(smooth(n)) v.push_back(n);
+  return v;
+}
+
+// Estimated arithmetic instructions of a row axis with residue blocks of m
+// points and q residues: the fused rows for one residue of one fold, else
+// transforms, the fold (a complex twiddle per term for residues r > 0) and
+// the post-twiddled accumulation.
+static double rowCost(const AxisPlan& a, long m, long q, int A, int B,
+                      int prec)
+{
+  if(q == 1 && a.L <= m)
+    return fusedCost(m,prec,A,B,false,a.kind != KIND_CENTERED && 2*a.L <= m);
+  const double pass=prec == PREC_F64 ? 2.0 : prec == PREC_FF ? 1.0 : 8.0;
   long p=ceilquotient(a.L,m);
-  return q*(A+B)*fftInstr(m)+A*(double) m*(2.0*p+(q-1)*6.0*p)+
-    B*(double) a.L*(2.0+(q-1)*6.0);
+  return q*(A+B)*(fftInstr(m)+pass*m)+
+    A*(double) m*(2.0*p+(q-1)*6.0*p)+B*(double) a.L*(2.0+(q-1)*6.0);
 }
 
 // The same for an outer axis: residue r > 0 folds p terms with a complex
@@ -310,7 +652,10 @@ static double outerCost(const AxisPlan& a, long m, long q, int A, int B)
 }
 
 // Inner (row) axis, complex data: residue block m and residue count q.
-static bool planRowComplex(AxisPlan& a, long mForce, int A, int B, int prec)
+// longer: whether other lengths than the least may be taken (a caller's
+// functor sees the padded length, so its plans keep the least).
+static bool planRowComplex(AxisPlan& a, long mForce, int A, int B, int prec,
+                           bool longer)
 {
   bool centered=a.kind == KIND_CENTERED;
   if(mForce > 0) {
@@ -321,14 +666,15 @@ static bool planRowComplex(AxisPlan& a, long mForce, int A, int B, int prec)
   } else {
     double best=1e300;
     long bm=0, bq=0;
-    for(long q=1; q <= 64; ++q) {
-      long m=nextfftsize(ceilquotient(a.M,q));
-      if(m*q < a.M) continue;
-      if(rowNeed(prec,a.L,m,A,B) > SMEM_MAX) continue;
-      double cost=rowCost(a,m,q,A,B);
+    auto consider=[&](long m, long q) {
+      if(m*q < a.M || rowNeed(prec,a.L,m,A,B) > SMEM_MAX) return;
+      double cost=rowCost(a,m,q,A,B,prec);
       if(cost < best) {best=cost; bm=m; bq=q;}
-    }
+    };
+    for(long q=1; q <= 64; ++q) consider(nextfftsize(ceilquotient(a.M,q)),q);
     if(!bm) return false;
+    if(longer)
+      for(long m : paddedLengths(a.M)) consider(m,1);
     a.m=bm; a.q=bq;
   }
   a.N=a.m*a.q;
@@ -345,7 +691,8 @@ static long evenSmooth(long M)
   return N;
 }
 
-static bool planRowHermitian(AxisPlan& a, long mForce, int A, int prec)
+static bool planRowHermitian(AxisPlan& a, long mForce, int A, int B, int prec,
+                             bool longer)
 {
   long M=a.M;
   if(mForce > 0) {
@@ -354,9 +701,20 @@ static bool planRowHermitian(AxisPlan& a, long mForce, int A, int prec)
     M=std::max<long>(M,mForce*q);
   }
   a.N=evenSmooth(M);
+  // Another even length a third longer at most where its stages cost less.
+  if(longer && mForce <= 0 && hermNeed(prec,a.N/2,A) <= SMEM_MAX) {
+    double best=fusedCost(a.N/2,prec,A,B,true,false);
+    for(long n : paddedLengths(a.N/2)) {
+      const double cost=fusedCost(n,prec,A,B,true,false);
+      if(cost < best && hermNeed(prec,n,A) <= SMEM_MAX) {
+        best=cost;
+        a.N=2*n;
+      }
+    }
+  }
   a.m=a.N; a.q=1; a.p=1;
   a.cshift=0;
-  return hermNeed(prec,a.stored,a.N/2,A) <= SMEM_MAX;
+  return hermNeed(prec,a.N/2,A) <= SMEM_MAX;
 }
 
 // Estimated FP64/FP32 arithmetic instructions of one length-n transform in
@@ -409,10 +767,7 @@ static void planOuter(AxisPlan& a, long mForce, int prec, long C, long nbatch,
     a.N=evenSmooth(mForce > 0 ? std::max(a.M,mForce) : a.M);
     a.m=a.N; a.q=1; a.p=1; a.cshift=0;
     a.rows=a.N/2+1;
-    long Nh=a.N/2;
-    auto sm=[&](int t) {
-      return FGB_BY_PREC(prec,outerRealSmem,a.L,Nh,t);
-    };
+    auto sm=[&](int t) {return realNeed(a,prec,t);};
     a.tile=pickTile(maxTile,C,nbatch*A,sm,minTile);
     a.tileB=pickTile(maxTile,C,nbatch*B,sm,minTile);
     return;
@@ -441,13 +796,8 @@ static void planOuter(AxisPlan& a, long mForce, int prec, long C, long nbatch,
   a.p=ceilquotient(a.L,a.m);
   a.cshift=centered ? (int) (a.L/2) : 0;
   a.rows=a.N;
-  const int ip=a.p == 1;     // in-place outer transforms (FP32-pipe modes)
-  auto smf=[&](int t) {
-    return FGB_BY_PREC(prec,outerFwdSmem,a.L,a.m,t,ip);
-  };
-  auto smb=[&](int t) {
-    return FGB_BY_PREC(prec,outerBwdSmem,a.L,a.m,t,(int) a.q,ip);
-  };
+  auto smf=[&](int t) {return outerFwdNeed(a,prec,t);};
+  auto smb=[&](int t) {return outerBwdNeed(a,prec,t);};
   a.tile=pickTile(maxTile,C,nbatch*a.q*A,smf,minTile);
   a.tileB=pickTile(maxTile,C,nbatch*B,smb,minTile);
   if(smf(a.tile) > SMEM_MAX || smb(a.tileB) > SMEM_MAX)
@@ -530,8 +880,9 @@ Conv::Conv(int dim, const int *kinds, const long *L, const long *M,
   AxisPlan& in=I.axis[dim-1];
   long mf=mForce ? mForce[dim-1] : 0;
   bool ok;
-  if(in.kind == KIND_HERMITIAN) ok=planRowHermitian(in,mf,A,prec);
-  else ok=planRowComplex(in,mf,A,B,prec);
+  const bool longer=mult != MULT_USER;
+  if(in.kind == KIND_HERMITIAN) ok=planRowHermitian(in,mf,A,B,prec,longer);
+  else ok=planRowComplex(in,mf,A,B,prec,longer);
   if(in.kind == KIND_REAL && dim == 1) in.rows=0;
   if(!ok) {
     // Long rows (beyond one CTA's shared memory), any kind: the row is a
@@ -568,17 +919,9 @@ Conv::Conv(int dim, const int *kinds, const long *L, const long *M,
   // Rows per CTA of the row kernel.
   long nrows=batch;
   for(int d=0; d < dim-1; ++d) nrows *= I.axis[d].rows;
-  if(I.longRow) {
-    in.rpc=pickRpc(I.rowM,A,I.rowQ*nrows,[&](int r) {
-      return rowNeed(prec,I.rowM,I.rowM,A,B,r,1);});
-  } else if(in.kind == KIND_HERMITIAN) {
-    in.rpc=pickRpc(in.N/2,A,nrows,[&](int r) {
-      return hermNeed(prec,in.stored,in.N/2,A,r);});
-  } else {
-    in.rpc=pickRpc(in.m,A,nrows,[&](int r) {
-      return rowNeed(prec,in.stored,in.m,A,B,r,
-                     in.q == 1 && in.stored <= in.m);});
-  }
+  in.rpc=pickRpc(I.longRow ? I.rowM : in.kind == KIND_HERMITIAN ? in.N/2 :
+                 in.m,A,I.longRow ? I.rowQ*nrows : nrows,[&](int r) {
+                   return innerNeed(I,in,r,256);});
   try {
     allocate();
     if(autotune && tuneSchedule) tune();
@@ -612,13 +955,15 @@ static std::vector<long> residueCandidates(const AxisPlan& a, bool outer,
       if(N % m == 0 && smooth(m) && outerNeed(prec,a.L,m,1) <= SMEM_MAX)
         c.push_back({outerCost(a,m,N/m,A,B),m});
   } else {
-    for(long q=1; q <= 64; ++q) {
-      long m=nextfftsize(ceilquotient(a.M,q));
-      if(m*q < a.M || rowNeed(prec,a.L,m,A,B) > SMEM_MAX) continue;
-      bool seen=false;
-      for(const auto& x : c) seen=seen || x.second == m;
-      if(!seen) c.push_back({rowCost(a,m,q,A,B),m});
-    }
+    auto add=[&](long m, long q) {
+      if(m*q < a.M || rowNeed(prec,a.L,m,A,B) > SMEM_MAX) return;
+      for(const auto& x : c)
+        if(x.second == m) return;
+      c.push_back({rowCost(a,m,q,A,B,prec),m});
+    };
+    for(long q=1; q <= 64; ++q) add(nextfftsize(ceilquotient(a.M,q)),q);
+    if(!c.empty())
+      for(long m : paddedLengths(a.M)) add(m,1);
   }
   std::sort(c.begin(),c.end());
   std::vector<long> out;
@@ -725,7 +1070,7 @@ bool Conv::applySchedule(const std::string& text)
   long v[19];
   for(long& x : v)
     if(!(in >> x)) return false;
-  const int dim=I.dim, prec=I.prec, A=I.A, B=I.B;
+  const int dim=I.dim, prec=I.prec;
   auto thrOk=[](long t) {return t == 128 || t == 256;};
   auto p2=[](long t) {return t >= 1 && (t & (t-1)) == 0;};
   AxisPlan ax[3];
@@ -739,15 +1084,8 @@ bool Conv::applySchedule(const std::string& text)
     if(d < dim-1 && !I.longRow) {
       const int tmax=wide(prec) ? 8 : 16;
       if(!p2(s[0]) || !p2(s[2]) || s[0] > tmax || s[2] > tmax) return false;
-      size_t sf, sb;
-      if(a.kind == KIND_REAL) {
-        sf=FGB_BY_PREC(prec,outerRealSmem,a.L,a.N/2,(int) s[0]);
-        sb=FGB_BY_PREC(prec,outerRealSmem,a.L,a.N/2,(int) s[2]);
-      } else {
-        sf=FGB_BY_PREC(prec,outerFwdSmem,a.L,a.m,(int) s[0],(int) (a.p == 1));
-        sb=FGB_BY_PREC(prec,outerBwdSmem,a.L,a.m,(int) s[2],(int) a.q,
-                       (int) (a.p == 1));
-      }
+      const size_t sf=outerFwdNeed(a,prec,(int) s[0]);
+      const size_t sb=outerBwdNeed(a,prec,(int) s[2]);
       if(sf > SMEM_MAX || sb > SMEM_MAX) return false;
       a.tile=(int) s[0];
       a.tileB=(int) s[2];
@@ -756,9 +1094,7 @@ bool Conv::applySchedule(const std::string& text)
       const long r=s[4];
       if(r != 1 && r != 2 && r != 3 && r != 4 && r != 6 && r != 8)
         return false;
-      const size_t need=I.longRow ? rowNeed(prec,I.rowM,I.rowM,A,B,r,1) :
-        a.kind == KIND_HERMITIAN ? hermNeed(prec,a.stored,a.N/2,A,r) :
-        rowNeed(prec,a.stored,a.m,A,B,r,a.q == 1 && a.stored <= a.m);
+      const size_t need=innerNeed(I,a,(int) r,a.thr);
       if(need > SMEM_MAX) return false;
       a.rpc=(int) r;
     }
@@ -924,11 +1260,8 @@ void Conv::tune()
     long avail=I.longRow ? I.rowQ*nrows : nrows;
     for(int r : {1,2,3,4,6,8}) {
       if(r > avail) break;
-      size_t need=I.longRow ? rowNeed(prec,I.rowM,I.rowM,A,B,r,1) :
-        in.kind == KIND_HERMITIAN ? hermNeed(prec,in.stored,in.N/2,A,r) :
-        rowNeed(prec,in.stored,in.m,A,B,r,in.q == 1 && in.stored <= in.m);
-      if(need <= SMEM_MAX)
-        for(int th : thrs) t.cands.push_back({r,th});
+      for(int th : thrs)
+        if(innerNeed(I,in,r,th) <= SMEM_MAX) t.cands.push_back({r,th});
     }
     if(t.cands.size() > 1) tn.push_back(t);
   }
@@ -946,14 +1279,7 @@ void Conv::tune()
       f.launch=d;
       b.launch=2*(dim-1)-d;
       for(int t=1; t <= (wide(prec) ? 8 : 16) && t <= C; t *= 2) {
-        size_t sf, sb;
-        if(a.kind == KIND_REAL) {
-          sf=sb=FGB_BY_PREC(prec,outerRealSmem,a.L,a.N/2,t);
-        } else {
-          sf=FGB_BY_PREC(prec,outerFwdSmem,a.L,a.m,t,(int) (a.p == 1));
-          sb=FGB_BY_PREC(prec,outerBwdSmem,a.L,a.m,t,(int) a.q,
-                         (int) (a.p == 1));
-        }
+        const size_t sf=outerFwdNeed(a,prec,t), sb=outerBwdNeed(a,prec,t);
         for(int th : thrs) {
           if(sf <= SMEM_MAX) f.cands.push_back({t,th});
           if(sb <= SMEM_MAX) b.cands.push_back({t,th});
@@ -1187,7 +1513,6 @@ cudaError_t Conv::runT(const void *const *in, void *const *out, cudaStream_t s)
 {
   typedef cplx<T> Cx;
   const int A=I.A, B=I.B;
-  const int threads=256;
   cudaError_t e;
   double scale=1.0;
   if(normalize)
@@ -1221,9 +1546,9 @@ cudaError_t Conv::runT(const void *const *in, void *const *out, cudaStream_t s)
       const AxisPlan& a=I.axis[d];
       im.m[d]=(int) a.m;
       im.q[d]=(int) a.q;
-      im.rev[d]=inplaceFFT<T>() && a.kind != KIND_REAL && a.p == 1;
+      im.rev[d]=outerFused(a);
       if(im.rev[d]) {
-        FFTPlanDev f=fftPlan(a.m,I.prec,true,true);   // as outerPlan
+        const FusedFFT f=outerFFT(a,I.prec,1);        // radices as outerPlan's
         im.nst[d]=f.nst;
         for(int k=0; k < f.nst; ++k) im.radix[d][k]=(unsigned char) f.radix[k];
       }
@@ -1238,8 +1563,13 @@ cudaError_t Conv::runT(const void *const *in, void *const *out, cudaStream_t s)
     P.realIO=a.kind == KIND_REAL && I.dim == 1;
     P.rpc=I.axis[I.dim-1].rpc;
     P.io64=0;
-    P.direct=a.q == 1 && a.stored <= a.m;
-    P.fp=fftPlan(a.m,I.prec,inplaceFFT<T>() || P.direct,true);
+    P.direct=rowDirect(a);
+    P.nteam=rowTeams(P.rpc,a.thr);
+    if(P.direct) {
+      P.fz=fusedRowPlan(a.m,I.prec,A,false,halfEmpty(a),P.nteam,
+                        widest(I.prec));
+      fusedTables(P.fz,I.prec);
+    } else P.fp=fftPlan(a.m,I.prec,inplaceFFT<T>(),true);
     P.twN=(const typename TwT<T>::type *) twiddles(a.N,I.prec);
   };
   auto hermPlan=[&](HermRowPlan<T>& P, const AxisPlan& a) {
@@ -1248,8 +1578,10 @@ cudaError_t Conv::runT(const void *const *in, void *const *out, cudaStream_t s)
     P.H=(int) a.stored; P.N=(int) a.N; P.Nh=(int) (a.N/2);
     P.A=A; P.B=B; P.mult=I.mult;
     P.rpc=a.rpc;
+    P.nteam=rowTeams(P.rpc,a.thr);
     P.io64=0;
-    P.fp=fftPlan(a.N/2,I.prec,inplaceFFT<T>(),true);
+    P.fz=fusedRowPlan(a.N/2,I.prec,A,true,false,P.nteam,widest(I.prec));
+    fusedTables(P.fz,I.prec);
     P.twN=(const typename TwT<T>::type *) twiddles(a.N,I.prec);
   };
   auto outerPlan=[&](OuterPlan<T>& P, const AxisPlan& a) {
@@ -1257,12 +1589,23 @@ cudaError_t Conv::runT(const void *const *in, void *const *out, cudaStream_t s)
     P.L=(int) a.L; P.m=(int) a.m; P.q=(int) a.q; P.N=(int) a.N;
     P.cshift=a.cshift; P.tile=a.tile;
     P.io64=0;
-    P.inplace=inplaceFFT<T>() && a.kind != KIND_REAL && a.p == 1;
+    P.fused=outerFused(a);
     P.conj=0;
-    P.fp=fftPlan(a.kind == KIND_REAL ? a.N/2 : a.m,I.prec,P.inplace != 0,
-                 true);
+    if(P.fused || a.kind == KIND_REAL) {
+      P.fz=P.fused ? outerFFT(a,I.prec,a.tile) :
+        realFFT(a.N,a.L,I.prec,a.tile);
+      fusedTables(P.fz,I.prec);
+    } else P.fp=fftPlan(a.m,I.prec);
     P.twN=(const typename TwT<T>::type *) twiddles(a.N,I.prec);
     P.twX=NULL; P.NX=1;
+  };
+  // The backward launch's column tile (the padding of a fused transform
+  // depends on it; its tables do not).
+  auto retile=[&](OuterPlan<T>& P, const AxisPlan& a) {
+    P.tile=a.tileB;
+    if(P.fused) P.fz.lg=outerFFT(a,I.prec,a.tileB).lg;
+    else if(a.kind == KIND_REAL)
+      P.fz.lg=realFFT(a.N,a.L,I.prec,a.tileB).lg;
   };
   // The first outer-axis launch.  While a host call copies the inputs in
   // (chunks > 0): input 0 one launch per column range, each on its own
@@ -1398,7 +1741,7 @@ cudaError_t Conv::runT(const void *const *in, void *const *out, cudaStream_t s)
     }
     if(e != cudaSuccess) return e;
     O.count=B;
-    O.tile=ax.tileB;
+    retile(O,ax);
     O.scale=(T) scale;
     O.io64=OUT64;
     O.inRow=C;                                  // staging side
@@ -1468,7 +1811,7 @@ cudaError_t Conv::runT(const void *const *in, void *const *out, cudaStream_t s)
   if(e != cudaSuccess) return e;
 
   Y.count=B;
-  Y.tile=ay.tileB;
+  retile(Y,ay);
   for(int i=0; i < B; ++i) {Y.in[i]=(const Cx *) by[i]; Y.out[i]=(Cx *) bx[i];}
   std::swap(Y.inBatch,Y.outBatch);
   e=launchOuterBwd<T>(Y,ay.thrB,s);
@@ -1476,7 +1819,7 @@ cudaError_t Conv::runT(const void *const *in, void *const *out, cudaStream_t s)
   if(e != cudaSuccess) return e;
 
   X.count=B;
-  X.tile=ax.tileB;
+  retile(X,ax);
   X.scale=(T) scale;
   X.io64=OUT64;
   X.inRow=Cx_;                                  // staging side
@@ -1514,7 +1857,7 @@ cudaError_t Conv::runLong(const void *const *in, void *const *out,
   O.twX=(const typename TwT<T>::type *) twiddles(N,I.prec);
   O.NX=N;
   O.io64=io64 & 1; O.ioShift=guard;
-  O.inplace=0; O.conj=0;
+  O.conj=0;
   O.flat=flat; O.flatC=a.cshift;
   O.count=A; O.nbatch=(int) nrows; O.inBatch=rowStride; O.outBatch=N;
   O.inRow=m; O.outRow=m; O.C=(int) m; O.Ltot=a.stored;
@@ -1529,7 +1872,9 @@ cudaError_t Conv::runLong(const void *const *in, void *const *out,
   P.L=(int) m; P.m=(int) m; P.q=1; P.N=(int) m; P.cshift=0;
   P.A=A; P.B=B; P.mult=I.mult; P.realIO=0;
   P.rpc=a.rpc; P.io64=0; P.direct=1; P.ioShift=NULL;
-  P.fp=fftPlan(m,I.prec,true,true);
+  P.nteam=rowTeams(P.rpc,a.thr);
+  P.fz=fusedRowPlan(m,I.prec,A,false,false,P.nteam,widest(I.prec));
+  fusedTables(P.fz,I.prec);
   P.twN=(const typename TwT<T>::type *) twiddles(m,I.prec);
   for(int i=0; i < A; ++i) P.in[i]=(const Cx *) lb[i];
   for(int i=0; i < B; ++i) P.out[i]=(Cx *) lb[i];
@@ -2071,10 +2416,13 @@ cudaError_t PadTransform::runT(const void *in, void *out, bool fwd,
   OuterPlan<T> P{};
   P.L=(int) a.L; P.m=(int) a.m; P.q=(int) a.q; P.N=(int) a.N;
   P.cshift=a.cshift; P.tile=fwd ? a.tile : a.tileB;
-  P.fp=fftPlan(a.kind == KIND_REAL ? a.N/2 : a.m,prec);
+  if(a.kind == KIND_REAL || a.kind == KIND_HERMITIAN) {
+    P.fz=realFFT(a.N,a.kind == KIND_REAL ? a.L : a.N,prec,P.tile);
+    fusedTables(P.fz,prec);
+  } else P.fp=fftPlan(a.m,prec);
   P.twN=(const typename TwT<T>::type *) twiddles(a.N,prec);
   P.twX=NULL; P.NX=1;
-  P.io64=0; P.inplace=0;     // the public layout is natural order
+  P.io64=0; P.fused=0;       // the public layout is natural order
   P.conj=0;
   P.count=1; P.nbatch=1; P.inBatch=P.outBatch=0;
   P.inRow=C; P.outRow=C; P.C=(int) C; P.Ltot=(long long) a.L*C;
@@ -2088,7 +2436,6 @@ cudaError_t PadTransform::runT(const void *in, void *out, bool fwd,
     // backward: N reals to the H modes with sign -1 (real-to-complex,
     // conjugated).
     P.L=(int) a.N;
-    P.fp=fftPlan(a.N/2,prec);
     P.conj=1;
     P.kc=(int) a.stored;
     return fwd ? launchOuterRealBwd<T>(P,threads,s) :
@@ -2141,8 +2488,8 @@ PlainFFT::PlainFFT(int kind, long n, int sign, long C, long B, long istride,
   int maxTile=wide(prec) ? 8 : 16;
   auto sm=[&](int t) -> size_t {
     if(kind == FFT_C2C)
-      return std::max(FGB_BY_PREC(prec,outerFwdSmem,n,n,t,0),
-                      FGB_BY_PREC(prec,outerBwdSmem,n,n,t,1,0));
+      return std::max(FGB_BY_PREC(prec,outerFwdSmem,n,n,t),
+                      FGB_BY_PREC(prec,outerBwdSmem,n,n,t,1));
     return FGB_BY_PREC(prec,outerRealSmem,n,n/2,t);
   };
   if(sm(1) > SMEM_MAX) {
@@ -2155,8 +2502,8 @@ PlainFFT::PlainFFT(int kind, long n, int sign, long C, long B, long istride,
     // n = n1 n2 with both passes in one CTA, n1 as close to sqrt(n) as
     // the factors allow.
     auto fits=[&](long k, int t) {
-      return std::max(FGB_BY_PREC(prec,outerFwdSmem,k,k,t,0),
-                      FGB_BY_PREC(prec,outerBwdSmem,k,k,t,1,0)) <= SMEM_MAX;
+      return std::max(FGB_BY_PREC(prec,outerFwdSmem,k,k,t),
+                      FGB_BY_PREC(prec,outerBwdSmem,k,k,t,1)) <= SMEM_MAX;
     };
     long best=0;
     for(long a=2; a*a <= n*4 && a < n; ++a)
@@ -2171,8 +2518,8 @@ PlainFFT::PlainFFT(int kind, long n, int sign, long C, long B, long istride,
     // stride takes whole tiles; the strided one single columns.
     auto smw=[&](long k) {
       return [&,k](int t) {
-        return std::max(FGB_BY_PREC(prec,outerFwdSmem,k,k,t,0),
-                        FGB_BY_PREC(prec,outerBwdSmem,k,k,t,1,0));
+        return std::max(FGB_BY_PREC(prec,outerFwdSmem,k,k,t),
+                        FGB_BY_PREC(prec,outerBwdSmem,k,k,t,1));
       };
     };
     tile1=pickTile(maxTile,sign > 0 ? n2 : n1,B,smw(sign > 0 ? n1 : n2));
@@ -2212,7 +2559,7 @@ cudaError_t PlainFFT::runTwoPass(const void *in, void *out, cudaStream_t s)
     P.fp=fftPlan(len,prec);
     P.twN=(const typename TwT<T>::type *) twiddles(len,prec);
     P.twX=NULL; P.NX=1;
-    P.io64=0; P.inplace=0; P.conj=0;
+    P.io64=0; P.fused=0; P.conj=0;
     P.count=1; P.nbatch=(int) B;
     P.Ltot=LLONG_MAX;
     P.scale=(T) 1;
@@ -2258,10 +2605,13 @@ cudaError_t PlainFFT::runT(const void *in, void *out, cudaStream_t s)
   const bool real=kind != FFT_C2C;
   P.L=(int) n; P.m=(int) n; P.q=1; P.N=(int) n; P.cshift=0;
   P.tile=tile;
-  P.fp=fftPlan(real ? n/2 : n,prec);
+  if(real) {
+    P.fz=realFFT(n,n,prec,tile);
+    fusedTables(P.fz,prec);
+  } else P.fp=fftPlan(n,prec);
   P.twN=(const typename TwT<T>::type *) twiddles(n,prec);
   P.twX=NULL; P.NX=1;
-  P.io64=0; P.inplace=0;
+  P.io64=0; P.fused=0;
   // The real kernels compute the sign +1 r2c and sign -1 c2r; FFTW's r2c
   // (-1) and c2r (+1) are their conjugates on the complex side.
   P.conj=real ? 1 : 0;

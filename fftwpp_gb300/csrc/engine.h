@@ -38,6 +38,14 @@ void refParameters(size_t L, size_t M, size_t m, bool centered,
 bool smooth(size_t n);   // n = 2^a 3^b 5^c 7^d
 // Radices of the shared-memory transforms of length n (engine.cu).
 int fftRadices(long n, int prec, bool oddFirst, bool allow16, int *radix);
+// Radices of the fused transforms (fft_fused.cuh) of length n for a row
+// kernel of A inputs (A = 1: an outer axis), at most maxR; herm: the
+// Hermitian rows' transform; half: the second half of the input is zero.
+// Returns their count, or -1.
+int fusedRadices(long n, int prec, int A, bool herm, bool half, int maxR,
+                 int *radix);
+int fusedPadding(const int *radix, int nst, int level);
+int rowTeams(int rpc, int threads);
 
 struct AxisPlan {
   int kind;

@@ -93,6 +93,10 @@ inline bool hasWideRadix(const FFTPlanDev& p)
 
 template<int R, int S, typename T> struct Codelet;
 
+template<int S, typename T> struct Codelet<1,S,T> {
+  static __device__ __forceinline__ void run(cplx<T> *) {}
+};
+
 template<int S, typename T> struct Codelet<2,S,T> {
   static __device__ __forceinline__ void run(cplx<T> *a) {
     cplx<T> t=a[0];

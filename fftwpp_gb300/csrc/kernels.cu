@@ -28,7 +28,7 @@ __device__ __forceinline__ long long dataCol(const OuterPlan<T>& P, int col)
 // ---------------------------------------------------------------------------
 // Outer forward, complex data: residue block r of the padded transform along
 // a strided axis for `tile` adjacent columns.
-template<typename T, bool CG, bool R16=false>
+template<typename T, bool CG>
 __device__ __forceinline__ void outerFwdTile(const OuterPlan<T>& P, int ctile,
                                              int r, int z,
                                              unsigned char *smemRaw)
@@ -143,21 +143,6 @@ __device__ __forceinline__ void outerFwdTile(const OuterPlan<T>& P, int ctile,
     __syncthreads();
   }
 
-  if constexpr(inplaceFFT<T>()) {
-    if(P.inplace) {
-      // Transform in place (digit-reversed j; the row kernels do not
-      // depend on row order and the backward undoes it).
-      fftDIF<T,1,R16>(x,P.fp,tile,tile,tid,nthr);
-      for(int i=tid; i < m*tile; i += nthr) {
-        int j=dTile(i), cc=i-j*tile;
-        int col=col0+cc;
-        if(col < P.C) dst[((long long) r*m+j)*P.outRow+col]=x[sp(i)];
-      }
-      __syncthreads();
-      return;
-    }
-  }
-
   cplx<T> *X=fftSmem<T,1>(x,y,P.fp,tile,tile,tid,nthr);
   for(int i=tid; i < m*tile; i += nthr) {
     int j=dTile(i), cc=i-j*tile;
@@ -185,7 +170,7 @@ outerFwdKernel(const OuterPlan<T> P)
 }
 
 // Outer backward, complex data: all residues of a column tile, accumulated.
-template<typename T, bool CG, bool R16=false>
+template<typename T, bool CG>
 __device__ __forceinline__ void outerBwdTile(const OuterPlan<T>& P, int ctile,
                                              int z, unsigned char *smemRaw)
 {
@@ -237,13 +222,7 @@ __device__ __forceinline__ void outerBwdTile(const OuterPlan<T>& P, int ctile,
       }
       __syncthreads();
     }
-    cplx<T> *X;
-    if(inplaceFFT<T>() && P.inplace) {
-      fftDIT<T,-1,R16>(x,P.fp,tile,tile,tid,nthr);
-      X=x;
-    } else {
-      X=fftSmem<T,-1>(x,y,P.fp,tile,tile,tid,nthr);
-    }
+    cplx<T> *X=fftSmem<T,-1>(x,y,P.fp,tile,tile,tid,nthr);
     if(direct && P.flat != FLAT_PAD) {
       // Long rows of the other kinds: the output of data index sx is the
       // flattened position n of its kind (FlatMode).
@@ -306,136 +285,540 @@ outerBwdKernel(const OuterPlan<T> P)
   outerBwdTile<T,false>(P,blockIdx.x,blockIdx.z,smemRaw);
 }
 
-// FP32 in-place plans with radix-16 or radix-6 stages: their own
-// instantiations, capped at 85 registers a thread (the wider codelets need
-// more registers than the others may take).
+// ---------------------------------------------------------------------------
+// Fused outer kernels (fft_fused.cuh), for residue blocks at least as long as
+// the data: the first forward stage reads the caller's columns and applies
+// the residue twiddle, the last one writes the staging rows, in the
+// digit-reversed order of the transform (the row kernels do not depend on
+// row order and the backward undoes it).  The column tile's values cross
+// shared memory once between stages and never before the first or after
+// the last.
+// Float-float (runStages): the tile's inputs into shared memory, and its
+// outputs out of it.  in(cc, j) gives element j of column cc.
+template<class In>
+__device__ __forceinline__ void loadTileFF(cplx<ff> *x, const FusedFFT& p,
+                                           int lt, int tid, int nthr,
+                                           const In& in)
+{
+#pragma unroll 4
+  for(int idx=tid; idx < p.n << lt; idx += nthr) {
+    const int j=idx >> lt, cc=idx & ((1 << lt)-1);
+    x[(spl(j,p.lg) << lt)+cc]=in(cc,j);
+  }
+}
+
+// FP64 bits read as a float-float value, converted in line (one place, whose
+// loads the loop issues together).
+__device__ __forceinline__ cplx<ff> fromBits(cplx<ff> v, int sh)
+{
+  return mk(toFF(__hiloint2double(__float_as_int(v.x.lo),
+                                  __float_as_int(v.x.hi)),sh),
+            toFF(__hiloint2double(__float_as_int(v.y.lo),
+                                  __float_as_int(v.y.hi)),sh));
+}
+
+template<class Store>
+__device__ __forceinline__ void storeTileFF(const cplx<ff> *x,
+                                            const FusedFFT& p, int lt, int tid,
+                                            int nthr, const Store& store)
+{
+#pragma unroll 2
+  for(int idx=tid; idx < p.n << lt; idx += nthr) {
+    const int j=idx >> lt, cc=idx & ((1 << lt)-1);
+    store(0,cc)(j,swapXY(x[(spl(j,p.lg) << lt)+cc]));
+  }
+}
+
+template<typename T, int R>
+__device__ __forceinline__ void outerLastFwd(const OuterPlan<T>& P,
+                                             const cplx<T> *x, cplx<T> *dst,
+                                             int col0, int nblk, int tid,
+                                             int nthr)
+{
+  typedef typename TwT<T>::type Tw;
+  const FusedFFT& p=P.fz;
+  const int lt=log2of(P.tile), total=nblk << lt;
+  const Tw *tw=(const Tw *) p.twb+(nblk-p.radix[0]);
+#pragma unroll 1
+  for(int idx=tid; idx < total; idx += nthr) {
+    const int b=idx >> lt, cc=idx & (P.tile-1), col=col0+cc;
+    const cplx<T> *xq=x+(spl(b*R,p.lg) << lt)+cc;
+    cplx<T> a[1][R];
+#pragma unroll
+    for(int r=0; r < R; ++r) a[0][r]=nrm(xq[r << lt]);
+    inTwiddleDFT<T,R,1>(a,tw,b,nblk);
+    if(col >= P.C) continue;
+    cplx<T> *d=dst+(long long) (b*R)*P.outRow+col;
+#pragma unroll
+    for(int r=0; r < R; ++r) d[r*P.outRow]=a[0][r];
+  }
+}
+
+template<typename T, bool WIDE>
+__device__ __forceinline__ void outerFwdFused(const OuterPlan<T>& P,
+                                              unsigned char *smemRaw)
+{
+  const int tile=P.tile, m=P.m, N=P.N, c=P.cshift, L=P.L;
+  cplx<T> *x=(cplx<T> *) smemRaw;
+  const int tid=threadIdx.x, nthr=blockDim.x;
+  const int col0=blockIdx.x*tile, r=blockIdx.y;
+  const int a=blockIdx.z % P.count;
+  const long long batch=blockIdx.z/P.count;
+  const cplx<T> *src=P.in[a]+batch*P.inBatch;
+  cplx<T> *dst=P.out[a]+batch*P.outBatch+(long long) r*m*P.outRow;
+  const int lt=log2of(tile);
+  const int sh=ioShift<T>(P.ioShift,a);
+  const auto load=[&](int, int cc) {
+    const int top=col0+cc < P.C ? L : 0;      // entries of a column that
+    const cplx<T> *f=src+dataCol(P,col0+cc);  // exists
+    return [=,&P](int j) {
+      int s=j+c;
+      if(s >= m) s -= m;
+      cplx<T> v=mk((T) 0,(T) 0);
+      if(s < top) {
+        v=loadIO(f+s*P.inRow,P.io64 & 1,sh);
+        if(r != 0) v=twmul<1>(v,P.twN[twExp(s,c,r,N)]);
+      }
+      return v;
+    };
+  };
+  if constexpr(std::is_same<T,ff>::value) {
+    loadTileFF(x,P.fz,lt,tid,nthr,[&](int cc, int j) {
+        int s=j+c;
+        if(s >= m) s -= m;
+        cplx<T> v=mk((T) 0,(T) 0);
+        if(s < L && col0+cc < P.C) {
+          v=src[s*P.inRow+dataCol(P,col0+cc)];
+          if(P.io64 & 1) v=fromBits(v,sh);
+          if(r != 0) v=twmul<1>(v,P.twN[twExp(s,c,r,N)]);
+        }
+        return v;
+      });
+    runStages<T>(x,0,1,0,P.fz,lt,0,0,tid,nthr,[] {});
+#pragma unroll 4
+    for(int idx=tid; idx < m << lt; idx += nthr) {
+      const int j=idx >> lt, cc=idx & (tile-1);
+      if(col0+cc < P.C)
+        dst[j*P.outRow+col0+cc]=x[(spl(j,P.fz.lg) << lt)+cc];
+    }
+    return;
+  }
+  runFusedFirst<T,WIDE>(x,0,1,P.fz,lt,tid,nthr,load);
+  const int nblk=runFusedMiddle<T,WIDE>(x,0,1,P.fz,lt,false,0,tid,nthr);
+  __syncthreads();
+  FGB_FUSED_SWITCH(P.fz.radix[P.fz.nst-1],
+                   (outerLastFwd<T,R_>(P,x,dst,col0,nblk,tid,nthr)))
+}
+
 template<typename T>
-__global__ void __launch_bounds__(256,3)
-outerFwdKernel16(const OuterPlan<T> P)
+__global__ void __launch_bounds__(256)
+outerFwdFusedKernel(const OuterPlan<T> P)
 {
   extern __shared__ __align__(16) unsigned char smemRaw[];
-  outerFwdTile<T,false,true>(P,blockIdx.x,blockIdx.y,blockIdx.z,smemRaw);
+  outerFwdFused<T,false>(P,smemRaw);
+}
+
+// The first inverse stage: staging rows into shared memory.
+template<typename T, int R>
+__device__ __forceinline__ void outerFirstInv(const OuterPlan<T>& P,
+                                              cplx<T> *x, const cplx<T> *src,
+                                              int col0, int tid, int nthr)
+{
+  const FusedFFT& p=P.fz;
+  const int lt=log2of(P.tile), total=p.n/R << lt;
+#pragma unroll 1
+  for(int idx=tid; idx < total; idx += nthr) {
+    const int b=idx >> lt, cc=idx & (P.tile-1), col=col0+cc;
+    const cplx<T> *s=src+(long long) (b*R)*P.inRow+col;
+    cplx<T> a[R];
+#pragma unroll
+    for(int r=0; r < R; ++r)
+      a[r]=col < P.C ? s[r*P.inRow] : mk((T) 0,(T) 0);
+#pragma unroll
+    for(int r=0; r < R; ++r) a[r]=nrm(swapXY(a[r]));
+    Codelet<R,1,T>::run(a);
+    cplx<T> *xq=x+(spl(b*R,p.lg) << lt)+cc;
+#pragma unroll
+    for(int r=0; r < R; ++r) xq[r << lt]=a[r];
+  }
+}
+
+// All residues of a column tile; with several, a thread adds the outputs it
+// computes into its own entries of an accumulator behind the tile.
+template<typename T, bool WIDE>
+__device__ __forceinline__ void outerBwdFused(const OuterPlan<T>& P,
+                                              unsigned char *smemRaw)
+{
+  const int tile=P.tile, m=P.m, N=P.N, c=P.cshift, L=P.L, q=P.q;
+  cplx<T> *x=(cplx<T> *) smemRaw;
+  cplx<T> *acc=x+fusedSpan(P.fz.n,P.fz.lg)*tile;
+  const int tid=threadIdx.x, nthr=blockDim.x;
+  const int col0=blockIdx.x*tile;
+  const int b=blockIdx.z % P.count;
+  const long long batch=blockIdx.z/P.count;
+  const cplx<T> *src=P.in[b]+batch*P.inBatch;
+  cplx<T> *dst=P.out[b]+batch*P.outBatch;
+  const int lt=log2of(tile);
+  const int sh=ioShift<T>(P.ioShift,8+b);
+  for(int r=0; r < q; ++r) {
+    const cplx<T> *sr=src+(long long) r*m*P.inRow;
+    const auto store=[&](int, int cc) {
+      const int top=col0+cc < P.C ? L : 0;
+      cplx<T> *f=dst+dataCol(P,col0+cc);
+      return [=,&P](int j, cplx<T> v) {
+        int s=j+c;
+        if(s >= m) s -= m;
+        if(s >= top) return;
+        if(q > 1) {
+          if(r != 0) v=accum(acc[s*tile+cc],
+                             twmul<-1>(v,P.twN[twExp(s,c,r,N)]));
+          if(r < q-1) {
+            acc[s*tile+cc]=v;
+            return;
+          }
+        }
+        storeIO(f+s*P.outRow,v*P.scale,P.io64 & 2,sh);
+      };
+    };
+    if constexpr(std::is_same<T,ff>::value) {
+      loadTileFF(x,P.fz,lt,tid,nthr,[&](int cc, int j) {
+          return col0+cc < P.C ? swapXY(sr[j*P.inRow+col0+cc]) :
+            mk((T) 0,(T) 0);
+        });
+      runStages<T>(x,0,0,1,P.fz,lt,0,0,tid,nthr,[] {});
+      storeTileFF(x,P.fz,lt,tid,nthr,store);
+    } else {
+      FGB_FUSED_SWITCH(P.fz.radix[P.fz.nst-1],
+                       (outerFirstInv<T,R_>(P,x,sr,col0,tid,nthr)))
+      runFusedMiddle<T,WIDE>(x,0,1,P.fz,lt,true,0,tid,nthr);
+      __syncthreads();
+      runFusedLast<T,WIDE>(x,0,1,P.fz,lt,tid,nthr,store);
+    }
+    if(r < q-1) __syncthreads();
+  }
+}
+
+template<typename T>
+__global__ void __launch_bounds__(256)
+outerBwdFusedKernel(const OuterPlan<T> P)
+{
+  extern __shared__ __align__(16) unsigned char smemRaw[];
+  outerBwdFused<T,false>(P,smemRaw);
+}
+
+// FP32 plans with a radix-16 stage: their own instantiations, capped at 85
+// registers a thread (the wider codelet needs more registers than the
+// others may take).
+template<typename T>
+__global__ void __launch_bounds__(256,3)
+outerFwdFusedKernel16(const OuterPlan<T> P)
+{
+  extern __shared__ __align__(16) unsigned char smemRaw[];
+  outerFwdFused<T,true>(P,smemRaw);
 }
 
 template<typename T>
 __global__ void __launch_bounds__(256,3)
-outerBwdKernel16(const OuterPlan<T> P)
+outerBwdFusedKernel16(const OuterPlan<T> P)
 {
   extern __shared__ __align__(16) unsigned char smemRaw[];
-  outerBwdTile<T,false,true>(P,blockIdx.x,blockIdx.z,smemRaw);
+  outerBwdFused<T,true>(P,smemRaw);
 }
 
 // ---------------------------------------------------------------------------
-// Outer forward, real data (fftPadReal with explicit padding to even N):
-// pack z[t] = f[2t] + i f[2t+1], sign +1 FFT of length N/2, unpack the
-// N/2+1 non-negative modes F(k) = E[k] + W_N^k O[k].
+// Outer axis, real data (fftPadReal with explicit padding to even N), both
+// directions in the fused form: z[t] = f[2t] + i f[2t+1] through a transform
+// of length Nh = N/2, the N/2+1 modes in natural order on the other side.
+// Unpacking pairs mode k with Nh-k; the last forward stage holds modes
+// kappa + nblk t of block b (kappa = rev(b)), whose partners are all in the
+// block of nblk - kappa, so one thread finishes both blocks of a pair
+// (FusedFFT::pairs, blocks in order: b, its partner, kappa; the first entry
+// holds blocks 0 and that of nblk/2, -1 if nblk is odd, which are their own
+// partners).  The inverse packs in the same pairs as it loads.
+
+// F[k] = e + W_N^k o and F[Nh-k] = conj(e - W_N^k o) from Z[k] and
+// Z[Nh-k], e = (Z[k] + conj Z[Nh-k])/2, o = -i (Z[k] - conj Z[Nh-k])/2.
 template<typename T>
-__global__ void __launch_bounds__(256)
-outerRealFwdKernel(const OuterPlan<T> P)
+__device__ __forceinline__ void realUnpack(cplx<T> zk, cplx<T> zm,
+                                           typename TwT<T>::type w,
+                                           cplx<T>& F, cplx<T>& Fc)
 {
-  extern __shared__ __align__(16) unsigned char smemRaw[];
-  const int tile=P.tile, L=P.L, Nh=P.N/2;
+  const T half=(T) 0.5;
+  const cplx<T> zb=conjg(zm);
+  const cplx<T> e=(zk+zb)*half, dd=zk-zb;
+  const cplx<T> o=mk(dd.y*half,-dd.x*half);
+  if constexpr(std::is_same<T,double>::value) {
+    F=fmaTw<1>(e,o,w);
+    Fc=mk(fma((T) 2,e.x,-F.x),fma((T) -2,e.y,F.y));
+  } else {
+    const cplx<T> q=twmul<1>(o,w);
+    F=e+q;
+    Fc=conjg(e-q);
+  }
+}
+
+// Y[k] = s + i d and Y[Nh-k] = conj(s - i d) from G[k] and G[Nh-k], s = G[k]
+// + conj G[Nh-k], d = W_N^{-k} (G[k] - conj G[Nh-k]).
+template<typename T>
+__device__ __forceinline__ void realPack(cplx<T> gk, cplx<T> gm,
+                                         typename TwT<T>::type w,
+                                         cplx<T>& Y, cplx<T>& Yc)
+{
+  const cplx<T> gb=conjg(gm);
+  const cplx<T> s=gk+gb;
+  const cplx<T> d=twmul<-1>(gk-gb,w);
+  Y=mk(s.x-d.y,s.y+d.x);
+  Yc=mk(s.x+d.y,d.x-s.y);
+}
+
+template<typename T, int R>
+__device__ __forceinline__ void realLastFwd(const OuterPlan<T>& P,
+                                            const cplx<T> *x, cplx<T> *dst,
+                                            int col0, int tid, int nthr)
+{
+  typedef typename TwT<T>::type Tw;
+  const FusedFFT& p=P.fz;
+  const int lt=log2of(P.tile), Nh=p.n, nblk=Nh/R, total=(nblk+1)/2 << lt;
+  const Tw *tw=(const Tw *) p.twb+(nblk-p.radix[0]);
+#pragma unroll 1
+  for(int idx=tid; idx < total; idx += nthr) {
+    const int i=idx >> lt, cc=idx & (P.tile-1), col=col0+cc;
+    const int4 pr=__ldg(p.pairs+i);
+    const int b=pr.x, b2=max(pr.y,0), kappa=pr.z;
+    cplx<T> u[1][R], v[1][R];
+    const cplx<T> *xq=x+(spl(b*R,p.lg) << lt)+cc;
+    const cplx<T> *xr=x+(spl(b2*R,p.lg) << lt)+cc;
+#pragma unroll
+    for(int r=0; r < R; ++r) {
+      u[0][r]=nrm(xq[r << lt]);
+      v[0][r]=nrm(xr[r << lt]);
+    }
+    inTwiddleDFT<T,R,1>(u,tw,b,nblk);
+    inTwiddleDFT<T,R,1>(v,tw,b2,nblk);
+    if(col >= P.C) continue;
+    cplx<T> *d=dst+col;
+    const int top=P.kc > 0 ? P.kc : Nh+1;
+    auto put=[&](int k, cplx<T> f) {
+      if(k < top) d[(long long) k*P.outRow]=P.conj ? conjg(f) : f;
+    };
+    cplx<T> F, Fc;
+    if(i != 0) {
+#pragma unroll
+      for(int r=0; r < R; ++r) {
+        const int k=kappa+r*nblk;
+        realUnpack(u[0][r],v[0][R-1-r],ldtw(P.twN+k),F,Fc);
+        put(k,F);
+        put(Nh-k,Fc);
+      }
+    } else {
+#pragma unroll
+      for(int r=0; r <= R/2; ++r) {
+        realUnpack(u[0][r],u[0][(R-r)%R],ldtw(P.twN+r*nblk),F,Fc);
+        put(r*nblk,F);
+        if(2*r < R) put(Nh-r*nblk,Fc);
+      }
+      if(pr.y >= 0) {
+#pragma unroll
+        for(int r=0; r < (R+1)/2; ++r) {
+          const int k=nblk/2+r*nblk;
+          realUnpack(v[0][r],v[0][R-1-r],ldtw(P.twN+k),F,Fc);
+          put(k,F);
+          if(2*r < R-1) put(Nh-k,Fc);
+        }
+      }
+    }
+  }
+}
+
+template<typename T, bool WIDE>
+__device__ __forceinline__ void outerRealFwd(const OuterPlan<T>& P,
+                                             unsigned char *smemRaw)
+{
+  const int tile=P.tile, L=P.L;
   cplx<T> *x=(cplx<T> *) smemRaw;
-  cplx<T> *y=x+padded(Nh*tile);
   const int tid=threadIdx.x, nthr=blockDim.x;
   const int col0=blockIdx.x*tile;
   const int a=blockIdx.z % P.count;
   const long long batch=blockIdx.z/P.count;
   const T *src=(const T *) P.in[a]+batch*P.inBatch;
   cplx<T> *dst=P.out[a]+batch*P.outBatch;
-  const typename TwT<T>::type *tw=P.twN;
-  const T half=(T) 0.5;
-  const UDiv dTile(tile);
-
-  for(int i=tid; i < Nh*tile; i += nthr) {
-    int t=dTile(i), cc=i-t*tile;
-    int col=col0+cc;
-    T re=(T) 0, im=(T) 0;
-    if(col < P.C) {
-      int s=2*t;
-      const long long dc=dataCol(P,col);
-      const int sh=ioShift<T>(P.ioShift,a);
-      if(s < L) re=loadIOr(src+(long long) s*P.inRow+dc,P.io64 & 1,sh);
-      if(s+1 < L) im=loadIOr(src+(long long) (s+1)*P.inRow+dc,P.io64 & 1,sh);
+  const int lt=log2of(tile);
+  const int sh=ioShift<T>(P.ioShift,a);
+  const auto load=[&](int, int cc) {
+    const int top=col0+cc < P.C ? L : 0;
+    const T *f=src+dataCol(P,col0+cc);
+    return [=,&P](int j) {
+      const int s=2*j;
+      cplx<T> v=mk((T) 0,(T) 0);
+      if(s < top) v.x=loadIOr(f+s*P.inRow,P.io64 & 1,sh);
+      if(s+1 < top) v.y=loadIOr(f+(s+1)*P.inRow,P.io64 & 1,sh);
+      return v;
+    };
+  };
+  if constexpr(std::is_same<T,ff>::value) {
+    loadTileFF(x,P.fz,lt,tid,nthr,[&](int cc, int j) {
+        const int s=2*j, top=col0+cc < P.C ? L : 0;
+        const T *f=src+dataCol(P,col0+cc);
+        cplx<T> v=mk((T) 0,(T) 0);
+        if(s < top) {
+          v.x=f[s*P.inRow];
+          if(s+1 < top) v.y=f[(s+1)*P.inRow];
+          if(P.io64 & 1) v=fromBits(v,sh);
+        }
+        return v;
+      });
+    runStages<T>(x,0,1,0,P.fz,lt,0,0,tid,nthr,[] {});
+    const int Nh=P.N/2, top=P.kc > 0 ? P.kc : Nh+1;
+#pragma unroll 2
+    for(int idx=tid; idx < (Nh/2+1) << lt; idx += nthr) {
+      const int k=idx >> lt, cc=idx & (tile-1), kk=Nh-k;
+      if(col0+cc >= P.C) continue;
+      cplx<T> *d=dst+col0+cc, F, Fc;
+      const cplx<T> zk=x[(spl(P.fz.pos[k],P.fz.lg) << lt)+cc];
+      const cplx<T> zm=x[(spl(P.fz.pos[k == 0 ? 0 : kk],P.fz.lg) << lt)+cc];
+      realUnpack(zk,zm,ldtw(P.twN+k),F,Fc);
+      if(k < top) d[k*P.outRow]=P.conj ? conjg(F) : F;
+      if(kk != k && kk < top) d[kk*P.outRow]=P.conj ? conjg(Fc) : Fc;
     }
-    x[sp(i)]=mk(re,im);
+    return;
   }
+  runFusedFirst<T,WIDE>(x,0,1,P.fz,lt,tid,nthr,load);
+  runFusedMiddle<T,WIDE>(x,0,1,P.fz,lt,false,0,tid,nthr);
   __syncthreads();
-  cplx<T> *X=fftSmem<T,1>(x,y,P.fp,tile,tile,tid,nthr);
-  for(int i=tid; i < (Nh+1)*tile; i += nthr) {
-    int k=dTile(i), cc=i-k*tile;
-    int col=col0+cc;
-    if(col >= P.C) continue;
-    if(P.kc > 0 && k >= P.kc) continue;
-    int k0=k == Nh ? 0 : k;
-    int km=k == 0 || k == Nh ? 0 : Nh-k;
-    cplx<T> zk=X[sp(k0*tile+cc)];
-    cplx<T> zm=conjg(X[sp(km*tile+cc)]);
-    cplx<T> e=(zk+zm)*half;
-    cplx<T> dd=zk-zm;
-    cplx<T> o=mk(dd.y*half,-dd.x*half);
-    cplx<T> v;
-    if(k == Nh) v=e-o;
-    else v=e+twmul<1>(o,tw[k]);
-    dst[(long long) k*P.outRow+col]=P.conj ? conjg(v) : v;
+  FGB_FUSED_SWITCH(P.fz.radix[P.fz.nst-1],
+                   (realLastFwd<T,R_>(P,x,dst,col0,tid,nthr)))
+}
+
+template<typename T, int R>
+__device__ __forceinline__ void realFirstInv(const OuterPlan<T>& P,
+                                             cplx<T> *x, const cplx<T> *src,
+                                             int col0, int tid, int nthr)
+{
+  const FusedFFT& p=P.fz;
+  const int lt=log2of(P.tile), Nh=p.n, nblk=Nh/R, total=(nblk+1)/2 << lt;
+  const int top=P.kc > 0 ? P.kc : Nh+1;
+#pragma unroll 1
+  for(int idx=tid; idx < total; idx += nthr) {
+    const int i=idx >> lt, cc=idx & (P.tile-1), col=col0+cc;
+    const int4 pr=__ldg(p.pairs+i);
+    const int b=pr.x, b2=max(pr.y,0), kappa=pr.z;
+    const int kappa2=i == 0 ? nblk/2 : nblk-kappa;
+    auto get=[&](int k) {
+      cplx<T> g=mk((T) 0,(T) 0);
+      if(col < P.C && k < top) g=src[(long long) k*P.inRow+col];
+      return P.conj ? conjg(g) : g;
+    };
+    cplx<T> g[R], h[R], u[R], v[R];
+#pragma unroll
+    for(int r=0; r < R; ++r) {
+      g[r]=get(kappa+r*nblk);
+      h[r]=get(kappa2+r*nblk);
+    }
+    if(i != 0) {
+#pragma unroll
+      for(int r=0; r < R; ++r)
+        realPack(g[r],h[R-1-r],ldtw(P.twN+kappa+r*nblk),u[r],v[R-1-r]);
+    } else {
+      cplx<T> dummy, gN=get(Nh);
+      g[0].y=gN.y=(T) 0;
+      realPack(g[0],gN,ldtw(P.twN),u[0],dummy);
+#pragma unroll
+      for(int r=1; r <= R/2; ++r)
+        realPack(g[r],g[R-r],ldtw(P.twN+r*nblk),u[r],
+                 2*r == R ? dummy : u[R-r]);
+#pragma unroll
+      for(int r=0; r < (R+1)/2; ++r)
+        realPack(h[r],h[R-1-r],ldtw(P.twN+nblk/2+r*nblk),v[r],
+                 2*r == R-1 ? dummy : v[R-1-r]);
+    }
+#pragma unroll
+    for(int r=0; r < R; ++r) {
+      u[r]=nrm(swapXY(u[r]));
+      v[r]=nrm(swapXY(v[r]));
+    }
+    Codelet<R,1,T>::run(u);
+    Codelet<R,1,T>::run(v);
+    cplx<T> *xq=x+(spl(b*R,p.lg) << lt)+cc;
+    cplx<T> *xr=x+(spl(b2*R,p.lg) << lt)+cc;
+#pragma unroll
+    for(int r=0; r < R; ++r) xq[r << lt]=u[r];
+    if(pr.y >= 0) {
+#pragma unroll
+      for(int r=0; r < R; ++r) xr[r << lt]=v[r];
+    }
   }
 }
 
-// Outer backward, real data: Hermitian-extend the N/2+1 modes, pack
-// Y[k] = (G[k] + conj G[Nh-k]) + i W_N^{-k} (G[k] - conj G[Nh-k]), sign -1
-// FFT of length N/2, unpack h[2t] = Re y[t], h[2t+1] = Im y[t].
-template<typename T>
-__global__ void __launch_bounds__(256)
-outerRealBwdKernel(const OuterPlan<T> P)
+template<typename T, bool WIDE>
+__device__ __forceinline__ void outerRealBwd(const OuterPlan<T>& P,
+                                             unsigned char *smemRaw)
 {
-  extern __shared__ __align__(16) unsigned char smemRaw[];
-  const int tile=P.tile, L=P.L, Nh=P.N/2;
+  const int tile=P.tile, L=P.L;
   cplx<T> *x=(cplx<T> *) smemRaw;
-  cplx<T> *y=x+padded(Nh*tile);
   const int tid=threadIdx.x, nthr=blockDim.x;
   const int col0=blockIdx.x*tile;
   const int b=blockIdx.z % P.count;
   const long long batch=blockIdx.z/P.count;
   const cplx<T> *src=P.in[b]+batch*P.inBatch;
   T *dst=(T *) P.out[b]+batch*P.outBatch;
-  const typename TwT<T>::type *tw=P.twN;
-  const UDiv dTile(tile);
-
-  for(int i=tid; i < Nh*tile; i += nthr) {
-    int k=dTile(i), cc=i-k*tile;
-    int col=col0+cc;
-    cplx<T> v=mk((T) 0,(T) 0);
-    if(col < P.C) {
-      const int kc=P.kc > 0 ? P.kc : Nh+1;
-      cplx<T> gk=k < kc ? src[(long long) k*P.inRow+col] : mk((T) 0,(T) 0);
-      cplx<T> gm=Nh-k < kc ? src[(long long) (Nh-k)*P.inRow+col] :
-        mk((T) 0,(T) 0);
+  const int lt=log2of(tile);
+  const int sh=ioShift<T>(P.ioShift,8+b);
+  const auto store=[&](int, int cc) {
+    const int top=col0+cc < P.C ? L : 0;
+    T *f=dst+dataCol(P,col0+cc);
+    return [=,&P](int j, cplx<T> v) {
+      const int s=2*j;
+      v=v*P.scale;
+      if(s < top) storeIOr(f+s*P.outRow,v.x,P.io64 & 2,sh);
+      if(s+1 < top) storeIOr(f+(s+1)*P.outRow,v.y,P.io64 & 2,sh);
+    };
+  };
+  if constexpr(std::is_same<T,ff>::value) {
+    const int Nh=P.N/2, top=P.kc > 0 ? P.kc : Nh+1;
+#pragma unroll 2
+    for(int idx=tid; idx < (Nh/2+1) << lt; idx += nthr) {
+      const int k=idx >> lt, cc=idx & (tile-1), kk=Nh-k;
+      cplx<T> gk=mk((T) 0,(T) 0), gm=gk, Y, Yc;
+      if(col0+cc < P.C) {
+        const cplx<T> *g=src+col0+cc;
+        if(k < top) gk=g[k*P.inRow];
+        if(kk < top) gm=g[kk*P.inRow];
+      }
       if(P.conj) {
         gk=conjg(gk);
         gm=conjg(gm);
       }
-      if(k == 0) gk.y=(T) 0;
-      if(k == 0) gm.y=(T) 0;
-      gm=conjg(gm);
-      cplx<T> s=gk+gm;
-      cplx<T> d=twmul<-1>(gk-gm,tw[k]);
-      v=mk(s.x-d.y,s.y+d.x);
+      if(k == 0) gk.y=gm.y=(T) 0;
+      realPack(gk,gm,ldtw(P.twN+k),Y,Yc);
+      x[(spl(P.fz.pos[k],P.fz.lg) << lt)+cc]=swapXY(Y);
+      if(k != 0 && kk != k)
+        x[(spl(P.fz.pos[kk],P.fz.lg) << lt)+cc]=swapXY(Yc);
     }
-    x[sp(i)]=v;
+    runStages<T>(x,0,0,1,P.fz,lt,0,0,tid,nthr,[] {});
+    storeTileFF(x,P.fz,lt,tid,nthr,store);
+    return;
   }
+  FGB_FUSED_SWITCH(P.fz.radix[P.fz.nst-1],
+                   (realFirstInv<T,R_>(P,x,src,col0,tid,nthr)))
+  runFusedMiddle<T,WIDE>(x,0,1,P.fz,lt,true,0,tid,nthr);
   __syncthreads();
-  cplx<T> *X=fftSmem<T,-1>(x,y,P.fp,tile,tile,tid,nthr);
-  for(int i=tid; i < Nh*tile; i += nthr) {
-    int t=dTile(i), cc=i-t*tile;
-    int col=col0+cc;
-    if(col >= P.C) continue;
-    cplx<T> v=X[sp(i)]*P.scale;
-    int s=2*t;
-    const long long dc=dataCol(P,col);
-    const int sh=ioShift<T>(P.ioShift,8+b);
-    if(s < L) storeIOr(dst+(long long) s*P.outRow+dc,v.x,P.io64 & 2,sh);
-    if(s+1 < L) storeIOr(dst+(long long) (s+1)*P.outRow+dc,v.y,P.io64 & 2,sh);
-  }
+  runFusedLast<T,WIDE>(x,0,1,P.fz,lt,tid,nthr,store);
+}
+
+template<typename T, bool WIDE>
+__global__ void __launch_bounds__(256,2)
+outerRealFwdKernel(const OuterPlan<T> P)
+{
+  extern __shared__ __align__(16) unsigned char smemRaw[];
+  outerRealFwd<T,WIDE>(P,smemRaw);
+}
+
+template<typename T, bool WIDE>
+__global__ void __launch_bounds__(256,2)
+outerRealBwdKernel(const OuterPlan<T> P)
+{
+  extern __shared__ __align__(16) unsigned char smemRaw[];
+  outerRealBwd<T,WIDE>(P,smemRaw);
 }
 
 // ---------------------------------------------------------------------------
@@ -513,11 +896,17 @@ batchKernel(const BatchArgs<T> P)
         rebase(R,R.A,rel & 1,rel & 2,P.inBase,P.outBase);
       __syncthreads();
       const BuiltinMult<K> mul;
-      if(tk.type == TASK_SMALL)
-        rowConvRow<T,false,BuiltinMult<K>>(R,tk.i,smemRaw,mul);
-      else if(R.direct)
-        rowConvRow<T,true,BuiltinMult<K>,true>(R,tk.i,smemRaw,mul);
-      else rowConvRow<T,true,BuiltinMult<K>>(R,tk.i,smemRaw,mul);
+      if(R.direct) {
+        // Fused rows, R.rpc of them one after another by teams.
+        const int nt=blockDim.x/R.nteam;
+        const int team=threadIdx.x/nt, th=threadIdx.x-team*nt;
+        const int cs=fusedSpan(R.fz.n,R.fz.lg);
+        cplx<T> *x=(cplx<T> *) smemRaw+team*R.A*cs;
+        for(int rho=team; rho < R.rpc; rho += R.nteam)
+          fusedRow<T,true,false>(R,mul,x,cs,(long long) tk.i*R.rpc+rho,team,
+                                 th,nt);
+        __syncthreads();
+      } else rowConvRow<T,false,BuiltinMult<K>>(R,tk.i,smemRaw,mul);
     } else {
       const bool fwd=tk.type == TASK_COLFWD;
       OuterPlan<T>& O=stagePlan(planBuf,fwd ? B->fwd : B->bwd);
@@ -592,30 +981,21 @@ int batchBlocksPerSM(int threads, size_t smem, int mult, int A, int B)
 
 // Shared-memory bytes: FFT ping-pong buffers are padded (sp()); the forward
 // outer kernel also stages its L x tile input block in the second buffer.
-template<typename T> size_t rowSmem(int L, int m, int A, int B, int rpc,
-                                    int direct)
-{
-  size_t nbuf=inplaceFFT<T>() || direct ? 1 : 2;
-  size_t stage=direct ? 0 : (size_t) (A+B)*rpc*L;
-  return sizeof(cplx<T>)*(stage+nbuf*(size_t) padded(m*A*rpc));
-}
-template<typename T> size_t hermRowSmem(int H, int Nh, int A, int rpc)
+template<typename T> size_t rowSmem(int L, int m, int A, int B, int rpc)
 {
   size_t nbuf=inplaceFFT<T>() ? 1 : 2;
-  return sizeof(cplx<T>)*nbuf*(size_t) padded(Nh*A*rpc);
+  return sizeof(cplx<T>)*((size_t) (A+B)*rpc*L+
+                          nbuf*(size_t) padded(m*A*rpc));
 }
-template<typename T> size_t outerFwdSmem(int L, int m, int tile, int inplace)
+template<typename T> size_t outerFwdSmem(int L, int m, int tile)
 {
   size_t pm=padded(m*tile);
-  if(inplaceFFT<T>() && inplace) return sizeof(cplx<T>)*pm;
   return sizeof(cplx<T>)*(pm+std::max(pm,(size_t) L*tile));
 }
-template<typename T> size_t outerBwdSmem(int L, int m, int tile, int q,
-                                         int inplace)
+template<typename T> size_t outerBwdSmem(int L, int m, int tile, int q)
 {
   size_t acc=q == 1 ? 0 : (size_t) L*tile;
-  size_t nbuf=inplaceFFT<T>() && inplace ? 1 : 2;
-  return sizeof(cplx<T>)*(acc+nbuf*(size_t) padded(m*tile));
+  return sizeof(cplx<T>)*(acc+2*(size_t) padded(m*tile));
 }
 template<typename T> size_t outerRealSmem(int L, int Nh, int tile)
 {
@@ -668,7 +1048,8 @@ cudaError_t launchHermRow(const HermRowPlan<T>& P, int threads,
 template<typename T>
 cudaError_t launchOuterFwd(const OuterPlan<T>& P, int threads, cudaStream_t s)
 {
-  size_t sm=outerFwdSmem<T>(P.L,P.m,P.tile,P.inplace);
+  size_t sm=P.fused ? fusedOuterSmem<T>(P.L,P.fz.n,P.fz.lg,P.tile,1) :
+    outerFwdSmem<T>(P.L,P.m,P.tile);
   dim3 grid((P.C+P.tile-1)/P.tile,P.q,P.nbatch*P.count);
   auto go=[&](auto kernel) {
     cudaError_t e=setSmem(kernel,sm);
@@ -676,15 +1057,42 @@ cudaError_t launchOuterFwd(const OuterPlan<T>& P, int threads, cudaStream_t s)
     kernel<<<grid,threads,sm,s>>>(P);
     return cudaGetLastError();
   };
-  if constexpr(std::is_same<T,float>::value)
-    if(P.inplace && hasWideRadix(P.fp)) return go(outerFwdKernel16<T>);
+  if(P.fused) {
+    if constexpr(std::is_same<T,float>::value)
+      if(wideFused(P.fz)) return go(outerFwdFusedKernel16<T>);
+    return go(outerFwdFusedKernel<T>);
+  }
   return go(outerFwdKernel<T>);
 }
 
 template<typename T>
 cudaError_t launchOuterBwd(const OuterPlan<T>& P, int threads, cudaStream_t s)
 {
-  size_t sm=outerBwdSmem<T>(P.L,P.m,P.tile,P.q,P.inplace);
+  size_t sm=P.fused ? fusedOuterSmem<T>(P.L,P.fz.n,P.fz.lg,P.tile,P.q) :
+    outerBwdSmem<T>(P.L,P.m,P.tile,P.q);
+  dim3 grid((P.C+P.tile-1)/P.tile,1,P.nbatch*P.count);
+  auto go=[&](auto kernel) {
+    cudaError_t e=setSmem(kernel,sm);
+    if(e != cudaSuccess) return e;
+    kernel<<<grid,threads,sm,s>>>(P);
+    return cudaGetLastError();
+  };
+  if(P.fused) {
+    if constexpr(std::is_same<T,float>::value)
+      if(wideFused(P.fz)) return go(outerBwdFusedKernel16<T>);
+    return go(outerBwdFusedKernel<T>);
+  }
+  return go(outerBwdKernel<T>);
+}
+
+// The real kernels take what two buffers of one element more per column
+// would hold, as planned.
+template<typename T>
+static cudaError_t launchOuterReal(const OuterPlan<T>& P, bool fwd,
+                                   int threads, cudaStream_t s)
+{
+  if(outerRealSmem<T>(P.L,P.N/2,1) > 227*1024) return cudaErrorInvalidValue;
+  const size_t sm=fusedOuterSmem<T>(P.L,P.fz.n,P.fz.lg,P.tile,1);
   dim3 grid((P.C+P.tile-1)/P.tile,1,P.nbatch*P.count);
   auto go=[&](auto kernel) {
     cudaError_t e=setSmem(kernel,sm);
@@ -693,50 +1101,61 @@ cudaError_t launchOuterBwd(const OuterPlan<T>& P, int threads, cudaStream_t s)
     return cudaGetLastError();
   };
   if constexpr(std::is_same<T,float>::value)
-    if(P.inplace && hasWideRadix(P.fp)) return go(outerBwdKernel16<T>);
-  return go(outerBwdKernel<T>);
+    if(wideFused(P.fz))
+      return fwd ? go(outerRealFwdKernel<T,true>) :
+        go(outerRealBwdKernel<T,true>);
+  return fwd ? go(outerRealFwdKernel<T,false>) :
+    go(outerRealBwdKernel<T,false>);
 }
 
 template<typename T>
 cudaError_t launchOuterRealFwd(const OuterPlan<T>& P, int threads,
                                cudaStream_t s)
 {
-  size_t sm=outerRealSmem<T>(P.L,P.N/2,P.tile);
-  cudaError_t e=setSmem(outerRealFwdKernel<T>,sm);
-  if(e != cudaSuccess) return e;
-  dim3 grid((P.C+P.tile-1)/P.tile,1,P.nbatch*P.count);
-  outerRealFwdKernel<T><<<grid,threads,sm,s>>>(P);
-  return cudaGetLastError();
+  return launchOuterReal(P,true,threads,s);
 }
 
 template<typename T>
 cudaError_t launchOuterRealBwd(const OuterPlan<T>& P, int threads,
                                cudaStream_t s)
 {
-  size_t sm=outerRealSmem<T>(P.L,P.N/2,P.tile);
-  cudaError_t e=setSmem(outerRealBwdKernel<T>,sm);
-  if(e != cudaSuccess) return e;
-  dim3 grid((P.C+P.tile-1)/P.tile,1,P.nbatch*P.count);
-  outerRealBwdKernel<T><<<grid,threads,sm,s>>>(P);
-  return cudaGetLastError();
+  return launchOuterReal(P,false,threads,s);
 }
 
-#define FGB_INSTANTIATE(T) \
-  template cudaError_t launchRow<T>(const RowPlan<T>&,int,long long,cudaStream_t); \
-  template cudaError_t launchHermRow<T>(const HermRowPlan<T>&,int,long long,cudaStream_t); \
-  template cudaError_t launchOuterFwd<T>(const OuterPlan<T>&,int,cudaStream_t); \
-  template cudaError_t launchOuterBwd<T>(const OuterPlan<T>&,int,cudaStream_t); \
-  template cudaError_t launchOuterRealFwd<T>(const OuterPlan<T>&,int,cudaStream_t); \
-  template cudaError_t launchOuterRealBwd<T>(const OuterPlan<T>&,int,cudaStream_t); \
-  template size_t rowSmem<T>(int,int,int,int,int,int); \
-  template size_t hermRowSmem<T>(int,int,int,int); \
-  template size_t outerFwdSmem<T>(int,int,int,int); \
-  template size_t outerBwdSmem<T>(int,int,int,int,int); \
-  template size_t outerRealSmem<T>(int,int,int); \
-  template cudaError_t launchBatch<T>(const BatchArgs<T>&,int,int,size_t,cudaStream_t); \
-  template int batchBlocksPerSM<T>(int,size_t,int,int,int);
+// build.py compiles this file once per precision (FGB_T) and kernel family
+// (FGB_PART), in parallel.
+#define FGB_ROWS 1
+#define FGB_HERM 2
+#define FGB_OUTER 3
+#define FGB_BATCH 4
+#define FGB_MISC 5
+#define FGB_REAL_OUTER 6
 
-#if !defined(FGB_ONLY_FLOAT) && !defined(FGB_ONLY_FF)
+#if FGB_PART == FGB_ROWS
+template cudaError_t launchRow<FGB_T>(const RowPlan<FGB_T>&,int,long long,
+                                      cudaStream_t);
+template size_t rowSmem<FGB_T>(int,int,int,int,int);
+#elif FGB_PART == FGB_HERM
+template cudaError_t launchHermRow<FGB_T>(const HermRowPlan<FGB_T>&,int,
+                                          long long,cudaStream_t);
+#elif FGB_PART == FGB_OUTER
+template cudaError_t launchOuterFwd<FGB_T>(const OuterPlan<FGB_T>&,int,
+                                           cudaStream_t);
+template cudaError_t launchOuterBwd<FGB_T>(const OuterPlan<FGB_T>&,int,
+                                           cudaStream_t);
+template size_t outerFwdSmem<FGB_T>(int,int,int);
+template size_t outerBwdSmem<FGB_T>(int,int,int,int);
+#elif FGB_PART == FGB_REAL_OUTER
+template cudaError_t launchOuterRealFwd<FGB_T>(const OuterPlan<FGB_T>&,int,
+                                               cudaStream_t);
+template cudaError_t launchOuterRealBwd<FGB_T>(const OuterPlan<FGB_T>&,int,
+                                               cudaStream_t);
+template size_t outerRealSmem<FGB_T>(int,int,int);
+#elif FGB_PART == FGB_BATCH
+template cudaError_t launchBatch<FGB_T>(const BatchArgs<FGB_T>&,int,int,size_t,
+                                        cudaStream_t);
+template int batchBlocksPerSM<FGB_T>(int,size_t,int,int,int);
+#else
 // Bulk copy by the SMs (16-byte vectors, four in flight per thread): between
 // page-locked host memory and the device it reads and writes whole lines
 // over the host link.
@@ -922,20 +1341,6 @@ cudaError_t launchBulkCopy(const CopyArgs& P, cudaStream_t s)
   bulkCopyKernel<<<152*8,256,0,s>>>(P);
   return cudaGetLastError();
 }
-#endif
-
-// Each precision may be compiled as its own translation unit (build.py
-// compiles this file once per precision, in parallel): FGB_ONLY_<P> keeps
-// one of DOUBLE, FLOAT and FF.
-#if !defined(FGB_ONLY_FLOAT) && !defined(FGB_ONLY_FF)
-FGB_INSTANTIATE(double)
-#endif
-#if !defined(FGB_ONLY_DOUBLE) && !defined(FGB_ONLY_FF)
-FGB_INSTANTIATE(float)
-#endif
-#if !defined(FGB_ONLY_DOUBLE) && !defined(FGB_ONLY_FLOAT)
-FGB_INSTANTIATE(ff)
-
 #endif
 
 } // namespace fgb

@@ -23,15 +23,15 @@
 //    axis (fftPadReal) uses an explicit packed real FFT instead.
 #pragma once
 
-#include "fft_smem.cuh"
+#include "fft_fused.cuh"
 
 #include <type_traits>
 
 namespace fgb {
 
-// The row and outer kernels transform in place (fftDIF/fftDIT, one buffer)
-// on the FP32 pipe; the FP64 form keeps the ping-pong Stockham transform,
-// which measured faster on GB300's FP64 pipe.
+// Rows of several residues or folds transform in place (fftDIF/fftDIT, one
+// buffer) on the FP32 pipe; the FP64 form keeps the ping-pong Stockham
+// transform, which measured faster on GB300's FP64 pipe.
 template<typename T> __host__ __device__ constexpr bool inplaceFFT()
 {
   return !std::is_same<T,double>::value;
@@ -85,14 +85,15 @@ struct RowPlan {
   int rpc;                 // rows per CTA (their columns are interleaved)
   int io64;                // float-float mode: bit 0, in[] holds FP64
                            // values; bit 1, out[] takes FP64 values
-  int direct;              // one residue and one fold (q = 1, L <= m): rows
-                           // load straight into the transform buffer and
-                           // store straight from it (no staging, no
-                           // accumulator)
+  int direct;              // one residue and one fold (q = 1, L <= m): the
+                           // fused rows, transformed by fz (fp unused)
+  int nteam;               // fused rows: teams of threads per CTA (divides
+                           // rpc; a team convolves whole rows)
   const int *ioShift;      // float-float range guard: device exponents,
                            // [a] input a, [8+b] output b (NULL: none)
   T scale;
   FFTPlanDev fp;           // length-m complex FFT
+  FusedFFT fz;
   const typename TwT<T>::type *twN;   // W_N^t, t < N
   IndexMap im;             // slot positions (position-dependent multipliers)
 };
@@ -107,10 +108,11 @@ struct HermRowPlan {
   int N, Nh;               // real padded length (even) and N/2
   int A, B, mult;
   int rpc;                 // rows per CTA
+  int nteam;               // as RowPlan::nteam
   int io64;                // as RowPlan::io64
   const int *ioShift;      // as RowPlan::ioShift
   T scale;
-  FFTPlanDev fp;           // length-Nh complex FFT
+  FusedFFT fz;             // length-Nh complex FFT
   const typename TwT<T>::type *twN;   // W_N^t, t < N
   IndexMap im;             // slot positions (position-dependent multipliers)
 };
@@ -132,9 +134,9 @@ struct OuterPlan {
   int tile;
   int io64;                // as RowPlan::io64
   const int *ioShift;      // as RowPlan::ioShift
-  int inplace;             // FP32-pipe modes with L <= m and no twX: fold
-                           // from memory and transform in place, rows of
-                           // a residue block in digit-reversed order
+  int fused;               // L <= m and no twX: the fused kernels, with the
+                           // rows of a residue block in fz's digit-reversed
+                           // order
   int conj;                // real kernels: conjugate the complex side
                            // (the sign -1 r2c / sign +1 c2r of plain FFTs)
   int cz;                  // data side with strides: column c lies at
@@ -150,6 +152,7 @@ struct OuterPlan {
   long long flatC;
   T scale;
   FFTPlanDev fp;           // length-m (complex) or length-N/2 (real) FFT
+  FusedFFT fz;             // the fused kernels' length-m (N/2) FFT
   const typename TwT<T>::type *twN;
   const typename TwT<T>::type *twX;  // optional W_NX^{col*k} (1D long path)
   long long NX;
@@ -273,15 +276,23 @@ struct RowLaunchers {
 };
 
 // Shared-memory bytes each kernel needs (for plan-time sizing).
-template<typename T> size_t rowSmem(int L, int m, int A, int B, int rpc=1,
-                                    int direct=0);
-template<typename T> size_t hermRowSmem(int H, int Nh, int A, int rpc=1);
-template<typename T> size_t outerFwdSmem(int L, int m, int tile,
-                                         int inplace=0);
+template<typename T> size_t rowSmem(int L, int m, int A, int B, int rpc=1);
+template<typename T> size_t outerFwdSmem(int L, int m, int tile);
 // q == 1: the backward writes its outputs without an accumulator; q = 0
 // sizes for any residue count.
-template<typename T> size_t outerBwdSmem(int L, int m, int tile, int q=0,
-                                         int inplace=0);
+template<typename T> size_t outerBwdSmem(int L, int m, int tile, int q=0);
 template<typename T> size_t outerRealSmem(int L, int Nh, int tile);
+// Fused kernels: nteam rows of A columns; a tile of columns (and, backward
+// with several residues, its accumulator).
+template<typename T> size_t fusedRowSmem(int n, int lg, int A, int nteam)
+{
+  return sizeof(cplx<T>)*(size_t) nteam*A*fusedSpan(n,lg);
+}
+template<typename T> size_t fusedOuterSmem(int L, int n, int lg, int tile,
+                                           int q)
+{
+  return sizeof(cplx<T>)*((size_t) fusedSpan(n,lg)*tile+
+                          (q > 1 ? (size_t) L*tile : 0));
+}
 
 } // namespace fgb

@@ -84,6 +84,10 @@ template<> struct MultArity<MULT_REALBINARY> {static const int A=2, B=1;};
 template<> struct MultArity<MULT_REALJACOBIAN> {static const int A=4, B=1;};
 template<> struct MultArity<MULT_REALJACADJ> {static const int A=5, B=4;};
 
+// Values in and out of a multiplier type, 0 where they are known only at run
+// time.
+template<class Mul> struct MulArity;
+
 // Multiply one transformed slot: the A values at X[sp(base+a*stride)] in,
 // the B results back to X[sp(base+b*stride)].
 template<int K, typename T>
@@ -129,6 +133,12 @@ inline int multVariant(int mult, int A, int B)
 
 template<int K> struct BuiltinMult {
   static constexpr bool positional=false;
+  // A slot held in registers (fixed arity).
+  template<typename T>
+  __device__ __forceinline__ void slot(cplx<T> *v) const
+  {
+    applyMult(K,v,MultArity<K>::A);
+  }
   template<typename T>
   __device__ __forceinline__ void operator()(cplx<T> *X, int base, int stride,
                                              int A, int B, int kind) const
@@ -210,6 +220,28 @@ __device__ __forceinline__ ff nrmS(ff a) {return nrm(a);}
 template<class F> struct UserMult {
   static constexpr bool positional=true;
   F f;
+  // A slot held in registers; the two real grid points k and k+1 of one.
+  template<typename T>
+  __device__ __forceinline__ void slot(cplx<T> *v, const Indices& ix) const
+  {
+    f(v,ix);
+  }
+  template<typename T>
+  __device__ __forceinline__ void slotReal(cplx<T> *v, Indices ix, int k) const
+  {
+    T u[F::A], w[F::A];
+#pragma unroll
+    for(int a=0; a < F::A; ++a) {
+      u[a]=v[a].x;
+      w[a]=v[a].y;
+    }
+    ix.index[ix.dim-1]=k;
+    f(u,ix);
+    ix.index[ix.dim-1]=k+1;
+    f(w,ix);
+#pragma unroll
+    for(int b=0; b < F::B; ++b) v[b]=mk(u[b],w[b]);
+  }
   template<typename T>
   __device__ __forceinline__ void at(cplx<T> *X, int base, int stride,
                                      const Indices& ix) const
@@ -221,25 +253,13 @@ template<class F> struct UserMult {
 #pragma unroll
     for(int b=0; b < F::B; ++b) X[sp(base+b*stride)]=v[b];
   }
-  // The two real grid points k and k+1 held by one complex slot.
-  template<typename T>
-  __device__ __forceinline__ void atReal(cplx<T> *X, int base, int stride,
-                                         Indices ix, int k) const
-  {
-    T u[F::A], w[F::A];
-#pragma unroll
-    for(int a=0; a < F::A; ++a) {
-      const cplx<T> c=X[sp(base+a*stride)];
-      u[a]=nrmS(c.x);
-      w[a]=nrmS(c.y);
-    }
-    ix.index[ix.dim-1]=k;
-    f(u,ix);
-    ix.index[ix.dim-1]=k+1;
-    f(w,ix);
-#pragma unroll
-    for(int b=0; b < F::B; ++b) X[sp(base+b*stride)]=mk(u[b],w[b]);
-  }
+};
+
+template<int K> struct MulArity<BuiltinMult<K>> {
+  static constexpr int A=MultArity<K>::A, B=MultArity<K>::B;
+};
+template<class F> struct MulArity<UserMult<F>> {
+  static constexpr int A=F::A, B=F::B;
 };
 
 // One slot of a complex row: entry j of residue r (REV: j in the
@@ -265,19 +285,37 @@ __device__ __forceinline__ void mulRowSlot(const Mul& mul, const RowPlan<T>& P,
   }
 }
 
-// One slot t of a Hermitian row (real grid points 2t and 2t+1).
-template<class Mul, bool REV, typename T>
-__device__ __forceinline__ void mulHermSlot(const Mul& mul,
-                                            const HermRowPlan<T>& P,
-                                            cplx<T> *X, int base, int stride,
-                                            long long row, int t)
+// One slot of a fused row held in registers: entry p of the transform's
+// digit-reversed order, of row `row`.
+template<class Mul, typename T>
+__device__ __forceinline__ void mulFusedSlot(const Mul& mul,
+                                             const RowPlan<T>& P, cplx<T> *v,
+                                             long long row, int p)
 {
   if constexpr(Mul::positional) {
-    const int tn=REV ? digitRev(t,P.fp.n,P.fp.nst,P.fp.radix) : t;
-    mul.atReal(X,base,stride,outerIndices(P.im,row),2*tn);
-  } else {
-    mul(X,base,stride,P.A,P.B,P.mult);
-  }
+    const int jn=digitRev(p,P.fz.n,P.fz.nst,P.fz.radix);
+    int k=jn;
+    long long orow=row;
+    if(P.im.longQ > 0) {                 // long rows: column k1 of outer row
+      orow=row/P.im.longQ;
+      k=(int) (row-orow*P.im.longQ)+P.im.longQ*jn;
+    }
+    Indices ix=outerIndices(P.im,orow);
+    ix.index[P.im.dim-1]=k;
+    mul.slot(v,ix);
+  } else mul.slot(v);
+}
+
+// The same for a Hermitian row (real grid points 2t and 2t+1).
+template<class Mul, typename T>
+__device__ __forceinline__ void mulFusedSlot(const Mul& mul,
+                                             const HermRowPlan<T>& P,
+                                             cplx<T> *v, long long row, int p)
+{
+  if constexpr(Mul::positional) {
+    const int tn=digitRev(p,P.fz.n,P.fz.nst,P.fz.radix);
+    mul.slotReal(v,outerIndices(P.im,row),2*tn);
+  } else mul.slot(v);
 }
 
 // ---------------------------------------------------------------------------
@@ -352,16 +390,24 @@ __device__ __forceinline__ int ioShift(const int *sh, int io)
   else return 0;
 }
 
+// Both components, out of line: the fused stages convert at dozens of
+// places, and inlined there the conversion was most of their code.
+static __device__ __noinline__ cplx<ff> toFF2(double2 d, int sh)
+{
+  return mk(toFF(d.x,sh),toFF(d.y,sh));
+}
+
+static __device__ __noinline__ double2 fromFF2(cplx<ff> v, int sh)
+{
+  return make_double2(fromFF(v.x,sh),fromFF(v.y,sh));
+}
+
 template<typename T>
 __device__ __forceinline__ cplx<T> loadIO(const cplx<T> *p, bool f64,
                                           int sh=0)
 {
-  if constexpr(std::is_same<T,ff>::value) {
-    if(f64) {
-      double2 d=*(const double2 *) p;
-      return mk(toFF(d.x,sh),toFF(d.y,sh));
-    }
-  }
+  if constexpr(std::is_same<T,ff>::value)
+    if(f64) return toFF2(*(const double2 *) p,sh);
   return *p;
 }
 
@@ -379,7 +425,7 @@ __device__ __forceinline__ void storeIO(cplx<T> *p, cplx<T> v, bool f64,
 {
   if constexpr(std::is_same<T,ff>::value) {
     if(f64) {
-      *(double2 *) p=make_double2(fromFF(v.x,sh),fromFF(v.y,sh));
+      *(double2 *) p=fromFF2(v,sh);
       return;
     }
   }
@@ -510,7 +556,7 @@ __device__ __forceinline__ void cpAsyncWait()
 // together as interleaved columns col = a*rpc + rho, so the B x rpc output
 // columns are a contiguous prefix for the inverse transforms.  Every thread
 // of the block calls it.
-template<typename T, bool CG, class Mul, bool D=false, bool R16=false>
+template<typename T, bool CG, class Mul, bool R16=false>
 __device__ __forceinline__ void rowConvRow(const RowPlan<T>& P,
                                            long long group,
                                            unsigned char *smemRaw,
@@ -528,49 +574,61 @@ __device__ __forceinline__ void rowConvRow(const RowPlan<T>& P,
   const UDiv dR(R);
   const long long row0=group*R;
 
-  if constexpr(D) {
-    // One residue, one fold (RowPlan::direct; its own instantiation, so
-    // that the staged path's registers do not weigh on it or it on them): slot t of column col holds f[(t + c) mod m]
-    // (zero beyond L).  Reads run along each row (coalesced), FGB_LOADS
-    // iterations of loads issued before any is used.
-    cplx<T> *x=(cplx<T> *) smemRaw;
-    cplx<T> *y=x+padded(m*ld);
-    const UDiv dM(m);
-    for(int i0=tid; i0 < m*ld; i0 += FGB_LOADS*nthr) {
-      cplx<T> v[FGB_LOADS];
+  // The loads of FGB_LOADS iterations are issued before any is used.
+  for(int i0=tid; i0 < ld*L; i0 += FGB_LOADS*nthr) {
+    cplx<T> v[FGB_LOADS];
 #pragma unroll
-      for(int u=0; u < FGB_LOADS; ++u) {
-        const int i=i0+u*nthr;
-        v[u]=mk((T) 0,(T) 0);
-        if(i >= m*ld) continue;
-        int col=dM(i), s=i-col*m;
-        int a=dR(col);
-        long long row=row0+col-a*R;
-        if(s < L && row < P.nrows) {
-          long long off=row*P.rowStride+s;
-          if(P.realIO)
-            v[u]=mk(loadIOr((const T *) P.in[a]+off,P.io64 & 1,
-                            ioShift<T>(P.ioShift,a)),(T) 0);
-          else if(P.io64 & 1)
-            v[u]=loadIO(P.in[a]+off,true,ioShift<T>(P.ioShift,a));
-          else v[u]=ldx<CG>(P.in[a]+off);
+    for(int u=0; u < FGB_LOADS; ++u) {
+      const int i=i0+u*nthr;
+      v[u]=mk((T) 0,(T) 0);
+      if(i >= ld*L) continue;
+      int col=dL(i), s=i-col*L;
+      int a=dR(col);
+      long long row=row0+col-a*R;
+      if(row < P.nrows) {
+        long long off=row*P.rowStride+s;
+        if(P.realIO)
+          v[u]=mk(loadIOr((const T *) P.in[a]+off,P.io64 & 1,
+                          ioShift<T>(P.ioShift,a)),(T) 0);
+        else if(P.io64 & 1)
+          v[u]=loadIO(P.in[a]+off,true,ioShift<T>(P.ioShift,a));
+        else v[u]=ldx<CG>(P.in[a]+off);
+      }
+    }
+#pragma unroll
+    for(int u=0; u < FGB_LOADS; ++u)
+      if(i0+u*nthr < ld*L) fin[i0+u*nthr]=v[u];
+  }
+  for(int i=tid; i < lb*L; i += nthr) acc[i]=mk((T) 0,(T) 0);
+  __syncthreads();
+
+  for(int r=0; r < P.q; ++r) {
+    // Fold the data into one length-m block with the residue twiddles.
+    for(int i=tid; i < m*ld; i += nthr) {
+      int t=dLd(i), col=i-t*ld;
+      int s0=posmod(t+c,m);
+      cplx<T> sum=mk((T) 0,(T) 0);
+      // The twiddle exponent advances by m r mod N from term to term.
+      int e=r != 0 ? twExp(s0,c,r,N) : 0;
+      const int de=r != 0 ? twStep(m,r,N) : 0;
+      for(int s=s0; s < L; s += m) {
+        cplx<T> v=fin[col*L+s];
+        if(r != 0) {
+          v=twmul<1>(v,tw[e]);
+          e += de;
+          if(e >= N) e -= N;
         }
+        sum=accum(sum,v);
       }
-#pragma unroll
-      for(int u=0; u < FGB_LOADS; ++u) {
-        const int i=i0+u*nthr;
-        if(i >= m*ld) break;
-        int col=dM(i), s=i-col*m;
-        x[sp(posmod(s-c,m)*ld+col)]=v[u];
-      }
+      x[sp(i)]=sum;
     }
     __syncthreads();
     const cplx<T> *Z;
-    if constexpr(inplaceFFT<T>() || D) {
+    if constexpr(inplaceFFT<T>()) {
       fftDIF<T,1,R16>(x,P.fp,ld,ld,tid,nthr);
       for(int i=tid; i < m*R; i += nthr) {
         int j=dR(i), rho=i-j*R;
-        mulRowSlot<Mul,true>(mul,P,x,j*ld+rho,R,row0+rho,j,0);
+        mulRowSlot<Mul,true>(mul,P,x,j*ld+rho,R,row0+rho,j,r);
       }
       __syncthreads();
       fftDIT<T,-1,R16>(x,P.fp,lb,ld,tid,nthr);
@@ -580,138 +638,294 @@ __device__ __forceinline__ void rowConvRow(const RowPlan<T>& P,
       cplx<T> *Y=X == x ? y : x;
       for(int i=tid; i < m*R; i += nthr) {
         int j=dR(i), rho=i-j*R;
-        mulRowSlot<Mul,false>(mul,P,X,j*ld+rho,R,row0+rho,j,0);
+        mulRowSlot<Mul,false>(mul,P,X,j*ld+rho,R,row0+rho,j,r);
       }
       __syncthreads();
       Z=fftSmem<T,-1>(X,Y,P.fp,lb,ld,tid,nthr);
     }
     for(int i=tid; i < lb*L; i += nthr) {
       int col=dL(i), s=i-col*L;
-      int b=dR(col);
-      long long row=row0+col-b*R;
-      if(row >= P.nrows) continue;
-      cplx<T> v=Z[sp(posmod(s-c,m)*ld+col)];
-      long long off=row*P.rowStride+s;
-      const int sh=ioShift<T>(P.ioShift,8+b);
-      if(P.realIO) storeIOr((T *) P.out[b]+off,v.x*P.scale,P.io64 & 2,sh);
-      else storeIO(P.out[b]+off,v*P.scale,P.io64 & 2,sh);
-    }
-    __syncthreads();
-  } else {
-    // The loads of FGB_LOADS iterations are issued before any is used.
-    for(int i0=tid; i0 < ld*L; i0 += FGB_LOADS*nthr) {
-      cplx<T> v[FGB_LOADS];
-#pragma unroll
-      for(int u=0; u < FGB_LOADS; ++u) {
-        const int i=i0+u*nthr;
-        v[u]=mk((T) 0,(T) 0);
-        if(i >= ld*L) continue;
-        int col=dL(i), s=i-col*L;
-        int a=dR(col);
-        long long row=row0+col-a*R;
-        if(row < P.nrows) {
-          long long off=row*P.rowStride+s;
-          if(P.realIO)
-            v[u]=mk(loadIOr((const T *) P.in[a]+off,P.io64 & 1,
-                            ioShift<T>(P.ioShift,a)),(T) 0);
-          else if(P.io64 & 1)
-            v[u]=loadIO(P.in[a]+off,true,ioShift<T>(P.ioShift,a));
-          else v[u]=ldx<CG>(P.in[a]+off);
-        }
-      }
-#pragma unroll
-      for(int u=0; u < FGB_LOADS; ++u)
-        if(i0+u*nthr < ld*L) fin[i0+u*nthr]=v[u];
-    }
-    for(int i=tid; i < lb*L; i += nthr) acc[i]=mk((T) 0,(T) 0);
-    __syncthreads();
-
-    for(int r=0; r < P.q; ++r) {
-      // Fold the data into one length-m block with the residue twiddles.
-      for(int i=tid; i < m*ld; i += nthr) {
-        int t=dLd(i), col=i-t*ld;
-        int s0=posmod(t+c,m);
-        cplx<T> sum=mk((T) 0,(T) 0);
-        // The twiddle exponent advances by m r mod N from term to term.
-        int e=r != 0 ? twExp(s0,c,r,N) : 0;
-        const int de=r != 0 ? twStep(m,r,N) : 0;
-        for(int s=s0; s < L; s += m) {
-          cplx<T> v=fin[col*L+s];
-          if(r != 0) {
-            v=twmul<1>(v,tw[e]);
-            e += de;
-            if(e >= N) e -= N;
-          }
-          sum=accum(sum,v);
-        }
-        x[sp(i)]=sum;
-      }
-      __syncthreads();
-      const cplx<T> *Z;
-      if constexpr(inplaceFFT<T>()) {
-        fftDIF<T,1,R16>(x,P.fp,ld,ld,tid,nthr);
-        for(int i=tid; i < m*R; i += nthr) {
-          int j=dR(i), rho=i-j*R;
-          mulRowSlot<Mul,true>(mul,P,x,j*ld+rho,R,row0+rho,j,r);
-        }
-        __syncthreads();
-        fftDIT<T,-1,R16>(x,P.fp,lb,ld,tid,nthr);
-        Z=x;
-      } else {
-        cplx<T> *X=fftSmem<T,1>(x,y,P.fp,ld,ld,tid,nthr);
-        cplx<T> *Y=X == x ? y : x;
-        for(int i=tid; i < m*R; i += nthr) {
-          int j=dR(i), rho=i-j*R;
-          mulRowSlot<Mul,false>(mul,P,X,j*ld+rho,R,row0+rho,j,r);
-        }
-        __syncthreads();
-        Z=fftSmem<T,-1>(X,Y,P.fp,lb,ld,tid,nthr);
-      }
-      for(int i=tid; i < lb*L; i += nthr) {
-        int col=dL(i), s=i-col*L;
-        int t=posmod(s-c,m);
-        cplx<T> v=Z[sp(t*ld+col)];
-        if(r != 0) v=twmul<-1>(v,tw[twExp(s,c,r,N)]);
-        acc[i]=accum(acc[i],v);
-      }
-      __syncthreads();
-    }
-    for(int i=tid; i < lb*L; i += nthr) {
-      int col=dL(i), s=i-col*L;
-      int b=dR(col);
-      long long row=row0+col-b*R;
-      if(row >= P.nrows) continue;
-      long long off=row*P.rowStride+s;
-      const int sh=ioShift<T>(P.ioShift,8+b);
-      if(P.realIO)
-        storeIOr((T *) P.out[b]+off,acc[i].x*P.scale,P.io64 & 2,sh);
-      else storeIO(P.out[b]+off,acc[i]*P.scale,P.io64 & 2,sh);
+      int t=posmod(s-c,m);
+      cplx<T> v=Z[sp(t*ld+col)];
+      if(r != 0) v=twmul<-1>(v,tw[twExp(s,c,r,N)]);
+      acc[i]=accum(acc[i],v);
     }
     __syncthreads();
   }
+  for(int i=tid; i < lb*L; i += nthr) {
+    int col=dL(i), s=i-col*L;
+    int b=dR(col);
+    long long row=row0+col-b*R;
+    if(row >= P.nrows) continue;
+    long long off=row*P.rowStride+s;
+    const int sh=ioShift<T>(P.ioShift,8+b);
+    if(P.realIO)
+      storeIOr((T *) P.out[b]+off,acc[i].x*P.scale,P.io64 & 2,sh);
+    else storeIO(P.out[b]+off,acc[i]*P.scale,P.io64 & 2,sh);
+  }
+  __syncthreads();
 }
 
-template<typename T, class Mul, bool D>
+template<typename T, class Mul>
 __global__ void __launch_bounds__(256)
 rowConvKernel(const RowPlan<T> P, const Mul mul)
 {
   extern __shared__ __align__(16) unsigned char smemRaw[];
   const long long groups=(P.nrows+P.rpc-1)/P.rpc;
   for(long long g=blockIdx.x; g < groups; g += gridDim.x)
-    rowConvRow<T,false,Mul,D>(P,g,smemRaw,mul);
+    rowConvRow<T,false,Mul>(P,g,smemRaw,mul);
 }
 
 // The same for FP32 plans with a radix-16 stage: the radix-16 code needs
 // more registers, so only those plans launch it, capped at 85 registers a
 // thread (three CTAs of 256 threads per SM).
-template<typename T, class Mul, bool D>
+template<typename T, class Mul>
 __global__ void __launch_bounds__(256,3)
 rowConvKernel16(const RowPlan<T> P, const Mul mul)
 {
   extern __shared__ __align__(16) unsigned char smemRaw[];
   const long long groups=(P.nrows+P.rpc-1)/P.rpc;
   for(long long g=blockIdx.x; g < groups; g += gridDim.x)
-    rowConvRow<T,false,Mul,D,true>(P,g,smemRaw,mul);
+    rowConvRow<T,false,Mul,true>(P,g,smemRaw,mul);
+}
+
+// ---------------------------------------------------------------------------
+// Fused rows (fft_fused.cuh): one residue, one fold.  A CTA's threads form
+// teams of P.nteam-th parts; a team convolves whole rows on its own (its
+// own A columns of shared memory, its own barriers), so the rows of a CTA
+// do not wait for one another.
+
+// Values a middle stage may hold in registers: R of each of the A inputs.
+template<typename T, int A> __device__ constexpr bool fusedMiddle(int R)
+{
+  return R*A <= 20;
+}
+
+// The multiplier alone on every slot of a row (parts exchanged in the
+// results).
+template<typename T, class Mul, class Plan>
+__device__ __forceinline__ void fusedMulSlots(const Plan& P, const Mul& mul,
+                                              cplx<T> *x, int cs,
+                                              long long row, int t, int nt)
+{
+  constexpr int KA=MulArity<Mul>::A, KB=MulArity<Mul>::B;
+#pragma unroll 1
+  for(int i=t; i < P.fz.n; i += nt) {
+    cplx<T> *xi=x+spl(i,P.fz.lg);
+    if constexpr(KA > 0) {
+      cplx<T> v[KA];
+#pragma unroll
+      for(int c=0; c < KA; ++c) v[c]=nrm(xi[c*cs]);
+      mulFusedSlot(mul,P,v,row,i);
+#pragma unroll
+      for(int c=0; c < KB; ++c) xi[c*cs]=swapXY(v[c]);
+    } else {
+      cplx<T> v[FGB_MAXA];
+      for(int a=0; a < P.A; ++a) v[a]=nrm(xi[a*cs]);
+      applyMult(P.mult,v,P.A);
+      for(int b=0; b < P.B; ++b) xi[b*cs]=swapXY(v[b]);
+    }
+  }
+}
+
+// The last forward stage, the multiplier and the first inverse stage of one
+// row: every butterfly of radix R holds R neighbouring slots of all A
+// inputs, multiplies them in registers and transforms the B products back
+// (parts exchanged).
+template<typename T, int R, class Mul, class Plan>
+__device__ __forceinline__ void fusedMulStage(const Plan& P, const Mul& mul,
+                                              cplx<T> *x, int cs,
+                                              long long row, int t, int nt)
+{
+  constexpr int A=MulArity<Mul>::A, B=MulArity<Mul>::B;
+  typedef typename TwT<T>::type Tw;
+  const FusedFFT& p=P.fz;
+  const int nblk=p.n/R;
+  const Tw *tw=(const Tw *) p.twb+(nblk-p.radix[0]);
+#pragma unroll 1
+  for(int b=t; b < nblk; b += nt) {
+    cplx<T> *xq=x+spl(b*R,p.lg);
+    cplx<T> a[A][R];
+#pragma unroll
+    for(int c=0; c < A; ++c)
+#pragma unroll
+      for(int r=0; r < R; ++r) a[c][r]=nrm(xq[c*cs+r]);
+    inTwiddleDFT<T,R,A>(a,tw,b,nblk);
+#pragma unroll
+    for(int r=0; r < R; ++r) {
+      cplx<T> v[A];
+#pragma unroll
+      for(int c=0; c < A; ++c) v[c]=nrm(a[c][r]);
+      mulFusedSlot(mul,P,v,row,b*R+r);
+#pragma unroll
+      for(int c=0; c < B; ++c) a[c][r]=nrm(swapXY(v[c]));
+    }
+#pragma unroll
+    for(int c=0; c < B; ++c) {
+      Codelet<R,1,T>::run(a[c]);
+#pragma unroll
+      for(int r=0; r < R; ++r) xq[c*cs+r]=a[c][r];
+    }
+  }
+}
+
+// Everything between the first forward and the last inverse stage of a row
+// whose A columns lie cs apart at x; ends synchronised.
+template<typename T, bool WIDE, class Mul, class Plan>
+__device__ __forceinline__ void fusedRowInner(const Plan& P, const Mul& mul,
+                                              cplx<T> *x, int cs,
+                                              long long row, int team, int t,
+                                              int nt)
+{
+  constexpr int KA=MulArity<Mul>::A;
+  const FusedFFT& p=P.fz;
+  const int A=P.A, B=P.B;
+  if constexpr(std::is_same<T,ff>::value) {
+    runStages<T>(x,cs,A,B,p,0,1,team,t,nt,[&] {
+        fusedMulSlots(P,mul,x,cs,row,t,nt);
+      });
+  } else {
+    const int nblk=runFusedMiddle<T,WIDE>(x,cs,A,p,0,false,team,t,nt);
+    teamSync(team,nt);
+    bool fused=KA > 0;
+    if constexpr(KA >= 4) {
+      // A thread of the fused step takes A + B butterflies one after the
+      // other; on rows with fewer butterflies than threads the three steps
+      // spread them (FP64 Jacobian rows of 180 points).
+      const int per=(nblk+nt-1)/nt;
+      fused=per*(A+B) <= (A*nblk+nt-1)/nt+(B*nblk+nt-1)/nt+2;
+    }
+    if(fused) {
+      if constexpr(KA > 0) switch(p.radix[p.nst-1]) {
+        case 1: fusedMulStage<T,1>(P,mul,x,cs,row,t,nt); break;
+        case 2: fusedMulStage<T,2>(P,mul,x,cs,row,t,nt); break;
+        case 3: fusedMulStage<T,3>(P,mul,x,cs,row,t,nt); break;
+        case 4: fusedMulStage<T,4>(P,mul,x,cs,row,t,nt); break;
+        case 5:
+          if constexpr(fusedMiddle<T,KA>(5))
+            fusedMulStage<T,5>(P,mul,x,cs,row,t,nt);
+          break;
+        case 7:
+          if constexpr(fusedMiddle<T,KA>(7))
+            fusedMulStage<T,7>(P,mul,x,cs,row,t,nt);
+          break;
+        case 8:
+          if constexpr(fusedMiddle<T,KA>(8))
+            fusedMulStage<T,8>(P,mul,x,cs,row,t,nt);
+          break;
+        case 16:
+          if constexpr(WIDE && fusedMiddle<T,KA>(16))
+            fusedMulStage<T,16>(P,mul,x,cs,row,t,nt);
+          break;
+        default: break;
+      }
+    } else if constexpr(KA == 0 || KA >= 4) {
+      // Arity known at run time (or as above): the three steps one after the
+      // other.
+      typedef typename TwT<T>::type Tw;
+      const Tw *twb=(const Tw *) p.twb+(nblk-p.radix[0]);
+      const Tw *twj=(const Tw *) p.twj;
+      const int R=p.radix[p.nst-1];
+      FGB_FUSED_SWITCH(R,(fusedStage<T,R_>(x,cs,A,p,0,1,twb,nblk,false,t,
+                                             nt)))
+      teamSync(team,nt);
+      fusedMulSlots(P,mul,x,cs,row,t,nt);
+      teamSync(team,nt);
+      FGB_FUSED_SWITCH(R,(fusedStage<T,R_>(x,cs,B,p,0,1,twj,1,true,t,nt)))
+    }
+    runFusedMiddle<T,WIDE>(x,cs,B,p,0,true,team,t,nt);
+    teamSync(team,nt);
+  }
+}
+
+// One row of complex (or, realIO, real) data by a team.
+template<typename T, bool CG, bool WIDE, class Mul>
+__device__ __forceinline__ void fusedRow(const RowPlan<T>& P, const Mul& mul,
+                                         cplx<T> *x, int cs, long long row,
+                                         int team, int t, int nt)
+{
+  const int m=P.m, c=P.cshift;
+  const int top=row < P.nrows ? P.L : 0;   // entries of a row that exists
+  const long long off0=row*P.rowStride;
+  const auto load=[&](int a, int) {
+    const cplx<T> *f=P.in[a]+(P.realIO ? 0 : off0);
+    const T *fr=(const T *) P.in[a]+off0;
+    const int sh=ioShift<T>(P.ioShift,a);
+    return [=,&P](int j) {
+      int s=j+c;
+      if(s >= m) s -= m;
+      cplx<T> v=mk((T) 0,(T) 0);
+      if(s < top) {
+        if(P.realIO) v.x=loadIOr(fr+s,P.io64 & 1,sh);
+        else if(P.io64 & 1) v=loadIO(f+s,true,sh);
+        else v=ldx<CG>(f+s);
+      }
+      return v;
+    };
+  };
+  const auto store=[&](int b, int) {
+    cplx<T> *f=P.out[b]+(P.realIO ? 0 : off0);
+    T *fr=(T *) P.out[b]+off0;
+    const int sh=ioShift<T>(P.ioShift,8+b);
+    return [=,&P](int j, cplx<T> v) {
+      int s=j+c;
+      if(s >= m) s -= m;
+      if(s >= top) return;
+      if(P.realIO) storeIOr(fr+s,v.x*P.scale,P.io64 & 2,sh);
+      else storeIO(f+s,v*P.scale,P.io64 & 2,sh);
+    };
+  };
+  if(P.A*(m/P.fz.radix[0]) < nt) {
+    const ColumnMap cols(m);             // the staged form (runStages)
+#pragma unroll 2
+    for(int i=t; i < P.A*m; i += nt) {
+      const int a=cols(i), j=i-a*m;
+      x[a*cs+spl(j,P.fz.lg)]=load(a,0)(j);
+    }
+    runStages<T,WIDE>(x,cs,P.A,P.B,P.fz,0,0,team,t,nt,[&] {
+        fusedMulSlots(P,mul,x,cs,row,t,nt);
+      });
+    for(int i=t; i < P.B*m; i += nt) {
+      const int b=cols(i), j=i-b*m;
+      store(b,0)(j,swapXY(x[b*cs+spl(j,P.fz.lg)]));
+    }
+  } else {
+    runFusedFirst<T,WIDE>(x,cs,P.A,P.fz,0,t,nt,load);
+    fusedRowInner<T,WIDE>(P,mul,x,cs,row,team,t,nt);
+    runFusedLast<T,WIDE>(x,cs,P.B,P.fz,0,t,nt,store);
+  }
+  teamSync(team,nt);
+}
+
+template<typename T, class Mul, bool WIDE>
+__device__ __forceinline__ void fusedRows(const RowPlan<T>& P, const Mul& mul,
+                                          unsigned char *smemRaw)
+{
+  const int nt=blockDim.x/P.nteam;
+  const int team=threadIdx.x/nt, t=threadIdx.x-team*nt;
+  const int cs=fusedSpan(P.fz.n,P.fz.lg);
+  cplx<T> *x=(cplx<T> *) smemRaw+team*P.A*cs;
+  const long long groups=(P.nrows+P.rpc-1)/P.rpc;
+  for(long long g=blockIdx.x; g < groups; g += gridDim.x)
+    for(int rho=team; rho < P.rpc; rho += P.nteam)
+      fusedRow<T,false,WIDE>(P,mul,x,cs,g*P.rpc+rho,team,t,nt);
+}
+
+template<typename T, class Mul>
+__global__ void __launch_bounds__(256,fusedBlocks<T>())
+rowFusedKernel(const RowPlan<T> P, const Mul mul)
+{
+  extern __shared__ __align__(16) unsigned char smemRaw[];
+  fusedRows<T,Mul,false>(P,mul,smemRaw);
+}
+
+// FP32 plans with a radix-16 stage.
+template<typename T, class Mul>
+__global__ void __launch_bounds__(256,fusedBlocks<T>())
+rowFusedKernel16(const RowPlan<T> P, const Mul mul)
+{
+  extern __shared__ __align__(16) unsigned char smemRaw[];
+  fusedRows<T,Mul,true>(P,mul,smemRaw);
 }
 
 // ---------------------------------------------------------------------------
@@ -721,141 +935,279 @@ rowConvKernel16(const RowPlan<T> P, const Mul mul)
 // physical values as (u[2t], u[2t+1]) pairs; the multiplier acts on those
 // doubles; the sign -1 FFT of the packed product is unpacked into the H
 // output modes (real-to-complex).
-template<typename T, class Mul, bool R16>
+//
+// The packing pairs k with Nh-k, and butterfly j of the first stage (inputs
+// j + r m) holds exactly the partners of butterfly m-j, so one thread packs
+// and transforms both; the unpacking does the same behind the last stage.
+
+// Y[k] = S + i W_N^k D with S = Z[k] + conj Z[Nh-k], D = Z[k] -
+// conj Z[Nh-k], and its partner Y[Nh-k] = conj(S) + i conj(W_N^k D) (since
+// W_N^{Nh} = -1): one twiddle multiply for both.
+template<typename T>
+__device__ __forceinline__ void hermPack(cplx<T> zk, cplx<T> zc,
+                                         typename TwT<T>::type w,
+                                         cplx<T>& Y, cplx<T>& Yc)
+{
+  const cplx<T> b=conjg(zc);
+  const cplx<T> S=zk+b;
+  if constexpr(std::is_same<T,double>::value) {
+    // FP64: S + (i D) W as four DFMAs, the partner as conj(2S - Y).
+    const cplx<T> D=zk-b;
+    Y=fmaTw<1>(S,mk(-D.y,D.x),w);
+    Yc=mk(fma((T) 2,S.x,-Y.x),fma((T) -2,S.y,Y.y));
+  } else {
+    const cplx<T> Pw=twmul<1>(zk-b,w);
+    Y=mk(S.x-Pw.y,S.y+Pw.x);
+    Yc=mk(S.x+Pw.y,Pw.x-S.y);
+  }
+}
+
+// V[k] = hs (s + Q) with s = Z[k] + conj Z[Nh-k], Q = W_N^{-k} (-i)(Z[k] -
+// conj Z[Nh-k]), and V[Nh-k] = hs conj(s - Q); zm is Z[Nh-k] (Z[0] for
+// k = 0).
+template<typename T>
+__device__ __forceinline__ void hermUnpack(cplx<T> zk, cplx<T> zm, T hs,
+                                           typename TwT<T>::type w,
+                                           cplx<T>& V, cplx<T>& Vc)
+{
+  const cplx<T> zb=conjg(zm);
+  if constexpr(std::is_same<T,double>::value) {
+    // FP64: hs sum, hs dd = 2 hs zk - hs sum, V = hs sum + hs Q as four
+    // DFMAs, the partner as conj(2 hs sum - V).
+    const cplx<T> hsum=(zk+zb)*hs;
+    const T h2=hs+hs;
+    const cplx<T> hdd=mk(fma(h2,zk.x,-hsum.x),fma(h2,zk.y,-hsum.y));
+    V=fmaTw<-1>(hsum,mk(hdd.y,-hdd.x),w);
+    Vc=mk(fma((T) 2,hsum.x,-V.x),fma((T) -2,hsum.y,V.y));
+  } else {
+    const cplx<T> sum=zk+zb, dd=zk-zb;
+    const cplx<T> Q=twmul<-1>(mk(dd.y,-dd.x),w);
+    V=(sum+Q)*hs;
+    Vc=conjg(sum-Q)*hs;
+  }
+}
+
+// First stage of a row's inputs (cs apart at x0): butterflies j and m-j, or
+// 0 and m/2 (each its own partner; only 0 when m is odd), so ceil(m/2)
+// threads' worth an input.
+template<typename T, int R>
+__device__ __forceinline__ void hermFirst(const HermRowPlan<T>& P, cplx<T> *x0,
+                                          int cs, long long row, int t, int nt)
+{
+  const FusedFFT& p=P.fz;
+  const int H=row < P.nrows ? P.H : 0, m=P.Nh/R;
+  const StageMap map(R,m,p.lg,0);
+  const bool even=m % 2 == 0;
+  const ColumnMap cols((m+1)/2);
+#pragma unroll 1
+  for(int i=t; i < P.A*cols.per; i += nt) {
+    const int c=cols(i), j=i-c*cols.per;
+    cplx<T> *x=x0+c*cs;
+    const cplx<T> *z=P.in[c]+row*P.rowStride;
+    const int sh=ioShift<T>(P.ioShift,c);
+    const int j2=j == 0 ? m/2 : m-j;
+    cplx<T> a[R], b[R], u[R], v[R];
+#pragma unroll
+    for(int r=0; r < R; ++r) {
+      const int k=j+r*m, k2=j2+r*m;
+      a[r]=k < H ? loadIO(z+k,P.io64 & 1,sh) : mk((T) 0,(T) 0);
+      b[r]=k2 < H ? loadIO(z+k2,P.io64 & 1,sh) : mk((T) 0,(T) 0);
+    }
+    if(j != 0) {
+#pragma unroll
+      for(int r=0; r < R; ++r)
+        hermPack(a[r],b[R-1-r],ldtw(P.twN+j+r*m),u[r],v[R-1-r]);
+    } else {
+      cplx<T> dummy;
+      a[0].y=(T) 0;
+      hermPack(a[0],mk((T) 0,(T) 0),ldtw(P.twN),u[0],dummy);
+#pragma unroll
+      for(int r=1; r <= R/2; ++r)
+        hermPack(a[r],a[R-r],ldtw(P.twN+r*m),u[r],
+                 2*r == R ? dummy : u[R-r]);
+#pragma unroll
+      for(int r=0; r < (R+1)/2; ++r)
+        hermPack(b[r],b[R-1-r],ldtw(P.twN+m/2+r*m),v[r],
+                 2*r == R-1 ? dummy : v[R-1-r]);
+    }
+#pragma unroll
+    for(int r=0; r < R; ++r) {
+      u[r]=nrm(u[r]);
+      v[r]=nrm(v[r]);
+    }
+    Codelet<R,1,T>::run(u);
+    Codelet<R,1,T>::run(v);
+    cplx<T> *xq=x+map.offset(j,0,0), *xr=x+map.offset(j2,0,0);
+#pragma unroll
+    for(int r=0; r < R; ++r) xq[r*map.step]=u[r];
+    if(j != 0 || even) {
+#pragma unroll
+      for(int r=0; r < R; ++r) xr[r*map.step]=v[r];
+    }
+  }
+}
+
+// Last inverse stage of one output row, unpacked: the same pairs.
+template<typename T, int R>
+__device__ __forceinline__ void hermLast(const HermRowPlan<T>& P,
+                                         const cplx<T> *x0, int cs,
+                                         long long row, int t, int nt)
+{
+  const FusedFFT& p=P.fz;
+  const int Nh=P.Nh, H=row < P.nrows ? P.H : 0, m=Nh/R;
+  const StageMap map(R,m,p.lg,0);
+  const bool even=m % 2 == 0;
+  const T hs=(T) 0.5*P.scale;
+  const ColumnMap cols((m+1)/2);
+#pragma unroll 1
+  for(int i=t; i < P.B*cols.per; i += nt) {
+    const int c=cols(i), j=i-c*cols.per;
+    const cplx<T> *x=x0+c*cs;
+    cplx<T> *o=P.out[c]+row*P.rowStride;
+    const int sh=ioShift<T>(P.ioShift,8+c);
+    auto put=[&](int k, cplx<T> v) {
+      if(k < H) storeIO(o+k,v,P.io64 & 2,sh);
+    };
+    cplx<T> a[1][R], b[1][R];
+    const int j2=j == 0 ? m/2 : m-j;
+    const cplx<T> *xq=x+map.offset(j,0,0), *xr=x+map.offset(j2,0,0);
+#pragma unroll
+    for(int r=0; r < R; ++r) {
+      a[0][r]=nrm(xq[r*map.step]);
+      b[0][r]=nrm(xr[r*map.step]);
+    }
+    const typename TwT<T>::type *tw=(const typename TwT<T>::type *) p.twj+
+      (m-1);
+    inTwiddleDFT<T,R,1>(a,tw,j,m);
+    inTwiddleDFT<T,R,1>(b,tw,j2,m);
+#pragma unroll
+    for(int r=0; r < R; ++r) {
+      a[0][r]=swapXY(a[0][r]);
+      b[0][r]=swapXY(b[0][r]);
+    }
+    cplx<T> V, Vc;
+    if(j != 0) {
+#pragma unroll
+      for(int r=0; r < R; ++r) {
+        const int k=j+r*m;
+        if(k >= H && Nh-k >= H) continue;
+        hermUnpack(a[0][r],b[0][R-1-r],hs,ldtw(P.twN+k),V,Vc);
+        put(k,V);
+        put(Nh-k,Vc);
+      }
+    } else {
+#pragma unroll
+      for(int r=0; r <= R/2; ++r) {
+        hermUnpack(a[0][r],a[0][(R-r)%R],hs,ldtw(P.twN+r*m),V,Vc);
+        put(r*m,V);
+        if(r > 0 && 2*r < R) put(Nh-r*m,Vc);
+      }
+      if(even) {
+#pragma unroll
+        for(int r=0; r < (R+1)/2; ++r) {
+          const int k=m/2+r*m;
+          hermUnpack(b[0][r],b[0][R-1-r],hs,ldtw(P.twN+k),V,Vc);
+          put(k,V);
+          if(2*r < R-1) put(Nh-k,Vc);
+        }
+      }
+    }
+  }
+}
+
+// The staged form (runStages) of a Hermitian row: the packing and unpacking
+// one pair at a time.
+template<typename T, bool WIDE, class Mul>
+__device__ __forceinline__ void hermRowStaged(const HermRowPlan<T>& P,
+                                              const Mul& mul, cplx<T> *x,
+                                              int cs, long long row, int team,
+                                              int t, int nt)
+{
+  const FusedFFT& p=P.fz;
+  const int Nh=P.Nh, H=row < P.nrows ? P.H : 0;
+  const ColumnMap cols(Nh/2+1);
+#pragma unroll 2
+  for(int i=t; i < P.A*cols.per; i += nt) {
+    const int c=cols(i), k=i-c*cols.per, kk=Nh-k;
+    const cplx<T> *z=P.in[c]+row*P.rowStride;
+    const int sh=ioShift<T>(P.ioShift,c);
+    cplx<T> a=mk((T) 0,(T) 0), b=a, Y, Yc;
+    if(k < H) a=loadIO(z+k,P.io64 & 1,sh);
+    if(kk < H) b=loadIO(z+kk,P.io64 & 1,sh);
+    if(k == 0) a.y=(T) 0;
+    hermPack(a,b,ldtw(P.twN+k),Y,Yc);
+    x[c*cs+spl(k,p.lg)]=Y;
+    if(k != 0 && 2*k != Nh) x[c*cs+spl(kk,p.lg)]=Yc;
+  }
+  runStages<T,WIDE>(x,cs,P.A,P.B,p,0,0,team,t,nt,[&] {
+      fusedMulSlots(P,mul,x,cs,row,t,nt);
+    });
+  const T hs=(T) 0.5*P.scale;
+#pragma unroll 1
+  for(int i=t; i < P.B*cols.per; i += nt) {
+    const int c=cols(i), k=i-c*cols.per, kk=k == 0 ? 0 : Nh-k;
+    if(k >= H && kk >= H) continue;
+    const cplx<T> zk=swapXY(x[c*cs+spl(k,p.lg)]);
+    const cplx<T> zm=swapXY(x[c*cs+spl(kk,p.lg)]);
+    cplx<T> *o=P.out[c]+row*P.rowStride, V, Vc;
+    const int sh=ioShift<T>(P.ioShift,8+c);
+    hermUnpack(zk,zm,hs,ldtw(P.twN+k),V,Vc);
+    if(k < H) storeIO(o+k,V,P.io64 & 2,sh);
+    if(kk > k && kk < H) storeIO(o+kk,Vc,P.io64 & 2,sh);
+  }
+}
+
+// First radices of fused Hermitian rows (the two butterflies of a pair are
+// in registers together).
+#define FGB_HERM_SWITCH(R,CALL) \
+  switch(R) { \
+    case 1: {constexpr int R_=1; CALL;} break; \
+    case 2: {constexpr int R_=2; CALL;} break; \
+    case 3: {constexpr int R_=3; CALL;} break; \
+    case 4: {constexpr int R_=4; CALL;} break; \
+    case 5: {constexpr int R_=5; CALL;} break; \
+    case 6: {constexpr int R_=6; CALL;} break; \
+    case 7: {constexpr int R_=7; CALL;} break; \
+    case 8: {constexpr int R_=8; CALL;} break; \
+    default: break; \
+  }
+
+template<typename T, class Mul, bool WIDE>
 __device__ __forceinline__ void hermRows(const HermRowPlan<T>& P,
                                          const Mul& mul,
                                          unsigned char *smemRaw)
 {
-  const int A=P.A, B=P.B, H=P.H, Nh=P.Nh, R=P.rpc;
-  const int ld=A*R, lb=B*R;
-  cplx<T> *x=(cplx<T> *) smemRaw;
-  cplx<T> *y=x+padded(Nh*ld);        // ping-pong buffer of the FP64 form
-  const int tid=threadIdx.x, nthr=blockDim.x;
-  const typename TwT<T>::type *tw=P.twN;
-  const T half=(T) 0.5;
-  const UDiv dH(H), dLd(ld);
-  const UDiv dR(R);
-  const long long groups=(P.nrows+R-1)/R;
-
-  // Rows g*R .. g*R+R-1 are transformed together; column col = a*R + rho.
-  for(long long g=blockIdx.x; g < groups; g += gridDim.x) {
-    const long long row0=g*R;
-    // Y[k] = S + i W_N^k D with S = Z[k] + conj Z[Nh-k], D = Z[k] -
-    // conj Z[Nh-k], Z read from the row itself.  One thread forms the pair
-    // k, Nh-k from the same two loads: Y[Nh-k] = conj(S) + i conj(W_N^k D)
-    // (since W_N^{Nh} = -1), so the pair costs one twiddle multiply.
-    // Every read of the group precedes its writes, so in = out is safe.
-    // The loads of FGB_LOADS iterations are issued before any is used.
-    const int np=Nh/2+1;                 // k = 0 .. floor(Nh/2)
-    for(int i0=tid; i0 < np*ld; i0 += FGB_LOADS*nthr) {
-      cplx<T> zk[FGB_LOADS], zc[FGB_LOADS];
-#pragma unroll
-      for(int u=0; u < FGB_LOADS; ++u) {
-        const int i=i0+u*nthr;
-        int k=dLd(i), col=i-k*ld;       // col < ld: a < A for every i
-        int a=dR(col);
-        long long row=row0+col-a*R;
-        const cplx<T> *zr=P.in[a]+row*P.rowStride;
-        const bool live=i < np*ld && row < P.nrows;
-        const int kk=Nh-k;
-        const int sh=ioShift<T>(P.ioShift,a);
-        zk[u]=live && k < H ? loadIO(zr+k,P.io64 & 1,sh) : mk((T) 0,(T) 0);
-        zc[u]=live && kk < H ? loadIO(zr+kk,P.io64 & 1,sh) : mk((T) 0,(T) 0);
+  const int nt=blockDim.x/P.nteam;
+  const int team=threadIdx.x/nt, t=threadIdx.x-team*nt;
+  const int cs=fusedSpan(P.Nh,P.fz.lg);
+  cplx<T> *x=(cplx<T> *) smemRaw+team*P.A*cs;
+  const int R0=P.fz.radix[0];
+  const bool staged=std::is_same<T,ff>::value || P.A*((P.Nh/R0+1)/2) < nt;
+  const long long groups=(P.nrows+P.rpc-1)/P.rpc;
+  for(long long g=blockIdx.x; g < groups; g += gridDim.x)
+    for(int rho=team; rho < P.rpc; rho += P.nteam) {
+      const long long row=g*P.rpc+rho;
+      if(staged) hermRowStaged<T,WIDE>(P,mul,x,cs,row,team,t,nt);
+      else if constexpr(!std::is_same<T,ff>::value) {
+        FGB_HERM_SWITCH(R0,(hermFirst<T,R_>(P,x,cs,row,t,nt)))
+        fusedRowInner<T,WIDE>(P,mul,x,cs,row,team,t,nt);
+        FGB_HERM_SWITCH(R0,(hermLast<T,R_>(P,x,cs,row,t,nt)))
       }
-#pragma unroll
-      for(int u=0; u < FGB_LOADS; ++u) {
-        const int i=i0+u*nthr;
-        if(i >= np*ld) break;
-        const int k=dLd(i), col=i-k*ld;
-        cplx<T> a=zk[u];
-        if(k == 0) a.y=(T) 0;
-        const cplx<T> b=conjg(zc[u]);
-        const cplx<T> S=a+b;
-        cplx<T> Y, Yc;
-        if constexpr(std::is_same<T,double>::value) {
-          // FP64: S + (i D) W as four DFMAs, the partner as conj(2S - Y).
-          const cplx<T> D=a-b;
-          Y=fmaTw<1>(S,mk(-D.y,D.x),tw[k]);
-          Yc=mk(fma((T) 2,S.x,-Y.x),fma((T) -2,S.y,Y.y));
-        } else {
-          const cplx<T> Pw=twmul<1>(a-b,tw[k]);
-          Y=mk(S.x-Pw.y,S.y+Pw.x);
-          Yc=mk(S.x+Pw.y,Pw.x-S.y);
-        }
-        x[sp(i)]=Y;
-        if(k != 0 && 2*k != Nh) x[sp((Nh-k)*ld+col)]=Yc;
-      }
+      teamSync(team,nt);
     }
-    __syncthreads();
-    const cplx<T> *Z;
-    if constexpr(inplaceFFT<T>()) {
-      fftDIF<T,1,R16>(x,P.fp,ld,ld,tid,nthr);
-      for(int i=tid; i < Nh*R; i += nthr) {
-        int t=dR(i), rho=i-t*R;
-        mulHermSlot<Mul,true>(mul,P,x,t*ld+rho,R,row0+rho,t);
-      }
-      __syncthreads();
-      fftDIT<T,-1,R16>(x,P.fp,lb,ld,tid,nthr);
-      Z=x;
-    } else {
-      cplx<T> *X=fftSmem<T,1>(x,y,P.fp,ld,ld,tid,nthr);
-      cplx<T> *Y=X == x ? y : x;
-      for(int i=tid; i < Nh*R; i += nthr) {
-        int t=dR(i), rho=i-t*R;
-        mulHermSlot<Mul,false>(mul,P,X,t*ld+rho,R,row0+rho,t);
-      }
-      __syncthreads();
-      Z=fftSmem<T,-1>(X,Y,P.fp,lb,ld,tid,nthr);
-    }
-    // V[k] = (s + Q)/2 with s = Z[k] + conj Z[m], Q = W_N^{-k} (-i)(Z[k] -
-    // conj Z[m]), m = Nh-k (m = 0 for k = 0).  When both k and Nh-k are
-    // stored modes the lower one also writes V[Nh-k] = conj(s - Q)/2, and
-    // the upper one skips.
-    const T hs=half*P.scale;
-    for(int i=tid; i < lb*H; i += nthr) {
-      int col=dH(i), k=i-col*H;
-      int b=dR(col);
-      long long row=row0+col-b*R;
-      const int km=k == 0 ? 0 : Nh-k;
-      const bool pair=k != 0 && km < H && km != k;
-      if(row >= P.nrows || (pair && km < k)) continue;
-      const cplx<T> zk=Z[sp(k*ld+col)];
-      const cplx<T> zm=conjg(Z[sp(km*ld+col)]);
-      cplx<T> V, Vc;
-      if constexpr(std::is_same<T,double>::value) {
-        // FP64: hs sum, hs dd = 2 hs zk - hs sum, V = hs sum + hs Q as
-        // four DFMAs, the partner as conj(2 hs sum - V).
-        const cplx<T> hsum=(zk+zm)*hs;
-        const T h2=hs+hs;
-        const cplx<T> hdd=mk(fma(h2,zk.x,-hsum.x),fma(h2,zk.y,-hsum.y));
-        V=fmaTw<-1>(hsum,mk(hdd.y,-hdd.x),tw[k]);
-        Vc=mk(fma((T) 2,hsum.x,-V.x),fma((T) -2,hsum.y,V.y));
-      } else {
-        const cplx<T> sum=zk+zm, dd=zk-zm;
-        const cplx<T> Q=twmul<-1>(mk(dd.y,-dd.x),tw[k]);
-        V=(sum+Q)*hs;
-        Vc=conjg(sum-Q)*hs;
-      }
-      cplx<T> *o=P.out[b]+row*P.rowStride;
-      const int sh=ioShift<T>(P.ioShift,8+b);
-      storeIO(o+k,V,P.io64 & 2,sh);
-      if(pair) storeIO(o+km,Vc,P.io64 & 2,sh);
-    }
-    __syncthreads();
-  }
 }
 
 template<typename T, class Mul>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256,fusedBlocks<T>())
 hermRowKernel(const HermRowPlan<T> P, const Mul mul)
 {
   extern __shared__ __align__(16) unsigned char smemRaw[];
   hermRows<T,Mul,false>(P,mul,smemRaw);
 }
 
-// FP32 plans with a radix-16 stage (as rowConvKernel16).
+// FP32 plans with a radix-16 stage.
 template<typename T, class Mul>
-__global__ void __launch_bounds__(256,3)
+__global__ void __launch_bounds__(256,fusedBlocks<T>())
 hermRowKernel16(const HermRowPlan<T> P, const Mul mul)
 {
   extern __shared__ __align__(16) unsigned char smemRaw[];
@@ -879,7 +1231,8 @@ template<typename T, class Mul>
 cudaError_t launchRowWith(const RowPlan<T>& P, const Mul& mul, int threads,
                           long long grid, cudaStream_t s)
 {
-  const size_t sm=rowSmem<T>(P.L,P.m,P.A,P.B,P.rpc,P.direct);
+  const size_t sm=P.direct ? fusedRowSmem<T>(P.fz.n,P.fz.lg,P.A,P.nteam) :
+    rowSmem<T>(P.L,P.m,P.A,P.B,P.rpc);
   const long long groups=(P.nrows+P.rpc-1)/P.rpc;
   grid=std::min(std::min(grid,groups),(long long) INT_MAX);
   if(grid < 1) return cudaSuccess;
@@ -889,20 +1242,19 @@ cudaError_t launchRowWith(const RowPlan<T>& P, const Mul& mul, int threads,
     kernel<<<(unsigned) grid,threads,sm,s>>>(P,mul);
     return cudaGetLastError();
   };
-  if constexpr(std::is_same<T,float>::value)
-    if(hasWideRadix(P.fp)) {
-      if(P.direct) return go(rowConvKernel16<T,Mul,true>);
-      return go(rowConvKernel16<T,Mul,false>);
-    }
-  if(P.direct) return go(rowConvKernel<T,Mul,true>);
-  return go(rowConvKernel<T,Mul,false>);
+  if constexpr(std::is_same<T,float>::value) {
+    if(P.direct && wideFused(P.fz)) return go(rowFusedKernel16<T,Mul>);
+    if(!P.direct && hasWideRadix(P.fp)) return go(rowConvKernel16<T,Mul>);
+  }
+  if(P.direct) return go(rowFusedKernel<T,Mul>);
+  return go(rowConvKernel<T,Mul>);
 }
 
 template<typename T, class Mul>
 cudaError_t launchHermRowWith(const HermRowPlan<T>& P, const Mul& mul,
                               int threads, long long grid, cudaStream_t s)
 {
-  const size_t sm=hermRowSmem<T>(P.H,P.Nh,P.A,P.rpc);
+  const size_t sm=fusedRowSmem<T>(P.fz.n,P.fz.lg,P.A,P.nteam);
   const long long groups=(P.nrows+P.rpc-1)/P.rpc;
   grid=std::min(std::min(grid,groups),(long long) INT_MAX);
   if(grid < 1) return cudaSuccess;
@@ -913,7 +1265,7 @@ cudaError_t launchHermRowWith(const HermRowPlan<T>& P, const Mul& mul,
     return cudaGetLastError();
   };
   if constexpr(std::is_same<T,float>::value)
-    if(hasWideRadix(P.fp)) return go(hermRowKernel16<T,Mul>);
+    if(wideFused(P.fz)) return go(hermRowKernel16<T,Mul>);
   return go(hermRowKernel<T,Mul>);
 }
 

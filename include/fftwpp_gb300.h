@@ -344,6 +344,16 @@ int fgb_batch_task_order(int nlong, const size_t *staging,
 int fgb_fft_radices(size_t n, int precision, int inplace, int wide,
                     int *radix, int max);
 
+/* Radices, stage by stage, of the fused transforms of length n (host
+ * arithmetic, no GPU): `inputs` columns share the registers of the middle
+ * stage, hermitian != 0 for the rows of Hermitian data, half != 0 for data
+ * that fill at most half of n.  padding (NULL or two entries) is set to the
+ * lg of the shared-memory padding, one element every 2^lg, that the kernels
+ * use and of the wider one they fall back on.  Writes at most max radices and
+ * returns their count, or -1. */
+int fgb_fused_radices(size_t n, int precision, int inputs, int hermitian,
+                      int half, int *radix, int max, int *padding);
+
 /* Transformed index of entry i of residue block r (fftBase::index,
  * convolve.h:297-326, and fftPadReal::index, convolve.h:956-979) for the
  * reference's parameters (m,p,q,n,D) of a 1D transform. */
