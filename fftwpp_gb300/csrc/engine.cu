@@ -555,6 +555,22 @@ static size_t outerBwdNeed(const AxisPlan& a, int prec, int tile)
   return FGB_BY_PREC(prec,outerBwdSmem,a.L,a.m,tile,(int) a.q);
 }
 
+// CTAs per complex row of padded length n (RowPlan::split): as many of 8, 4
+// or 2 as leave every row its own SMs and every CTA at least 64 points of a
+// length they divide; 1 otherwise.  Measured against one CTA per row (kernel
+// and event, us): FP64 n = 2048, 1 / 38 / 76 rows 66 -> 29 / 45 / 49, n = 512
+// 27 -> 22 to 25, float-float 43 -> 26 / 30 / 34; from n = 128 down no
+// faster, and FP32, whose rows are bound by latency alone, slower (n = 2048,
+// 76 rows 16 -> 21).
+static int rowSplit(long n, long nrows, int prec)
+{
+  static const int sms=152;
+  if(prec == PREC_F32 || n < 512) return 1;
+  for(int q : {8,4,2})
+    if(n % q == 0 && n/q >= 64 && smooth(n/q) && nrows*q <= sms) return q;
+  return 1;
+}
+
 // Whether a Hermitian row goes to one CTA or to the long path; the line
 // stays where a ping-pong FP64 transform put it.
 static size_t hermNeed(int prec, long Nh, int A)
@@ -634,10 +650,13 @@ static double rowCost(const AxisPlan& a, long m, long q, int A, int B,
 {
   if(q == 1 && a.L <= m)
     return fusedCost(m,prec,A,B,false,a.kind != KIND_CENTERED && 2*a.L <= m);
-  const double pass=prec == PREC_F64 ? 2.0 : prec == PREC_FF ? 1.0 : 8.0;
+  // The fused rows run an instruction's worth in 0.55 (FP32) to 0.9 of the
+  // time (4096 rows of 1024: FP32 175 -> 83 us, FP64 1728 -> 1425).
+  const double slower=prec == PREC_F32 ? 1.8 : 1.1;
   long p=ceilquotient(a.L,m);
-  return q*(A+B)*(fftInstr(m)+pass*m)+
-    A*(double) m*(2.0*p+(q-1)*6.0*p)+B*(double) a.L*(2.0+(q-1)*6.0);
+  return slower*(q*(A+B)*(fftInstr(m)+2.0*m)+
+                 A*(double) m*(2.0*p+(q-1)*6.0*p)+
+                 B*(double) a.L*(2.0+(q-1)*6.0));
 }
 
 // The same for an outer axis: residue r > 0 folds p terms with a complex
@@ -1555,7 +1574,7 @@ cudaError_t Conv::runT(const void *const *in, void *const *out, cudaStream_t s)
     }
     if(I.longRow) im.longQ=(int) I.rowQ;    // long rows: k = k1 + q k2
   }
-  auto rowPlan=[&](RowPlan<T>& P, const AxisPlan& a) {
+  auto rowPlan=[&](RowPlan<T>& P, const AxisPlan& a, long nrows) {
     P.im=im;
     P.ioShift=guard;
     P.L=(int) a.stored; P.m=(int) a.m; P.q=(int) a.q; P.N=(int) a.N;
@@ -1565,7 +1584,15 @@ cudaError_t Conv::runT(const void *const *in, void *const *out, cudaStream_t s)
     P.io64=0;
     P.direct=rowDirect(a);
     P.nteam=rowTeams(P.rpc,a.thr);
-    if(P.direct) {
+    P.split=I.mult != MULT_USER ? rowSplit(a.N,nrows,I.prec) : 1;
+    if(P.split > 1) {
+      P.fz=fusedRowPlan(a.N/P.split,I.prec,A,false,false,1,8);
+      if(FGB_BY_PREC(I.prec,fusedRowSmem,P.fz.n,P.fz.lg,A,1) > SMEM_MAX)
+        P.split=1;
+    }
+    if(P.split > 1) {
+      fusedTables(P.fz,I.prec);
+    } else if(P.direct) {
       P.fz=fusedRowPlan(a.m,I.prec,A,false,halfEmpty(a),P.nteam,
                         widest(I.prec));
       fusedTables(P.fz,I.prec);
@@ -1687,7 +1714,7 @@ cudaError_t Conv::runT(const void *const *in, void *const *out, cudaStream_t s)
       return e;
     }
     RowPlan<T> P{};
-    rowPlan(P,a);
+    rowPlan(P,a,batch);
     for(int i=0; i < A; ++i) P.in[i]=(const Cx *) in[i];
     for(int i=0; i < B; ++i) P.out[i]=(Cx *) out[i];
     P.rowStride=a.stored; P.nrows=batch; P.scale=(T) scale;
@@ -1732,7 +1759,7 @@ cudaError_t Conv::runT(const void *const *in, void *const *out, cudaStream_t s)
       tick(s);
     } else {
       RowPlan<T> P{};
-      rowPlan(P,ay);
+      rowPlan(P,ay,ax.rows);
       for(int i=0; i < A; ++i) P.in[i]=(const Cx *) bufs[i];
       for(int i=0; i < B; ++i) P.out[i]=(Cx *) bufs[i];
       P.rowStride=C; P.nrows=ax.rows; P.scale=(T) 1;
@@ -1801,7 +1828,7 @@ cudaError_t Conv::runT(const void *const *in, void *const *out, cudaStream_t s)
     tick(s);
   } else {
     RowPlan<T> P{};
-    rowPlan(P,az);
+    rowPlan(P,az,nrows);
     for(int i=0; i < A; ++i) P.in[i]=(const Cx *) by[i];
     for(int i=0; i < B; ++i) P.out[i]=(Cx *) by[i];
     P.rowStride=nz; P.nrows=nrows; P.scale=(T) 1;

@@ -219,13 +219,35 @@ struct ColumnMap {
   }
 };
 
+// Calls f(c, idx) for this thread's butterflies idx < per of the ncol column
+// groups c: all of them in one loop, or (WIDE: the long FP32 transforms with
+// radix 16, whose registers are short) one group after the other.
+template<bool WIDE, class F>
+__device__ __forceinline__ void forColumns(int ncol, int per, int t, int nt,
+                                           const F& f)
+{
+  if constexpr(WIDE) {
+#pragma unroll 1
+    for(int c=0; c < ncol; ++c)
+#pragma unroll 1
+      for(int idx=t; idx < per; idx += nt) f(c,idx);
+  } else {
+    const ColumnMap cols(per);
+#pragma unroll 1
+    for(int k=t; k < ncol*per; k += nt) {
+      const int c=cols(k);
+      f(c,k-c*per);
+    }
+  }
+}
+
 // The first forward stage (one block, no twiddles): load(c, cc)(j) gives
 // input j of interleaved column cc of group c (groups cs apart, `ncol` of
 // them).  HALF: inputs j >= n/2 are zero.  (A thread takes one column
 // through a stage at a time: two at once, sharing twiddles, need 128
 // registers where three CTAs per SM at 85 serve better, 3D real FP32 rows
 // of 512 points 481 against 508 us; FP64 measured the same either way.)
-template<typename T, int R, bool HALF, class Load>
+template<typename T, int R, bool HALF, bool WIDE, class Load>
 __device__ __forceinline__ void fusedFirst(cplx<T> *x, int cs, int ncol,
                                            const FusedFFT& p, int lt, int t,
                                            int nt, const Load& load)
@@ -233,10 +255,7 @@ __device__ __forceinline__ void fusedFirst(cplx<T> *x, int cs, int ncol,
   const int m=p.n/R;
   const StageMap map(R,m,p.lg,lt);
   constexpr int NZ=HALF ? R/2 : R;
-  const ColumnMap cols(m << lt);
-#pragma unroll 1
-  for(int k=t; k < ncol*cols.per; k += nt) {
-    const int c=cols(k), idx=k-c*cols.per;
+  forColumns<WIDE>(ncol,m << lt,t,nt,[&](int c, int idx) {
     const int j=idx >> lt, cc=idx & ((1 << lt)-1);
     cplx<T> a[R];
     const auto in=load(c,cc);
@@ -249,13 +268,15 @@ __device__ __forceinline__ void fusedFirst(cplx<T> *x, int cs, int ncol,
     else Codelet<R,1,T>::run(a);
 #pragma unroll
     for(int r=0; r < R; ++r) xq[r*map.step]=a[r];
-  }
+  });
 }
 
 // A stage in place, of either direction: twiddles tw[(r-1) stride + b]
 // (forward, b the block) or tw[(r-1) stride + j] (inverse, j the position in
-// it); tw NULL: none (runStages).
-template<typename T, int R>
+// it).  OPT: tw may be NULL, no twiddles (runStages; a test before the
+// twiddles keeps their loads behind those of the inputs, 94 against 83 us on
+// 4096 FP32 pairs of 1024, so the fused form has none).
+template<typename T, int R, bool WIDE, bool OPT=false>
 __device__ __forceinline__ void fusedStage(cplx<T> *x, int cs, int ncol,
                                            const FusedFFT& p, int lt, int m,
                                            const typename TwT<T>::type *tw,
@@ -263,10 +284,7 @@ __device__ __forceinline__ void fusedStage(cplx<T> *x, int cs, int ncol,
                                            int nt)
 {
   const StageMap map(R,m,p.lg,lt);
-  const ColumnMap cols(p.n/R << lt);
-#pragma unroll 1
-  for(int w=t; w < ncol*cols.per; w += nt) {
-    const int c=cols(w), idx=w-c*cols.per;
+  forColumns<WIDE>(ncol,p.n/R << lt,t,nt,[&](int c, int idx) {
     const int i=idx >> lt, cc=idx & ((1 << lt)-1);
     const int b=map.block(i);
     cplx<T> *xq=x+c*cs+map.offset(i,b,cc);
@@ -274,7 +292,8 @@ __device__ __forceinline__ void fusedStage(cplx<T> *x, int cs, int ncol,
 #pragma unroll
     for(int r=0; r < R; ++r) a[0][r]=nrm(xq[r*map.step]);
     const int k=inverse ? i-b*m : b;
-    if constexpr(fusedTw<T,R>()) {
+    if constexpr(!OPT) inTwiddleDFT<T,R,1>(a,tw,k,stride);
+    else if constexpr(fusedTw<T,R>()) {
       if(tw) inTwiddleDFT<T,R,1>(a,tw,k,stride);
       else Codelet<R,1,T>::run(a[0]);
     } else {
@@ -287,13 +306,13 @@ __device__ __forceinline__ void fusedStage(cplx<T> *x, int cs, int ncol,
     }
 #pragma unroll
     for(int r=0; r < R; ++r) xq[r*map.step]=a[0][r];
-  }
+  });
 }
 
 // The last inverse stage: store(c, cc)(j, v) takes output j, its parts in
 // their own places again (HALF: only j < n/2, the others are not
 // computed).
-template<typename T, int R, bool HALF, class Store>
+template<typename T, int R, bool HALF, bool WIDE, class Store>
 __device__ __forceinline__ void fusedLast(const cplx<T> *x, int cs, int ncol,
                                           const FusedFFT& p, int lt, int t,
                                           int nt, const Store& store)
@@ -302,10 +321,7 @@ __device__ __forceinline__ void fusedLast(const cplx<T> *x, int cs, int ncol,
   const StageMap map(R,m,p.lg,lt);
   constexpr int NZ=HALF ? R/2 : R;
   const typename TwT<T>::type *tw=(const typename TwT<T>::type *) p.twj+(m-1);
-  const ColumnMap cols(m << lt);
-#pragma unroll 1
-  for(int k=t; k < ncol*cols.per; k += nt) {
-    const int c=cols(k), idx=k-c*cols.per;
+  forColumns<WIDE>(ncol,m << lt,t,nt,[&](int c, int idx) {
     const int j=idx >> lt, cc=idx & ((1 << lt)-1);
     const cplx<T> *xq=x+c*cs+map.offset(j,0,cc);
     cplx<T> a[1][R];
@@ -315,7 +331,7 @@ __device__ __forceinline__ void fusedLast(const cplx<T> *x, int cs, int ncol,
     const auto out=store(c,cc);
 #pragma unroll
     for(int r=0; r < NZ; ++r) out(j+r*m,swapXY(a[0][r]));
-  }
+  });
 }
 
 // Whether the kernels of T hold radix R as an inner or first stage.  WIDE:
@@ -347,20 +363,20 @@ __device__ __forceinline__ void runFusedFirst(cplx<T> *x, int cs, int ncol,
 {
   if(p.half) {
     switch(p.radix[0]) {
-      case 2: fusedFirst<T,2,true>(x,cs,ncol,p,lt,t,nt,load); break;
-      case 4: fusedFirst<T,4,true>(x,cs,ncol,p,lt,t,nt,load); break;
-      case 6: fusedFirst<T,6,true>(x,cs,ncol,p,lt,t,nt,load); break;
-      case 8: fusedFirst<T,8,true>(x,cs,ncol,p,lt,t,nt,load); break;
+      case 2: fusedFirst<T,2,true,WIDE>(x,cs,ncol,p,lt,t,nt,load); break;
+      case 4: fusedFirst<T,4,true,WIDE>(x,cs,ncol,p,lt,t,nt,load); break;
+      case 6: fusedFirst<T,6,true,WIDE>(x,cs,ncol,p,lt,t,nt,load); break;
+      case 8: fusedFirst<T,8,true,WIDE>(x,cs,ncol,p,lt,t,nt,load); break;
       case 16:
         if constexpr(fusedRadix<T,WIDE>(16))
-          fusedFirst<T,16,true>(x,cs,ncol,p,lt,t,nt,load);
+          fusedFirst<T,16,true,WIDE>(x,cs,ncol,p,lt,t,nt,load);
         break;
       default: break;
     }
     return;
   }
   FGB_FUSED_SWITCH(p.radix[0],
-                   (fusedFirst<T,R_,false>(x,cs,ncol,p,lt,t,nt,load)))
+                   (fusedFirst<T,R_,false,WIDE>(x,cs,ncol,p,lt,t,nt,load)))
 }
 
 template<typename T, bool WIDE, class Store>
@@ -371,20 +387,20 @@ __device__ __forceinline__ void runFusedLast(const cplx<T> *x, int cs,
 {
   if(p.half) {
     switch(p.radix[0]) {
-      case 2: fusedLast<T,2,true>(x,cs,ncol,p,lt,t,nt,store); break;
-      case 4: fusedLast<T,4,true>(x,cs,ncol,p,lt,t,nt,store); break;
-      case 6: fusedLast<T,6,true>(x,cs,ncol,p,lt,t,nt,store); break;
-      case 8: fusedLast<T,8,true>(x,cs,ncol,p,lt,t,nt,store); break;
+      case 2: fusedLast<T,2,true,WIDE>(x,cs,ncol,p,lt,t,nt,store); break;
+      case 4: fusedLast<T,4,true,WIDE>(x,cs,ncol,p,lt,t,nt,store); break;
+      case 6: fusedLast<T,6,true,WIDE>(x,cs,ncol,p,lt,t,nt,store); break;
+      case 8: fusedLast<T,8,true,WIDE>(x,cs,ncol,p,lt,t,nt,store); break;
       case 16:
         if constexpr(fusedRadix<T,WIDE>(16))
-          fusedLast<T,16,true>(x,cs,ncol,p,lt,t,nt,store);
+          fusedLast<T,16,true,WIDE>(x,cs,ncol,p,lt,t,nt,store);
         break;
       default: break;
     }
     return;
   }
   FGB_FUSED_SWITCH(p.radix[0],
-                   (fusedLast<T,R_,false>(x,cs,ncol,p,lt,t,nt,store)))
+                   (fusedLast<T,R_,false,WIDE>(x,cs,ncol,p,lt,t,nt,store)))
 }
 
 // CTAs of 256 threads per SM the row kernels' registers leave room for.
@@ -413,7 +429,7 @@ __device__ __forceinline__ int runFusedMiddle(cplx<T> *x, int cs, int ncol,
     const Tw *tw=inverse ? twj+(m-1) : twb+(nblk-R0);
     const int stride=inverse ? m : nblk;
     teamSync(team,nt);
-    FGB_FUSED_SWITCH(R,(fusedStage<T,R_>(x,cs,ncol,p,lt,m,tw,stride,
+    FGB_FUSED_SWITCH(R,(fusedStage<T,R_,WIDE>(x,cs,ncol,p,lt,m,tw,stride,
                                             inverse,t,nt)))
     if(inverse) m *= R;
     else nblk *= R;
@@ -465,8 +481,8 @@ __device__ __forceinline__ void runStages(cplx<T> *x, int cs, int A, int B,
       (s > 0 ? twb+(nblk-R0) : NULL);
     const int stride=inverse ? m : nblk, ncol=inverse ? B : A;
     teamSync(team,nt);
-    FGB_FUSED_SWITCH(R,(fusedStage<T,R_>(x,cs,ncol,p,lt,m,tw,stride,inverse,
-                                         t,nt)))
+    FGB_FUSED_SWITCH(R,(fusedStage<T,R_,WIDE,true>(x,cs,ncol,p,lt,m,tw,stride,
+                                                   inverse,t,nt)))
     if(inverse) m *= R;
     else nblk *= R;
   }

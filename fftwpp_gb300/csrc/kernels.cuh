@@ -89,6 +89,9 @@ struct RowPlan {
                            // fused rows, transformed by fz (fp unused)
   int nteam;               // fused rows: teams of threads per CTA (divides
                            // rpc; a team convolves whole rows)
+  int split;               // > 1: this many CTAs (a cluster) per row, fz the
+                           // transform of N/split points (rowSplitKernel;
+                           // not for a caller's functor)
   const int *ioShift;      // float-float range guard: device exponents,
                            // [a] input a, [8+b] output b (NULL: none)
   T scale;

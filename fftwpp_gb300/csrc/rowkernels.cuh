@@ -11,6 +11,7 @@
 
 #include <algorithm>
 #include <climits>
+#include <cooperative_groups.h>
 #include <type_traits>
 
 namespace fgb {
@@ -826,12 +827,12 @@ __device__ __forceinline__ void fusedRowInner(const Plan& P, const Mul& mul,
       const Tw *twb=(const Tw *) p.twb+(nblk-p.radix[0]);
       const Tw *twj=(const Tw *) p.twj;
       const int R=p.radix[p.nst-1];
-      FGB_FUSED_SWITCH(R,(fusedStage<T,R_>(x,cs,A,p,0,1,twb,nblk,false,t,
+      FGB_FUSED_SWITCH(R,(fusedStage<T,R_,WIDE>(x,cs,A,p,0,1,twb,nblk,false,t,
                                              nt)))
       teamSync(team,nt);
       fusedMulSlots(P,mul,x,cs,row,t,nt);
       teamSync(team,nt);
-      FGB_FUSED_SWITCH(R,(fusedStage<T,R_>(x,cs,B,p,0,1,twj,1,true,t,nt)))
+      FGB_FUSED_SWITCH(R,(fusedStage<T,R_,WIDE>(x,cs,B,p,0,1,twj,1,true,t,nt)))
     }
     runFusedMiddle<T,WIDE>(x,cs,B,p,0,true,team,t,nt);
     teamSync(team,nt);
@@ -926,6 +927,103 @@ rowFusedKernel16(const RowPlan<T> P, const Mul mul)
 {
   extern __shared__ __align__(16) unsigned char smemRaw[];
   fusedRows<T,Mul,true>(P,mul,smemRaw);
+}
+
+// ---------------------------------------------------------------------------
+// Split rows: with few rows (RowPlan::split CTAs per row still fit the SMs) a
+// cluster of P.split CTAs convolves each row, CTA r the residue r of the
+// padded transform: it folds the data into a block of N/split points with
+// the residue twiddles, transforms, multiplies and transforms back on its
+// own; then every CTA adds a share of the outputs over the blocks of the
+// cluster, read through distributed shared memory, with their
+// post-twiddles.  A row alone is bound by the FP64 pipe and the latency of
+// its one SM: one pair of 1024 points (2048 padded) took 66 us in FP64, 29
+// split eight ways (rowSplit in engine.cu).
+template<typename T, class Mul>
+__global__ void __launch_bounds__(256,2)
+rowSplitKernel(const RowPlan<T> P, const Mul mul)
+{
+  namespace cg=cooperative_groups;
+  extern __shared__ __align__(16) unsigned char smemRaw[];
+  cg::cluster_group cluster=cg::this_cluster();
+  const int Q=P.split, r=(int) cluster.block_rank();
+  const long long row=blockIdx.x/Q;
+  const int L=P.L, c=P.cshift, N=P.N, m=P.fz.n;
+  const int t=threadIdx.x, nt=blockDim.x;
+  const int cs=fusedSpan(m,P.fz.lg);
+  cplx<T> *x=(cplx<T> *) smemRaw;
+  const typename TwT<T>::type *tw=P.twN;
+  const long long off0=row*P.rowStride;
+  const ColumnMap cols(m);
+  const int step=twStep(m,r,N);
+#pragma unroll 1
+  for(int i=t; i < P.A*m; i += nt) {
+    const int a=cols(i), j=i-a*m;
+    const int sh=ioShift<T>(P.ioShift,a);
+    cplx<T> sum=mk((T) 0,(T) 0);
+    int s=posmod(j+c,m);
+    int e=twExp(s,c,r,N);
+#pragma unroll 4
+    for(; s < L; s += m) {
+      cplx<T> v=mk((T) 0,(T) 0);
+      if(P.realIO)
+        v.x=loadIOr((const T *) P.in[a]+off0+s,P.io64 & 1,sh);
+      else v=loadIO(P.in[a]+off0+s,P.io64 & 1,sh);
+      sum=accum(sum,twmul<1>(v,ldtw(tw+e)));
+      e += step;
+      if(e >= N) e -= N;
+    }
+    x[a*cs+spl(j,P.fz.lg)]=sum;
+  }
+  runStages<T>(x,cs,P.A,P.B,P.fz,0,0,0,t,nt,[&] {
+      fusedMulSlots(P,mul,x,cs,row,t,nt);
+    });
+  cluster.sync();
+  const int share=(L+Q-1)/Q, s0=r*share, n=max(0,min(L-s0,share));
+#pragma unroll 1
+  for(int i=t; i < P.B*n; i += nt) {
+    const int b=i/n, s=s0+i-b*n;
+    const int at=b*cs+spl(posmod(s-c,m),P.fz.lg);
+    const int de=twExp(s,c,1,N);
+    cplx<T> sum=mk((T) 0,(T) 0);
+    int e=0;
+#pragma unroll 4
+    for(int k=0; k < Q; ++k) {
+      const cplx<T> v=swapXY(cluster.map_shared_rank(x,k)[at]);
+      sum=accum(sum,twmul<-1>(v,ldtw(tw+e)));
+      e += de;
+      if(e >= N) e -= N;
+    }
+    const int sh=ioShift<T>(P.ioShift,8+b);
+    if(P.realIO)
+      storeIOr((T *) P.out[b]+off0+s,sum.x*P.scale,P.io64 & 2,sh);
+    else storeIO(P.out[b]+off0+s,sum*P.scale,P.io64 & 2,sh);
+  }
+  cluster.sync();                 // until the others have read this block
+}
+
+template<typename T, class Mul>
+cudaError_t launchRowSplit(const RowPlan<T>& P, const Mul& mul, int threads,
+                           size_t smem, cudaStream_t s)
+{
+  cudaError_t e=cudaSuccess;
+  if(smem > 48*1024)
+    e=cudaFuncSetAttribute(rowSplitKernel<T,Mul>,
+                           cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int) smem);
+  if(e != cudaSuccess) return e;
+  cudaLaunchConfig_t cfg={};
+  cfg.gridDim=dim3((unsigned) (P.nrows*P.split));
+  cfg.blockDim=dim3(threads);
+  cfg.dynamicSmemBytes=smem;
+  cfg.stream=s;
+  cudaLaunchAttribute at[1];
+  at[0].id=cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x=P.split;
+  at[0].val.clusterDim.y=at[0].val.clusterDim.z=1;
+  cfg.attrs=at;
+  cfg.numAttrs=1;
+  return cudaLaunchKernelEx(&cfg,rowSplitKernel<T,Mul>,P,mul);
 }
 
 // ---------------------------------------------------------------------------
@@ -1231,6 +1329,10 @@ template<typename T, class Mul>
 cudaError_t launchRowWith(const RowPlan<T>& P, const Mul& mul, int threads,
                           long long grid, cudaStream_t s)
 {
+  if constexpr(!Mul::positional)
+    if(P.split > 1)
+      return launchRowSplit(P,mul,threads,
+                            fusedRowSmem<T>(P.fz.n,P.fz.lg,P.A,1),s);
   const size_t sm=P.direct ? fusedRowSmem<T>(P.fz.n,P.fz.lg,P.A,P.nteam) :
     rowSmem<T>(P.L,P.m,P.A,P.B,P.rpc);
   const long long groups=(P.nrows+P.rpc-1)/P.rpc;
