@@ -453,7 +453,13 @@ int rowTeams(int rpc, int threads)
   return t;
 }
 
-static int widest(int prec) {return prec == PREC_F32 ? 16 : 8;}
+// The widest radix of a fused transform: 16 in FP32, for rows from 640 points
+// on (shorter ones leave most of a team without a radix-16 butterfly: 441
+// rows of 384 points 15 us with 3 16 8, 13 with 3 4 4 8).
+static int widest(int prec, long rowLength=640)
+{
+  return prec == PREC_F32 && rowLength >= 640 ? 16 : 8;
+}
 
 FusedFFT fusedRowPlan(long n, int prec, int A, bool herm, bool half,
                       int nteam, int maxR)
@@ -493,7 +499,7 @@ static size_t fusedRowNeed(int prec, long n, int A, bool herm, bool half,
                            int rpc, int threads)
 {
   const int teams=rowTeams(rpc,threads);
-  const FusedFFT p=fusedRowPlan(n,prec,A,herm,half,teams,widest(prec));
+  const FusedFFT p=fusedRowPlan(n,prec,A,herm,half,teams,widest(prec,n));
   return FGB_BY_PREC(prec,fusedRowSmem,p.n,p.lg,A,teams);
 }
 
@@ -609,8 +615,7 @@ static int pickRpc(long n, int A, long nrows, F smem)
 static double fusedCost(long n, int prec, int A, int B, bool herm, bool half)
 {
   int rad[FGB_FUSED_STAGES+8];
-  const int nst=fusedRadices(n,prec,A,herm,half,prec == PREC_F32 ? 16 : 8,
-                             rad);
+  const int nst=fusedRadices(n,prec,A,herm,half,widest(prec,n),rad);
   if(nst < 0) return 1e300;
   auto with=[](int R) {
     return R == 1 ? 0.0 : R == 2 ? 3.0 : R == 3 ? 6.0 : R == 4 ? 6.0 :
@@ -1594,7 +1599,7 @@ cudaError_t Conv::runT(const void *const *in, void *const *out, cudaStream_t s)
       fusedTables(P.fz,I.prec);
     } else if(P.direct) {
       P.fz=fusedRowPlan(a.m,I.prec,A,false,halfEmpty(a),P.nteam,
-                        widest(I.prec));
+                        widest(I.prec,a.m));
       fusedTables(P.fz,I.prec);
     } else P.fp=fftPlan(a.m,I.prec,inplaceFFT<T>(),true);
     P.twN=(const typename TwT<T>::type *) twiddles(a.N,I.prec);
@@ -1607,7 +1612,8 @@ cudaError_t Conv::runT(const void *const *in, void *const *out, cudaStream_t s)
     P.rpc=a.rpc;
     P.nteam=rowTeams(P.rpc,a.thr);
     P.io64=0;
-    P.fz=fusedRowPlan(a.N/2,I.prec,A,true,false,P.nteam,widest(I.prec));
+    P.fz=fusedRowPlan(a.N/2,I.prec,A,true,false,P.nteam,
+                      widest(I.prec,a.N/2));
     fusedTables(P.fz,I.prec);
     P.twN=(const typename TwT<T>::type *) twiddles(a.N,I.prec);
   };

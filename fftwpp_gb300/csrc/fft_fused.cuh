@@ -184,11 +184,12 @@ struct StageMap {
   int m, lg, lt, sh, step, skip;
   float inv;
   __device__ __forceinline__ StageMap(int R, int m, int lg, int lt)
-    : m(m), lg(lg), lt(lt), sh(-1), skip((R-1)*m), inv(1.0f/(float) m) {
-    step=(m >> lg ? spl(m,lg) : m) << lt;
+    : m(m), lg(lg), lt(lt), sh(-1), step(spl(m,lg) << lt), skip((R-1)*m),
+      inv(0.0f) {
 #ifdef __CUDA_ARCH__
     if((m & (m-1)) == 0) sh=__ffs(m)-1;
 #endif
+    if(sh < 0) inv=1.0f/(float) m;
   }
   __device__ __forceinline__ int block(int i) const {
     return sh >= 0 ? i >> sh : fdiv(i,inv);

@@ -49,11 +49,12 @@ struct UDiv {
   int sh;
   bool p2;
   __device__ __forceinline__ explicit UDiv(int d)
-    : inv(1.0f/(float) d), sh(0), p2((d & (d-1)) == 0)
+    : inv(0.0f), sh(0), p2((d & (d-1)) == 0)
   {
 #ifdef __CUDA_ARCH__
     sh=__ffs(d)-1;
 #endif
+    if(!p2) inv=1.0f/(float) d;
   }
   __device__ __forceinline__ int operator()(int a) const
   {

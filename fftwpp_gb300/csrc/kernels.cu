@@ -150,11 +150,7 @@ __device__ __forceinline__ void outerFwdTile(const OuterPlan<T>& P, int ctile,
     if(col < P.C) {
       cplx<T> v=X[sp(i)];
       long long k=(long long) r*m+j;
-      if(P.twX) {
-        unsigned long long e=((unsigned long long) col*(unsigned long long) k)
-          % (unsigned long long) P.NX;
-        v=twmul<1>(v,P.twX[e]);
-      }
+      if(P.twX) v=twmul<1>(v,P.twX[col*k]);   // col k < C m = NX
       dst[k*P.outRow+col]=v;
     }
   }
@@ -194,12 +190,18 @@ __device__ __forceinline__ void outerBwdTile(const OuterPlan<T>& P, int ctile,
     for(int i=tid; i < L*tile; i += nthr) acc[i]=mk((T) 0,(T) 0);
   for(int r=0; r < P.q; ++r) {
     if(CG) {
-      // Data written by other CTAs of this launch: L2 loads.
+      // Data written by other CTAs of this launch: L2 loads, four of a thread
+      // issued before the first is used, twiddled on the way.
+#pragma unroll 4
       for(int i=tid; i < m*tile; i += nthr) {
         int j=dTile(i), cc=i-j*tile;
         int col=col0+cc;
         cplx<T> v=mk((T) 0,(T) 0);
-        if(col < P.C) v=ldx<CG>(src+((long long) r*m+j)*P.inRow+col);
+        const long long k=(long long) r*m+j;
+        if(col < P.C) {
+          v=ldx<CG>(src+k*P.inRow+col);
+          if(P.twX) v=twmul<-1>(v,P.twX[col*k]);
+        }
         x[sp(i)]=v;
       }
     } else {
@@ -212,13 +214,12 @@ __device__ __forceinline__ void outerBwdTile(const OuterPlan<T>& P, int ctile,
       cpAsyncWait();
     }
     __syncthreads();
-    if(P.twX) {
+    if(!CG && P.twX) {
       for(int i=tid; i < m*tile; i += nthr) {
         int j=dTile(i), cc=i-j*tile;
-        unsigned long long e=((unsigned long long) (col0+cc)*
-                              (unsigned long long) ((long long) r*m+j)) %
-          (unsigned long long) P.NX;
-        x[sp(i)]=twmul<-1>(x[sp(i)],P.twX[e]);
+        int col=col0+cc;
+        if(col < P.C)
+          x[sp(i)]=twmul<-1>(x[sp(i)],P.twX[col*((long long) r*m+j)]);
       }
       __syncthreads();
     }
@@ -851,8 +852,15 @@ __device__ __forceinline__ Plan& stagePlan(unsigned char *buf, const Plan& src)
   return *(Plan *) buf;
 }
 
+// CTAs per SM: three in FP32 (512 uneven problems 592 us, with two 722), two in
+// FP64, whose registers three would spill (29 problems 215 against 246 us).
+template<typename T> constexpr int batchBlocks()
+{
+  return std::is_same<T,float>::value ? 3 : 2;
+}
+
 template<typename T, int K>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256,batchBlocks<T>())
 batchKernel(const BatchArgs<T> P)
 {
   extern __shared__ __align__(16) unsigned char smemRaw[];
