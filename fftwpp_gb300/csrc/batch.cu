@@ -68,7 +68,10 @@ std::vector<long> BatchConv::candidates(long L, long M, int A, int B,
   std::vector<std::pair<double,long>> c;
   for(long q=1; q <= 16; ++q) {
     long m=nextfftsize(ceilquotient(M,q));
-    if(m*q < M || rowNeedB(prec,L,m,A,B) > budget) continue;
+    // One residue of one fold takes the fused rows, without staging.
+    const size_t need=q == 1 && L <= m ? fusedNeedB(prec,m,A,false,1) :
+      rowNeedB(prec,L,m,A,B);
+    if(m*q < M || need > budget) continue;
     long p=ceilquotient(L,m);
     double cost=q*((A+B)*fftCostB(m)+A*p*(double) m+(A+B)*(double) m);
     bool dup=false;
@@ -368,6 +371,7 @@ void BatchConv::build()
       F.tile=tile; F.fp=fftPlanPublic(qc,prec,false);
       F.twN=(const Tw *) twiddles(qc,prec);
       F.twX=(const Tw *) twiddles(N,prec); F.NX=N;
+      F.twC=(const Tw *) twiddles(N,prec,256);
       F.count=A; F.nbatch=1; F.inBatch=F.outBatch=0;
       F.inRow=m; F.outRow=m; F.C=(int) m; F.Ltot=L; F.scale=(T) 1;
       for(int a=0; a < A; ++a) F.in[a]=(const cplx<T> *) (offsets[i]*e);

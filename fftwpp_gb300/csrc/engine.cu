@@ -164,21 +164,21 @@ static void *rootTable(const std::vector<double>& c,
   return d;
 }
 
-const void *twiddles(long n, int prec)
+const void *twiddles(long n, int prec, long step)
 {
   if(prec == PREC_FF) prec=PREC_F32;        // the same hi+lo float4 table
   static std::mutex mu;
-  static std::map<std::tuple<int,long,int>,void *> cache;
+  static std::map<std::tuple<int,long,int,long>,void *> cache;
   int dev=0;
   cudaGetDevice(&dev);
   std::lock_guard<std::mutex> lock(mu);
-  auto key=std::make_tuple(dev,n,prec);
+  auto key=std::make_tuple(dev,n,prec,step);
   auto it=cache.find(key);
   if(it != cache.end()) return it->second;
   std::vector<double> c, s;
   unitRoots(n,c,s);
-  std::vector<long> e(n);
-  for(long t=0; t < n; ++t) e[t]=t;
+  std::vector<long> e;
+  for(long t=0; t < n; t += step) e.push_back(t);
   void *d=rootTable(c,s,e,prec);
   if(d) cache[key]=d;
   return d;
@@ -1888,6 +1888,7 @@ cudaError_t Conv::runLong(const void *const *in, void *const *out,
   O.fp=fftPlan(q,I.prec);
   O.twN=(const typename TwT<T>::type *) twiddles(q,I.prec);
   O.twX=(const typename TwT<T>::type *) twiddles(N,I.prec);
+  O.twC=(const typename TwT<T>::type *) twiddles(N,I.prec,256);
   O.NX=N;
   O.io64=io64 & 1; O.ioShift=guard;
   O.conj=0;
@@ -2601,6 +2602,7 @@ cudaError_t PlainFFT::runTwoPass(const void *in, void *out, cudaStream_t s)
   if(sign > 0) {
     base(P,n1);
     P.twX=(const typename TwT<T>::type *) twiddles(n,prec); P.NX=n;
+    P.twC=(const typename TwT<T>::type *) twiddles(n,prec,256);
     P.tile=tile1;
     P.C=(int) n2; P.inRow=n2; P.outRow=n2;
     P.inBatch=ibatch; P.outBatch=n;
@@ -2623,6 +2625,7 @@ cudaError_t PlainFFT::runTwoPass(const void *in, void *out, cudaStream_t s)
   OuterPlan<T> Q{};
   base(Q,n1);
   Q.twX=(const typename TwT<T>::type *) twiddles(n,prec); Q.NX=n;
+  Q.twC=(const typename TwT<T>::type *) twiddles(n,prec,256);
   Q.tile=tile2;
   Q.C=(int) n2; Q.inRow=n2; Q.outRow=n2;
   Q.inBatch=n; Q.outBatch=obatch;

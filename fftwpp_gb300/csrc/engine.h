@@ -340,7 +340,7 @@ private:
                                               cudaStream_t s);
 };
 
-const void *twiddles(long n, int prec);
+const void *twiddles(long n, int prec, long step=1);   // every step-th t
 
 // Every device allocation of the library goes through devAlloc.  Failure
 // injection for tests (host side): failAllocationAfter(n) makes the n-th

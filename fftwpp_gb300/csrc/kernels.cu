@@ -25,6 +25,25 @@ __device__ __forceinline__ long long dataCol(const OuterPlan<T>& P, int col)
   return (long long) g*P.cs+(col-g*P.cz);
 }
 
+// The four-step twiddle W_NX^{col k} (col k < C m = NX).  FP32 multiplies two
+// entries that stay in L1, W^{e mod 256} and W^{e - e mod 256}, in
+// float-float (to 2^-44, far below the data's rounding): neighbouring
+// columns' entries lie k apart in the full table, so reading it moved 32
+// bytes from L2 for every 8 of data (512 uneven problems 576 us, against
+// TIMEHERE).  FP64, bound by its pipe, reads the table.
+template<typename T>
+__device__ __forceinline__ typename TwT<T>::type fourStep(const OuterPlan<T>& P,
+                                                          long long e)
+{
+  if constexpr(std::is_same<T,float>::value) {
+    const int i=(int) e;
+    const float4 a=ldtw(P.twX+(i & 255)), b=ldtw(P.twC+(i >> 8));
+    const cplx<ff> w=cmul(mk(ff(a.x,a.z),ff(a.y,a.w)),
+                          mk(ff(b.x,b.z),ff(b.y,b.w)));
+    return make_float4(w.x.hi,w.y.hi,w.x.lo,w.y.lo);
+  } else return P.twX[e];
+}
+
 // ---------------------------------------------------------------------------
 // Outer forward, complex data: residue block r of the padded transform along
 // a strided axis for `tile` adjacent columns.
@@ -150,7 +169,7 @@ __device__ __forceinline__ void outerFwdTile(const OuterPlan<T>& P, int ctile,
     if(col < P.C) {
       cplx<T> v=X[sp(i)];
       long long k=(long long) r*m+j;
-      if(P.twX) v=twmul<1>(v,P.twX[col*k]);   // col k < C m = NX
+      if(P.twX) v=twmul<1>(v,fourStep(P,col*k));
       dst[k*P.outRow+col]=v;
     }
   }
@@ -200,7 +219,7 @@ __device__ __forceinline__ void outerBwdTile(const OuterPlan<T>& P, int ctile,
         const long long k=(long long) r*m+j;
         if(col < P.C) {
           v=ldx<CG>(src+k*P.inRow+col);
-          if(P.twX) v=twmul<-1>(v,P.twX[col*k]);
+          if(P.twX) v=twmul<-1>(v,fourStep(P,col*k));
         }
         x[sp(i)]=v;
       }
@@ -219,7 +238,8 @@ __device__ __forceinline__ void outerBwdTile(const OuterPlan<T>& P, int ctile,
         int j=dTile(i), cc=i-j*tile;
         int col=col0+cc;
         if(col < P.C)
-          x[sp(i)]=twmul<-1>(x[sp(i)],P.twX[col*((long long) r*m+j)]);
+          x[sp(i)]=twmul<-1>(x[sp(i)],
+                             fourStep(P,col*((long long) r*m+j)));
       }
       __syncthreads();
     }

@@ -158,6 +158,7 @@ struct OuterPlan {
   FusedFFT fz;             // the fused kernels' length-m (N/2) FFT
   const typename TwT<T>::type *twN;
   const typename TwT<T>::type *twX;  // optional W_NX^{col*k} (1D long path)
+  const typename TwT<T>::type *twC;  // FP32: W_NX^{256 i} (fourStep)
   long long NX;
 };
 
