@@ -48,13 +48,15 @@ static size_t fusedNeedB(int prec, long m, int A, bool half, int nteam)
     fusedRowSmem<float>(p.n,p.lg,A,nteam);
 }
 
-static size_t outerNeedB(int prec, long L, long m, int tile)
+FusedFFT fusedColumnPlan(long n, int prec, bool half, int tile);
+
+// Shared memory of a column task of a long problem: tile columns of n points,
+// L of them data.
+static size_t outerNeedB(int prec, long L, long n, int tile)
 {
-  size_t f=prec == PREC_F64 ? outerFwdSmem<double>(L,m,tile) :
-    outerFwdSmem<float>(L,m,tile);
-  size_t b=prec == PREC_F64 ? outerBwdSmem<double>(L,m,tile) :
-    outerBwdSmem<float>(L,m,tile);
-  return std::max(f,b);
+  const FusedFFT p=fusedColumnPlan(n,prec,2*L <= n,tile);
+  return prec == PREC_F64 ? fusedOuterSmem<double>(L,p.n,p.lg,tile,1) :
+    fusedOuterSmem<float>(L,p.n,p.lg,tile,1);
 }
 
 static double fftCostB(long m) {return m*std::log2((double) std::max(m,2L));}
@@ -368,7 +370,10 @@ void BatchConv::build()
       stagingBytes += e*(size_t) N*A;
       OuterPlan<T>& F=P.fwd;
       F.L=(int) pc; F.m=(int) qc; F.q=1; F.N=(int) qc; F.cshift=0;
-      F.tile=tile; F.fp=fftPlanPublic(qc,prec,false);
+      F.tile=tile;
+      F.fused=1;
+      F.fz=fusedColumnPlan(qc,prec,2*pc <= qc,tile);
+      fusedRowTables(F.fz,prec);
       F.twN=(const Tw *) twiddles(qc,prec);
       F.twX=(const Tw *) twiddles(N,prec); F.NX=N;
       F.twC=(const Tw *) twiddles(N,prec,256);

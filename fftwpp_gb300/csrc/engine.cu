@@ -358,7 +358,7 @@ static FusedFFT fusedPlan(long n, int prec, int A, bool herm, bool half,
   p.half=half && rad[0] % 2 == 0;
   p.twb=p.twj=NULL;
   p.pairs=NULL;
-  p.pos=NULL;
+  p.pos=p.rev=NULL;
   const size_t e=prec == PREC_F32 ? 8 : 16;
   for(int level=0; level < 3; ++level) {
     p.lg=level < 2 ? fusedPadding(rad,p.nst,level) : 30;
@@ -374,7 +374,7 @@ static void fusedTables(FusedFFT& p, int prec)
 {
   if(prec == PREC_FF) prec=PREC_F32;
   static std::mutex mu;
-  struct Tables {void *twb, *twj, *pairs, *pos;};
+  struct Tables {void *twb, *twj, *pairs, *pos, *rev;};
   static std::map<std::tuple<int,int,std::string>,Tables> cache;
   int dev=0;
   cudaGetDevice(&dev);
@@ -391,12 +391,14 @@ static void fusedTables(FusedFFT& p, int prec)
     std::vector<long> rev(p.radix[0]);
     for(long b=0; b < nblk; ++b) rev[b]=b;
     std::vector<int4> pairs;
+    std::vector<int> blocks;
     for(int st=1; st < p.nst; ++st) {
       const int R=p.radix[st];
       for(int r=1; r < R; ++r)
         for(long b=0; b < nblk; ++b)
           eb.push_back(r*rev[b]*(n/(nblk*R)) % n);
       if(st == p.nst-1) {
+        blocks.assign(rev.begin(),rev.end());
         // Partner blocks of the last stage: rev(b) and nblk - rev(b).
         std::vector<int> at(nblk);
         for(long b=0; b < nblk; ++b) at[rev[b]]=(int) b;
@@ -425,23 +427,27 @@ static void fusedTables(FusedFFT& p, int prec)
     Tables t;
     t.twb=rootTable(c,s,eb,prec);
     t.twj=rootTable(c,s,ej,prec);
-    t.pairs=t.pos=NULL;
+    t.pairs=t.pos=t.rev=NULL;
     std::vector<int> pos(n);
     for(long b=0; b < n; ++b) pos[rev[b]]=(int) b;
     const size_t pb=pairs.size()*sizeof(int4), nb=n*sizeof(int);
+    const size_t rb=blocks.size()*sizeof(int);
     if(!t.twb || !t.twj || devAlloc(&t.pairs,pb) != cudaSuccess ||
-       devAlloc(&t.pos,nb) != cudaSuccess) {
-      for(void *q : {t.twb,t.twj,t.pairs,t.pos}) if(q) cudaFree(q);
+       devAlloc(&t.pos,nb) != cudaSuccess ||
+       devAlloc(&t.rev,rb) != cudaSuccess) {
+      for(void *q : {t.twb,t.twj,t.pairs,t.pos,t.rev}) if(q) cudaFree(q);
       throw std::runtime_error("twiddle table allocation failed");
     }
     cudaMemcpy(t.pairs,pairs.data(),pb,cudaMemcpyHostToDevice);
     cudaMemcpy(t.pos,pos.data(),nb,cudaMemcpyHostToDevice);
+    cudaMemcpy(t.rev,blocks.data(),rb,cudaMemcpyHostToDevice);
     it=cache.emplace(key,t).first;
   }
   p.twb=it->second.twb;
   p.twj=it->second.twj;
   p.pairs=(const int4 *) it->second.pairs;
   p.pos=(const int *) it->second.pos;
+  p.rev=(const int *) it->second.rev;
 }
 
 // Teams of a fused row launch: one per row where a team keeps at least eight
@@ -468,6 +474,12 @@ FusedFFT fusedRowPlan(long n, int prec, int A, bool herm, bool half,
 }
 
 void fusedRowTables(FusedFFT& p, int prec) {fusedTables(p,prec);}
+
+// The fused column transforms of the batched launch's long problems.
+FusedFFT fusedColumnPlan(long n, int prec, bool half, int tile)
+{
+  return fusedPlan(n,prec,1,false,half,8,tile);
+}
 
 // ---------------------------------------------------------------------------
 // Planning.

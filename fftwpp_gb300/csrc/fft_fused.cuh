@@ -58,6 +58,7 @@ struct FusedFFT {
                            // partner, rev(block)), ceil(nblk/2) entries
   const int *pos;          // position of natural index k after the last
                            // forward stage
+  const int *rev;          // rev(b) of the last stage's blocks
 };
 
 // Whether a plan holds a radix-16 stage (its kernels need the WIDE form).

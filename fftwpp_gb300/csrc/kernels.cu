@@ -47,7 +47,7 @@ __device__ __forceinline__ typename TwT<T>::type fourStep(const OuterPlan<T>& P,
 // ---------------------------------------------------------------------------
 // Outer forward, complex data: residue block r of the padded transform along
 // a strided axis for `tile` adjacent columns.
-template<typename T, bool CG>
+template<typename T>
 __device__ __forceinline__ void outerFwdTile(const OuterPlan<T>& P, int ctile,
                                              int r, int z,
                                              unsigned char *smemRaw)
@@ -181,11 +181,11 @@ __global__ void __launch_bounds__(256)
 outerFwdKernel(const OuterPlan<T> P)
 {
   extern __shared__ __align__(16) unsigned char smemRaw[];
-  outerFwdTile<T,false>(P,blockIdx.x,blockIdx.y,blockIdx.z,smemRaw);
+  outerFwdTile<T>(P,blockIdx.x,blockIdx.y,blockIdx.z,smemRaw);
 }
 
 // Outer backward, complex data: all residues of a column tile, accumulated.
-template<typename T, bool CG>
+template<typename T>
 __device__ __forceinline__ void outerBwdTile(const OuterPlan<T>& P, int ctile,
                                              int z, unsigned char *smemRaw)
 {
@@ -208,32 +208,15 @@ __device__ __forceinline__ void outerBwdTile(const OuterPlan<T>& P, int ctile,
   if(!direct)
     for(int i=tid; i < L*tile; i += nthr) acc[i]=mk((T) 0,(T) 0);
   for(int r=0; r < P.q; ++r) {
-    if(CG) {
-      // Data written by other CTAs of this launch: L2 loads, four of a thread
-      // issued before the first is used, twiddled on the way.
-#pragma unroll 4
-      for(int i=tid; i < m*tile; i += nthr) {
-        int j=dTile(i), cc=i-j*tile;
-        int col=col0+cc;
-        cplx<T> v=mk((T) 0,(T) 0);
-        const long long k=(long long) r*m+j;
-        if(col < P.C) {
-          v=ldx<CG>(src+k*P.inRow+col);
-          if(P.twX) v=twmul<-1>(v,fourStep(P,col*k));
-        }
-        x[sp(i)]=v;
-      }
-    } else {
-      for(int i=tid; i < m*tile; i += nthr) {
-        int j=dTile(i), cc=i-j*tile;
-        int col=col0+cc;
-        if(col < P.C) cpAsync(x+sp(i),src+((long long) r*m+j)*P.inRow+col);
-        else x[sp(i)]=mk((T) 0,(T) 0);
-      }
-      cpAsyncWait();
+    for(int i=tid; i < m*tile; i += nthr) {
+      int j=dTile(i), cc=i-j*tile;
+      int col=col0+cc;
+      if(col < P.C) cpAsync(x+sp(i),src+((long long) r*m+j)*P.inRow+col);
+      else x[sp(i)]=mk((T) 0,(T) 0);
     }
+    cpAsyncWait();
     __syncthreads();
-    if(!CG && P.twX) {
+    if(P.twX) {
       for(int i=tid; i < m*tile; i += nthr) {
         int j=dTile(i), cc=i-j*tile;
         int col=col0+cc;
@@ -303,7 +286,7 @@ __global__ void __launch_bounds__(256)
 outerBwdKernel(const OuterPlan<T> P)
 {
   extern __shared__ __align__(16) unsigned char smemRaw[];
-  outerBwdTile<T,false>(P,blockIdx.x,blockIdx.z,smemRaw);
+  outerBwdTile<T>(P,blockIdx.x,blockIdx.z,smemRaw);
 }
 
 // ---------------------------------------------------------------------------
@@ -369,29 +352,48 @@ __device__ __forceinline__ void outerLastFwd(const OuterPlan<T>& P,
     for(int r=0; r < R; ++r) a[0][r]=nrm(xq[r << lt]);
     inTwiddleDFT<T,R,1>(a,tw,b,nblk);
     if(col >= P.C) continue;
+    if(P.twX) {
+      // Position b R + r holds entry rev(b) + r nblk.
+      const int k=P.fz.rev[b];
+#pragma unroll
+      for(int r=0; r < R; ++r)
+        a[0][r]=twmul<1>(a[0][r],fourStep(P,(long long) col*(k+r*nblk)));
+    }
     cplx<T> *d=dst+(long long) (b*R)*P.outRow+col;
 #pragma unroll
     for(int r=0; r < R; ++r) d[r*P.outRow]=a[0][r];
   }
 }
 
+// Data entries of column col: all L, but for the flattened rows of the
+// batched launch (twX), whose last one may be short.
+template<typename T>
+__device__ __forceinline__ int columnTop(const OuterPlan<T>& P, int col,
+                                         long long row)
+{
+  if(col >= P.C) return 0;
+  if(!P.twX) return P.L;
+  return ((int) P.Ltot-col+(int) row-1)/(int) row;
+}
+
 template<typename T, bool WIDE>
-__device__ __forceinline__ void outerFwdFused(const OuterPlan<T>& P,
+__device__ __forceinline__ void outerFwdFused(const OuterPlan<T>& P, int ctile,
+                                              int r, int z,
                                               unsigned char *smemRaw)
 {
   const int tile=P.tile, m=P.m, N=P.N, c=P.cshift, L=P.L;
   cplx<T> *x=(cplx<T> *) smemRaw;
   const int tid=threadIdx.x, nthr=blockDim.x;
-  const int col0=blockIdx.x*tile, r=blockIdx.y;
-  const int a=blockIdx.z % P.count;
-  const long long batch=blockIdx.z/P.count;
+  const int col0=ctile*tile;
+  const int a=z % P.count;
+  const long long batch=z/P.count;
   const cplx<T> *src=P.in[a]+batch*P.inBatch;
   cplx<T> *dst=P.out[a]+batch*P.outBatch+(long long) r*m*P.outRow;
   const int lt=log2of(tile);
   const int sh=ioShift<T>(P.ioShift,a);
   const auto load=[&](int, int cc) {
-    const int top=col0+cc < P.C ? L : 0;      // entries of a column that
-    const cplx<T> *f=src+dataCol(P,col0+cc);  // exists
+    const int top=columnTop(P,col0+cc,P.inRow);
+    const cplx<T> *f=src+dataCol(P,col0+cc);
     return [=,&P](int j) {
       int s=j+c;
       if(s >= m) s -= m;
@@ -436,11 +438,11 @@ __global__ void __launch_bounds__(256)
 outerFwdFusedKernel(const OuterPlan<T> P)
 {
   extern __shared__ __align__(16) unsigned char smemRaw[];
-  outerFwdFused<T,false>(P,smemRaw);
+  outerFwdFused<T,false>(P,blockIdx.x,blockIdx.y,blockIdx.z,smemRaw);
 }
 
 // The first inverse stage: staging rows into shared memory.
-template<typename T, int R>
+template<typename T, int R, bool CG>
 __device__ __forceinline__ void outerFirstInv(const OuterPlan<T>& P,
                                               cplx<T> *x, const cplx<T> *src,
                                               int col0, int tid, int nthr)
@@ -454,7 +456,13 @@ __device__ __forceinline__ void outerFirstInv(const OuterPlan<T>& P,
     cplx<T> a[R];
 #pragma unroll
     for(int r=0; r < R; ++r)
-      a[r]=col < P.C ? s[r*P.inRow] : mk((T) 0,(T) 0);
+      a[r]=col < P.C ? ldx<CG>(s+r*P.inRow) : mk((T) 0,(T) 0);
+    if(P.twX && col < P.C) {
+      const int k=P.fz.rev[b], nblk=p.n/R;
+#pragma unroll
+      for(int r=0; r < R; ++r)
+        a[r]=twmul<-1>(a[r],fourStep(P,(long long) col*(k+r*nblk)));
+    }
 #pragma unroll
     for(int r=0; r < R; ++r) a[r]=nrm(swapXY(a[r]));
     Codelet<R,1,T>::run(a);
@@ -466,17 +474,17 @@ __device__ __forceinline__ void outerFirstInv(const OuterPlan<T>& P,
 
 // All residues of a column tile; with several, a thread adds the outputs it
 // computes into its own entries of an accumulator behind the tile.
-template<typename T, bool WIDE>
-__device__ __forceinline__ void outerBwdFused(const OuterPlan<T>& P,
-                                              unsigned char *smemRaw)
+template<typename T, bool WIDE, bool CG>
+__device__ __forceinline__ void outerBwdFused(const OuterPlan<T>& P, int ctile,
+                                              int z, unsigned char *smemRaw)
 {
   const int tile=P.tile, m=P.m, N=P.N, c=P.cshift, L=P.L, q=P.q;
   cplx<T> *x=(cplx<T> *) smemRaw;
   cplx<T> *acc=x+fusedSpan(P.fz.n,P.fz.lg)*tile;
   const int tid=threadIdx.x, nthr=blockDim.x;
-  const int col0=blockIdx.x*tile;
-  const int b=blockIdx.z % P.count;
-  const long long batch=blockIdx.z/P.count;
+  const int col0=ctile*tile;
+  const int b=z % P.count;
+  const long long batch=z/P.count;
   const cplx<T> *src=P.in[b]+batch*P.inBatch;
   cplx<T> *dst=P.out[b]+batch*P.outBatch;
   const int lt=log2of(tile);
@@ -484,7 +492,7 @@ __device__ __forceinline__ void outerBwdFused(const OuterPlan<T>& P,
   for(int r=0; r < q; ++r) {
     const cplx<T> *sr=src+(long long) r*m*P.inRow;
     const auto store=[&](int, int cc) {
-      const int top=col0+cc < P.C ? L : 0;
+      const int top=columnTop(P,col0+cc,P.outRow);
       cplx<T> *f=dst+dataCol(P,col0+cc);
       return [=,&P](int j, cplx<T> v) {
         int s=j+c;
@@ -510,7 +518,7 @@ __device__ __forceinline__ void outerBwdFused(const OuterPlan<T>& P,
       storeTileFF(x,P.fz,lt,tid,nthr,store);
     } else {
       FGB_FUSED_SWITCH(P.fz.radix[P.fz.nst-1],
-                       (outerFirstInv<T,R_>(P,x,sr,col0,tid,nthr)))
+                       (outerFirstInv<T,R_,CG>(P,x,sr,col0,tid,nthr)))
       runFusedMiddle<T,WIDE>(x,0,1,P.fz,lt,true,0,tid,nthr);
       __syncthreads();
       runFusedLast<T,WIDE>(x,0,1,P.fz,lt,tid,nthr,store);
@@ -524,7 +532,7 @@ __global__ void __launch_bounds__(256)
 outerBwdFusedKernel(const OuterPlan<T> P)
 {
   extern __shared__ __align__(16) unsigned char smemRaw[];
-  outerBwdFused<T,false>(P,smemRaw);
+  outerBwdFused<T,false,false>(P,blockIdx.x,blockIdx.z,smemRaw);
 }
 
 // FP32 plans with a radix-16 stage: their own instantiations, capped at 85
@@ -535,7 +543,7 @@ __global__ void __launch_bounds__(256,3)
 outerFwdFusedKernel16(const OuterPlan<T> P)
 {
   extern __shared__ __align__(16) unsigned char smemRaw[];
-  outerFwdFused<T,true>(P,smemRaw);
+  outerFwdFused<T,true>(P,blockIdx.x,blockIdx.y,blockIdx.z,smemRaw);
 }
 
 template<typename T>
@@ -543,7 +551,7 @@ __global__ void __launch_bounds__(256,3)
 outerBwdFusedKernel16(const OuterPlan<T> P)
 {
   extern __shared__ __align__(16) unsigned char smemRaw[];
-  outerBwdFused<T,true>(P,smemRaw);
+  outerBwdFused<T,true,false>(P,blockIdx.x,blockIdx.z,smemRaw);
 }
 
 // ---------------------------------------------------------------------------
@@ -943,8 +951,9 @@ batchKernel(const BatchArgs<T> P)
         rebase(O,O.count,fwd && (rel & 4),!fwd && (rel & 8),P.inBase,
                P.outBase);
       __syncthreads();
-      if(fwd) outerFwdTile<T,false>(O,tk.i,0,tk.j,smemRaw);
-      else outerBwdTile<T,true>(O,tk.i,tk.j,smemRaw);
+      if(fwd) outerFwdFused<T,false>(O,tk.i,0,tk.j,smemRaw);
+      else outerBwdFused<T,false,true>(O,tk.i,tk.j,smemRaw);
+      __syncthreads();
     }
     if(tk.type == TASK_COLFWD || tk.type == TASK_ROW) {
       __threadfence();
