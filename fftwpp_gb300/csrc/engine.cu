@@ -960,6 +960,7 @@ Conv::Conv(int dim, const int *kinds, const long *L, const long *M,
                    return innerNeed(I,in,r,256);});
   try {
     allocate();
+    makeTables();
     if(autotune && tuneSchedule) tune();
   } catch(...) {
     // A throwing constructor runs no destructor: release what was taken.
@@ -1991,6 +1992,19 @@ cudaError_t Conv::runHostWith(const RowLaunchers *L, const void *const *in,
   return e;
 }
 
+// No exception leaves a launch sequence (its callers are C entries): a table
+// that cannot be allocated is an error status.
+template<class F>
+static cudaError_t noThrow(const F& run)
+{
+  try {
+    return run();
+  } catch(std::exception& x) {
+    setLastError(x.what());
+    return cudaErrorMemoryAllocation;
+  }
+}
+
 cudaError_t Conv::run(const void *const *in, void *const *out, cudaStream_t s)
 {
   if(I.mult == MULT_USER && !user && !tuning) {
@@ -2001,9 +2015,40 @@ cudaError_t Conv::run(const void *const *in, void *const *out, cudaStream_t s)
   }
   marks=0;
   tick(s);
-  if(I.prec == PREC_F64) return runT<double>(in,out,s);
-  if(I.prec == PREC_F32) return runT<float>(in,out,s);
-  return runT<ff>(in,out,s);        // float-float, FP64 at the interface
+  return noThrow([&] {
+      if(I.prec == PREC_F64) return runT<double>(in,out,s);
+      if(I.prec == PREC_F32) return runT<float>(in,out,s);
+      return runT<ff>(in,out,s);    // float-float, FP64 at the interface
+    });
+}
+
+// The tables of the fused transforms, made with the plan: its first run may
+// be under stream capture, where nothing can be allocated.
+void Conv::makeTables()
+{
+  auto make=[&](FusedFFT p) {fusedTables(p,I.prec);};
+  for(int d=0; d < I.dim-1; ++d) {
+    const AxisPlan& a=I.axis[d];
+    if(outerFused(a)) make(outerFFT(a,I.prec,1));
+    else if(a.kind == KIND_REAL) make(realFFT(a.N,a.L,I.prec,1));
+  }
+  const AxisPlan& a=I.axis[I.dim-1];
+  long nrows=batch;
+  for(int d=0; d < I.dim-1; ++d) nrows *= I.axis[d].rows;
+  const int A=I.A;
+  if(I.longRow) {
+    make(fusedRowPlan(I.rowM,I.prec,A,false,false,1,widest(I.prec)));
+    return;
+  }
+  if(a.kind == KIND_HERMITIAN) {
+    make(fusedRowPlan(a.N/2,I.prec,A,true,false,1,widest(I.prec,a.N/2)));
+    return;
+  }
+  const int split=I.mult != MULT_USER ? rowSplit(a.N,nrows,I.prec) : 1;
+  if(split > 1) make(fusedRowPlan(a.N/split,I.prec,A,false,false,1,8));
+  if(rowDirect(a))
+    make(fusedRowPlan(a.m,I.prec,A,false,halfEmpty(a),1,
+                      widest(I.prec,a.m)));
 }
 
 bool Conv::zeroCopy=true;
@@ -2495,14 +2540,18 @@ cudaError_t PadTransform::runT(const void *in, void *out, bool fwd,
 
 cudaError_t PadTransform::forward(const void *f, void *F, cudaStream_t s)
 {
-  return prec == PREC_F64 ? runT<double>(f,F,true,s) :
-    runT<float>(f,F,true,s);
+  return noThrow([&] {
+      return prec == PREC_F64 ? runT<double>(f,F,true,s) :
+        runT<float>(f,F,true,s);
+    });
 }
 
 cudaError_t PadTransform::backward(const void *F, void *f, cudaStream_t s)
 {
-  return prec == PREC_F64 ? runT<double>(F,f,false,s) :
-    runT<float>(F,f,false,s);
+  return noThrow([&] {
+      return prec == PREC_F64 ? runT<double>(F,f,false,s) :
+        runT<float>(F,f,false,s);
+    });
 }
 
 // ---------------------------------------------------------------------------
@@ -2688,10 +2737,12 @@ bool PlainFFT::aligned(const void *in, const void *out) const
 
 cudaError_t PlainFFT::execute(const void *in, void *out, cudaStream_t s)
 {
-  if(n1 > 0)
-    return prec == PREC_F64 ? runTwoPass<double>(in,out,s) :
-      runTwoPass<float>(in,out,s);
-  return prec == PREC_F64 ? runT<double>(in,out,s) : runT<float>(in,out,s);
+  return noThrow([&] {
+      if(n1 > 0)
+        return prec == PREC_F64 ? runTwoPass<double>(in,out,s) :
+          runTwoPass<float>(in,out,s);
+      return prec == PREC_F64 ? runT<double>(in,out,s) : runT<float>(in,out,s);
+    });
 }
 
 } // namespace fgb

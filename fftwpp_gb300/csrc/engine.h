@@ -253,6 +253,7 @@ private:
   cudaEvent_t outDone[CHUNKS], outCopied;
   cudaError_t planOutputs(cudaStream_t s);
   void allocate();
+  void makeTables();
   void tune();
   bool directSegments() const;
   cudaError_t runZeroCopy(const void *const *hin, const void *const *in,

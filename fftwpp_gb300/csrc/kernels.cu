@@ -29,8 +29,8 @@ __device__ __forceinline__ long long dataCol(const OuterPlan<T>& P, int col)
 // entries that stay in L1, W^{e mod 256} and W^{e - e mod 256}, in
 // float-float (to 2^-44, far below the data's rounding): neighbouring
 // columns' entries lie k apart in the full table, so reading it moved 32
-// bytes from L2 for every 8 of data (512 uneven problems 576 us, against
-// TIMEHERE).  FP64, bound by its pipe, reads the table.
+// bytes from L2 for every 8 of data (512 uneven problems 576 us, 490 this
+// way).  FP64, bound by its pipe, reads the table.
 template<typename T>
 __device__ __forceinline__ typename TwT<T>::type fourStep(const OuterPlan<T>& P,
                                                           long long e)
@@ -299,8 +299,8 @@ outerBwdKernel(const OuterPlan<T> P)
 // the last.
 // Float-float (runStages): the tile's inputs into shared memory, and its
 // outputs out of it.  in(cc, j) gives element j of column cc.
-template<class In>
-__device__ __forceinline__ void loadTileFF(cplx<ff> *x, const FusedFFT& p,
+template<typename T, class In>
+__device__ __forceinline__ void loadTileFF(cplx<T> *x, const FusedFFT& p,
                                            int lt, int tid, int nthr,
                                            const In& in)
 {
@@ -313,6 +313,8 @@ __device__ __forceinline__ void loadTileFF(cplx<ff> *x, const FusedFFT& p,
 
 // FP64 bits read as a float-float value, converted in line (one place, whose
 // loads the loop issues together).
+template<typename T>
+__device__ __forceinline__ cplx<T> fromBits(cplx<T> v, int) {return v;}
 __device__ __forceinline__ cplx<ff> fromBits(cplx<ff> v, int sh)
 {
   return mk(toFF(__hiloint2double(__float_as_int(v.x.lo),
@@ -321,8 +323,8 @@ __device__ __forceinline__ cplx<ff> fromBits(cplx<ff> v, int sh)
                                   __float_as_int(v.y.hi)),sh));
 }
 
-template<class Store>
-__device__ __forceinline__ void storeTileFF(const cplx<ff> *x,
+template<typename T, class Store>
+__device__ __forceinline__ void storeTileFF(const cplx<T> *x,
                                             const FusedFFT& p, int lt, int tid,
                                             int nthr, const Store& store)
 {
@@ -376,6 +378,17 @@ __device__ __forceinline__ int columnTop(const OuterPlan<T>& P, int col,
   return ((int) P.Ltot-col+(int) row-1)/(int) row;
 }
 
+// Whether a fused outer launch takes the staged form: float-float with few
+// columns, where fetching the code dominates (39 x 93 convolution 43 us fused,
+// 34 staged), not from 1024 on, where the pruned halves count (3D real 256^3,
+// y transforms of 131 584 columns back 558 us staged, 416 before).
+template<typename T>
+__device__ __forceinline__ bool stagedColumns(const OuterPlan<T>& P)
+{
+  return std::is_same<T,ff>::value &&
+    (long long) P.C*P.nbatch*P.count < 1024;
+}
+
 template<typename T, bool WIDE>
 __device__ __forceinline__ void outerFwdFused(const OuterPlan<T>& P, int ctile,
                                               int r, int z,
@@ -405,7 +418,7 @@ __device__ __forceinline__ void outerFwdFused(const OuterPlan<T>& P, int ctile,
       return v;
     };
   };
-  if constexpr(std::is_same<T,ff>::value) {
+  if(stagedColumns(P)) {
     loadTileFF(x,P.fz,lt,tid,nthr,[&](int cc, int j) {
         int s=j+c;
         if(s >= m) s -= m;
@@ -509,7 +522,7 @@ __device__ __forceinline__ void outerBwdFused(const OuterPlan<T>& P, int ctile,
         storeIO(f+s*P.outRow,v*P.scale,P.io64 & 2,sh);
       };
     };
-    if constexpr(std::is_same<T,ff>::value) {
+    if(stagedColumns(P)) {
       loadTileFF(x,P.fz,lt,tid,nthr,[&](int cc, int j) {
           return col0+cc < P.C ? swapXY(sr[j*P.inRow+col0+cc]) :
             mk((T) 0,(T) 0);
