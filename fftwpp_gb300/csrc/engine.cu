@@ -794,8 +794,10 @@ static int pickTile(int maxTile, long C, long factor, F smem, int minTile=1)
   return tile;
 }
 
+// natural: the caller launches the natural-order kernels (two buffers a tile)
+// whatever the fold count, so their shared memory sizes the complex tiles.
 static void planOuter(AxisPlan& a, long mForce, int prec, long C, long nbatch,
-                      int A, int B)
+                      int A, int B, bool natural=false)
 {
   int maxTile=wide(prec) ? 8 : 16;
   int minTile=wide(prec) ? 2 : 4;
@@ -832,8 +834,14 @@ static void planOuter(AxisPlan& a, long mForce, int prec, long C, long nbatch,
   a.p=ceilquotient(a.L,a.m);
   a.cshift=centered ? (int) (a.L/2) : 0;
   a.rows=a.N;
-  auto smf=[&](int t) {return outerFwdNeed(a,prec,t);};
-  auto smb=[&](int t) {return outerBwdNeed(a,prec,t);};
+  auto smf=[&](int t) {
+    return natural ? FGB_BY_PREC(prec,outerFwdSmem,a.L,a.m,t) :
+      outerFwdNeed(a,prec,t);
+  };
+  auto smb=[&](int t) {
+    return natural ? FGB_BY_PREC(prec,outerBwdSmem,a.L,a.m,t,(int) a.q) :
+      outerBwdNeed(a,prec,t);
+  };
   a.tile=pickTile(maxTile,C,nbatch*a.q*A,smf,minTile);
   a.tileB=pickTile(maxTile,C,nbatch*B,smb,minTile);
   if(smf(a.tile) > SMEM_MAX || smb(a.tileB) > SMEM_MAX)
@@ -2486,7 +2494,7 @@ PadTransform::PadTransform(int kind, long L, long M, long C, long mForce,
     a.tileB=a.tile;
     return;
   }
-  planOuter(a,mForce,prec,C,1,1,1);
+  planOuter(a,mForce,prec,C,1,1,1,true);
 }
 
 size_t PadTransform::inElements() const {return (size_t) a.stored*C;}
