@@ -63,16 +63,19 @@ static double fftCostB(long m) {return m*std::log2((double) std::max(m,2L));}
 
 // Candidate plans of one problem, cheapest (by the cost model) first.
 // choice > 0: short problem with residue block m = choice;
-// choice < 0: long problem with row length -choice.
+// choice < 0: long problem with row length -choice.  longer: whether any
+// padded length >= M gives the same results (anyLength); where it does not,
+// the staged rows' shared memory decides which lengths there are, and the
+// cheapest candidate's is the only one.
 std::vector<long> BatchConv::candidates(long L, long M, int A, int B,
-                                        int prec, size_t budget)
+                                        int prec, size_t budget, bool longer)
 {
   std::vector<std::pair<double,long>> c;
   for(long q=1; q <= 16; ++q) {
     long m=nextfftsize(ceilquotient(M,q));
     // One residue of one fold takes the fused rows, without staging.
-    const size_t need=q == 1 && L <= m ? fusedNeedB(prec,m,A,false,1) :
-      rowNeedB(prec,L,m,A,B);
+    const size_t need=q == 1 && L <= m && longer ?
+      fusedNeedB(prec,m,A,false,1) : rowNeedB(prec,L,m,A,B);
     if(m*q < M || need > budget) continue;
     long p=ceilquotient(L,m);
     double cost=q*((A+B)*fftCostB(m)+A*p*(double) m+(A+B)*(double) m);
@@ -93,8 +96,11 @@ std::vector<long> BatchConv::candidates(long L, long M, int A, int B,
     }
   }
   std::sort(c.begin(),c.end());
+  auto length=[&](long m) {return m > 0 ? m*(long) ceilquotient(M,m) : 0;};
   std::vector<long> out;
-  for(auto& x : c) out.push_back(x.second);
+  for(auto& x : c)
+    if(longer || length(x.second) == length(c[0].second))
+      out.push_back(x.second);
   return out;
 }
 
@@ -130,7 +136,8 @@ BatchConv::BatchConv(int nprob, const long *L, const long *M,
   choices.resize(nprob);
   for(int i=0; i < nprob; ++i) {
     if(choice && choice[i]) {choices[i]=choice[i]; continue;}
-    std::vector<long> cand=candidates(Ls[i],Ms[i],A,B,prec,budget);
+    std::vector<long> cand=candidates(Ls[i],Ms[i],A,B,prec,budget,
+                                      anyLength(kind,Ls[i],Ms[i],mult));
     if(cand.empty())
       throw std::runtime_error("no batched plan for L="+std::to_string(Ls[i]));
     choices[i]=tune ? tuned(Ls[i],Ms[i],cand) : cand[0];

@@ -58,7 +58,7 @@ public:
   int outputs() const {return B;}
 
   static std::vector<long> candidates(long L, long M, int A, int B, int prec,
-                                      size_t budget);
+                                      size_t budget, bool longer);
 
 private:
   int n, A, B, mult, prec, kind;

@@ -1101,6 +1101,25 @@ int fgb_fft_radices(size_t n, int precision, int inplace, int wide,
   return nst;
 }
 
+int fgb_row_length(int kind, size_t L, size_t M, size_t m, int A, int B,
+                   int mult, int precision, long *info)
+{
+  if(!info || L < 1 || L > M || kind < KIND_PAD || kind > KIND_REAL ||
+     B < 1 || A < B || A > FGB_MAXA || precision < PREC_F64 ||
+     precision > PREC_FF) {
+    setLastError("fgb_row_length: bad arguments");
+    return -1;
+  }
+  try {
+    info[3]=anyLength(kind,(long) L,(long) M,mult) ? 1 : 0;
+    return planRowLength(kind,(long) L,(long) M,(long) m,A,B,mult,precision,
+                         info,info+1,info+2) ? 1 : 0;
+  } catch(std::exception& e) {
+    report("fgb_row_length",e.what());
+    return -1;
+  }
+}
+
 int fgb_fused_radices(size_t n, int precision, int inputs, int hermitian,
                       int half, int *radix, int max, int *padding)
 {

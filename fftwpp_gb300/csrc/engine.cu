@@ -659,9 +659,16 @@ static std::vector<long> paddedLengths(long M)
 }
 
 // Estimated arithmetic instructions of a row axis with residue blocks of m
-// points and q residues: the fused rows for one residue of one fold, else
-// transforms, the fold (a complex twiddle per term for residues r > 0) and
-// the post-twiddled accumulation.
+// points and q residues: transforms, the fold (a complex twiddle per term
+// for residues r > 0) and the post-twiddled accumulation.
+static double stagedRowCost(const AxisPlan& a, long m, long q, int A, int B)
+{
+  long p=ceilquotient(a.L,m);
+  return q*(A+B)*fftInstr(m)+A*(double) m*(2.0*p+(q-1)*6.0*p)+
+    B*(double) a.L*(2.0+(q-1)*6.0);
+}
+
+// The same with the fused rows for one residue of one fold.
 static double rowCost(const AxisPlan& a, long m, long q, int A, int B,
                       int prec)
 {
@@ -670,10 +677,26 @@ static double rowCost(const AxisPlan& a, long m, long q, int A, int B,
   // The fused rows run an instruction's worth in 0.55 (FP32) to 0.9 of the
   // time (4096 rows of 1024: FP32 175 -> 83 us, FP64 1728 -> 1425).
   const double slower=prec == PREC_F32 ? 1.8 : 1.1;
-  long p=ceilquotient(a.L,m);
-  return slower*(q*(A+B)*(fftInstr(m)+2.0*m)+
-                 A*(double) m*(2.0*p+(q-1)*6.0*p)+
-                 B*(double) a.L*(2.0+(q-1)*6.0));
+  return slower*(stagedRowCost(a,m,q,A,B)+2.0*(A+B)*(double) (q*m));
+}
+
+// Whether the results along an axis are the same for every padded length
+// N >= M.  The built-in products are bilinear: with indices in [-c, L-1-c]
+// (c = 0, floor(L/2) or, Hermitian, H-1 of 2H-1), a sum or difference of two
+// of them returns into that range modulo N only if N < L+max(c, L-1-c).
+// Below that length which outputs alias depends on N.  It always does for a
+// caller's functor, which sees the grid, and for a multiplier of the other
+// kind of data, which acts on real and imaginary parts, or on neighbouring
+// grid points, in its own way.
+bool anyLength(int kind, long L, long M, int mult)
+{
+  const bool real=mult == MULT_REALBINARY || mult == MULT_REALJACOBIAN ||
+    mult == MULT_REALJACADJ || mult == MULT_REALDOT;
+  if(mult == MULT_USER) return false;
+  if(kind == KIND_HERMITIAN)
+    return (real || mult == MULT_NONE) &&
+      M >= 3*(long) ceilquotient(L,2)-2;
+  return !real && M >= (kind == KIND_CENTERED ? L+L/2 : 2*L-1);
 }
 
 // The same for an outer axis: residue r > 0 folds p terms with a complex
@@ -688,8 +711,9 @@ static double outerCost(const AxisPlan& a, long m, long q, int A, int B)
 }
 
 // Inner (row) axis, complex data: residue block m and residue count q.
-// longer: whether other lengths than the least may be taken (a caller's
-// functor sees the padded length, so its plans keep the least).
+// longer: whether another padded length than the staged rows' cheapest may be
+// taken (anyLength); otherwise that length stays, whatever the fused rows
+// make cheaper, because the results depend on it.
 static bool planRowComplex(AxisPlan& a, long mForce, int A, int B, int prec,
                            bool longer)
 {
@@ -700,17 +724,28 @@ static bool planRowComplex(AxisPlan& a, long mForce, int A, int B, int prec,
     if(!smooth(mForce)) return false;
     a.m=mForce; a.q=q;
   } else {
-    double best=1e300;
-    long bm=0, bq=0;
-    auto consider=[&](long m, long q) {
-      if(m*q < a.M || rowNeed(prec,a.L,m,A,B) > SMEM_MAX) return;
-      double cost=rowCost(a,m,q,A,B,prec);
-      if(cost < best) {best=cost; bm=m; bq=q;}
+    const double never=1e300;
+    double best=never;
+    long bm=0, bq=0, N=0;
+    auto consider=[&](long m, long q, auto cost) {
+      if(m*q < a.M || (N && m*q != N) ||
+         rowNeed(prec,a.L,m,A,B) > SMEM_MAX) return;
+      const double c=cost(m,q);
+      if(c < best) {best=c; bm=m; bq=q;}
     };
-    for(long q=1; q <= 64; ++q) consider(nextfftsize(ceilquotient(a.M,q)),q);
+    auto staged=[&](long m, long q) {return stagedRowCost(a,m,q,A,B);};
+    auto all=[&](long m, long q) {return rowCost(a,m,q,A,B,prec);};
+    if(!longer) {
+      for(long q=1; q <= 64; ++q)
+        consider(nextfftsize(ceilquotient(a.M,q)),q,staged);
+      N=bm*bq;
+      best=never;
+    }
+    for(long q=1; q <= 64; ++q)
+      consider(nextfftsize(ceilquotient(a.M,q)),q,all);
     if(!bm) return false;
     if(longer)
-      for(long m : paddedLengths(a.M)) consider(m,1);
+      for(long m : paddedLengths(a.M)) consider(m,1,all);
     a.m=bm; a.q=bq;
   }
   a.N=a.m*a.q;
@@ -751,6 +786,40 @@ static bool planRowHermitian(AxisPlan& a, long mForce, int A, int B, int prec,
   a.m=a.N; a.q=1; a.p=1;
   a.cshift=0;
   return hermNeed(prec,a.N/2,A) <= SMEM_MAX;
+}
+
+// The innermost axis where one CTA (or cluster) holds a row; false: too long.
+static bool planRow(AxisPlan& a, long mForce, int A, int B, int mult, int prec)
+{
+  const bool longer=anyLength(a.kind,a.L,a.M,mult);
+  return a.kind == KIND_HERMITIAN ?
+    planRowHermitian(a,mForce,A,B,prec,longer) :
+    planRowComplex(a,mForce,A,B,prec,longer);
+}
+
+static AxisPlan newAxis(int kind, long L, long M)
+{
+  AxisPlan a;
+  a.kind=kind;
+  a.L=L;
+  a.M=M;
+  a.stored=kind == KIND_HERMITIAN ? (long) ceilquotient(L,2) : L;
+  a.m=a.p=a.q=a.N=0;
+  a.cshift=0;
+  a.tile=a.tileB=1;
+  a.rpc=1;
+  a.thr=a.thrB=256;
+  a.rows=0;
+  return a;
+}
+
+bool planRowLength(int kind, long L, long M, long mForce, int A, int B,
+                   int mult, int prec, long *m, long *q, long *N)
+{
+  AxisPlan a=newAxis(kind,L,M);
+  if(!planRow(a,mForce,A,B,mult,prec)) return false;
+  *m=a.m; *q=a.q; *N=a.N;
+  return true;
 }
 
 // Estimated FP64/FP32 arithmetic instructions of one length-n transform in
@@ -894,9 +963,7 @@ Conv::Conv(int dim, const int *kinds, const long *L, const long *M,
   I.longRow=false; I.rowM=I.rowQ=0;
   for(int d=0; d < dim; ++d) {
     AxisPlan& a=I.axis[d];
-    a.kind=kinds[d];
-    a.L=L[d];
-    a.M=M[d];
+    a=newAxis(kinds[d],L[d],M[d]);
     if(a.kind < 0 || a.kind > 3) throw std::runtime_error("unknown axis kind");
     if(a.L < 1) throw std::runtime_error("L must be positive");
     if(a.L > a.M)
@@ -906,11 +973,6 @@ Conv::Conv(int dim, const int *kinds, const long *L, const long *M,
       throw std::runtime_error("a Hermitian axis must be the innermost");
     if(a.kind == KIND_REAL && d != 0)
       throw std::runtime_error("a real axis must be the outermost");
-    a.stored=a.kind == KIND_HERMITIAN ? (long) ceilquotient(a.L,2) : a.L;
-    a.tile=a.tileB=1;
-    a.rpc=1;
-    a.thr=a.thrB=256;
-    a.rows=0;
   }
   if(dim > 1 && batch != 1)
     throw std::runtime_error("batched problems are one-dimensional");
@@ -922,11 +984,7 @@ Conv::Conv(int dim, const int *kinds, const long *L, const long *M,
     planOuter(I.axis[d],mForce ? mForce[d] : 0,prec,C,nb,A,B);
   }
   AxisPlan& in=I.axis[dim-1];
-  long mf=mForce ? mForce[dim-1] : 0;
-  bool ok;
-  const bool longer=mult != MULT_USER;
-  if(in.kind == KIND_HERMITIAN) ok=planRowHermitian(in,mf,A,B,prec,longer);
-  else ok=planRowComplex(in,mf,A,B,prec,longer);
+  const bool ok=planRow(in,mForce ? mForce[dim-1] : 0,A,B,mult,prec);
   if(in.kind == KIND_REAL && dim == 1) in.rows=0;
   if(!ok) {
     // Long rows (beyond one CTA's shared memory), any kind: the row is a
@@ -990,8 +1048,9 @@ void Conv::setResidueSearch(bool on) {residueSearch=on;}
 
 // Candidate residue block lengths of a complex axis for the timed search:
 // at most three, cheapest estimate first, each within 1.5x of the cheapest.
+// longer: as planRowComplex.
 static std::vector<long> residueCandidates(const AxisPlan& a, bool outer,
-                                           int prec, int A, int B)
+                                           int prec, int A, int B, bool longer)
 {
   std::vector<std::pair<double,long>> c;
   if(outer) {
@@ -1001,7 +1060,8 @@ static std::vector<long> residueCandidates(const AxisPlan& a, bool outer,
         c.push_back({outerCost(a,m,N/m,A,B),m});
   } else {
     auto add=[&](long m, long q) {
-      if(m*q < a.M || rowNeed(prec,a.L,m,A,B) > SMEM_MAX) return;
+      if(m*q < a.M || (!longer && m*q != a.N) ||
+         rowNeed(prec,a.L,m,A,B) > SMEM_MAX) return;
       for(const auto& x : c)
         if(x.second == m) return;
       c.push_back({rowCost(a,m,q,A,B,prec),m});
@@ -1179,7 +1239,14 @@ Conv *Conv::create(int dim, const int *kinds, const long *L, const long *M,
       try {
         std::unique_ptr<Conv> c(new Conv(dim,kinds,L,M,mw,A,B,mult,prec,batch,
                                          false));
-        if(c->applySchedule(rest)) return c.release();
+        // A record may hold another padded length than this plan's, but not
+        // where the results depend on it.
+        const AxisPlan& a=c->info().axis[dim-1];
+        long m0=0, q0=0, N0=0;
+        const bool length=anyLength(a.kind,a.L,a.M,mult) ||
+          (planRowLength(a.kind,a.L,a.M,mForce ? mForce[dim-1] : 0,A,B,mult,
+                         prec,&m0,&q0,&N0) ? a.N == N0 : c->info().longRow);
+        if(length && c->applySchedule(rest)) return c.release();
       } catch(std::exception& x) {
         // A record that no longer plans: plan afresh.  Failures of the
         // device (allocations) are the caller's to see.
@@ -1217,7 +1284,8 @@ Conv *Conv::createSearched(int dim, const int *kinds, const long *L,
     const AxisPlan& a=I0.axis[d];
     if(I0.longRow || mf[d] > 0 ||
        (a.kind != KIND_PAD && a.kind != KIND_CENTERED)) continue;
-    cands[d]=residueCandidates(a,d < dim-1,prec,A,B);
+    cands[d]=residueCandidates(a,d < dim-1,prec,A,B,
+                               anyLength(a.kind,a.L,a.M,mult));
     any=any || cands[d].size() > 1;
   }
   if(!any) {
@@ -1264,6 +1332,9 @@ Conv *Conv::createSearched(int dim, const int *kinds, const long *L,
       trial[d]=m;
       try {
         Conv c(dim,kinds,L,M,trial,A,B,mult,prec,batch,false);
+        // The residues that go with m may make another length of it.
+        const AxisPlan& a=c.info().axis[d];
+        if(a.N != I0.axis[d].N && !anyLength(a.kind,a.L,a.M,mult)) continue;
         double t=timeOf(c);
         if(t < 0.97*bestT) {bestT=t; mf[d]=m;}
       } catch(std::exception&) {}     // a candidate that does not plan

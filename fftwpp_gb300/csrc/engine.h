@@ -47,6 +47,14 @@ int fusedRadices(long n, int prec, int A, bool herm, bool half, int maxR,
 int fusedPadding(const int *radix, int nst, int level);
 int rowTeams(int rpc, int threads);
 
+// Whether a convolution's results are the same for every padded length
+// N >= M of an axis (engine.cu).
+bool anyLength(int kind, long L, long M, int mult);
+// The innermost axis' residue block m, residue count q and padded length N of
+// a plan (mForce: a forced m or 0); false for the long path.
+bool planRowLength(int kind, long L, long M, long mForce, int A, int B,
+                   int mult, int prec, long *m, long *q, long *N);
+
 struct AxisPlan {
   int kind;
   long L, M;          // data length, minimum padded length

@@ -344,6 +344,16 @@ int fgb_batch_task_order(int nlong, const size_t *staging,
 int fgb_fft_radices(size_t n, int precision, int inplace, int wide,
                     int *radix, int max);
 
+/* The plan of a convolution's innermost axis before any timing (host
+ * arithmetic, no GPU): info[0] residue block m, [1] residue count, [2] padded
+ * length, [3] whether the results are the same for every padded length >= M
+ * (M at least the dealiasing length, a built-in multiplier for this kind of
+ * data); where they are not, the plan keeps the length that the staged rows'
+ * estimate picks, and neither timing nor wisdom changes it.  Returns 1, 0 for
+ * a row too long for one CTA (info[0..2] unset), -1 for bad arguments. */
+int fgb_row_length(int kind, size_t L, size_t M, size_t m, int A, int B,
+                   int mult, int precision, long *info);
+
 /* Radices, stage by stage, of the fused transforms of length n (host
  * arithmetic, no GPU): `inputs` columns share the registers of the middle
  * stage, hermitian != 0 for the rows of Hermitian data, half != 0 for data
