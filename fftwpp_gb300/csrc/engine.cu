@@ -138,30 +138,51 @@ static void unitRoots(long n, std::vector<double>& c, std::vector<double>& s)
   }
 }
 
+// A new device table of host values, whole when this returns: a copy from
+// pageable memory may still be under way when cudaMemcpy does, and the
+// kernels' streams need not follow the default one.
+static void *upload(const void *h, size_t bytes)
+{
+  void *d=NULL;
+  cudaError_t e=devAlloc(&d,bytes);
+  if(e == cudaSuccess) {
+    e=cudaMemcpy(d,h,bytes,cudaMemcpyHostToDevice);
+    if(e == cudaSuccess) e=cudaStreamSynchronize(cudaStreamLegacy);
+    if(e != cudaSuccess) cudaFree(d);
+  }
+  if(e != cudaSuccess) {
+    cudaGetLastError();
+    throw std::runtime_error("twiddle table allocation failed: "+
+                             std::string(cudaGetErrorString(e)));
+  }
+  return d;
+}
+
+template<class V>
+static void *upload(const std::vector<V>& h)
+{
+  return upload(h.data(),h.size()*sizeof(V));
+}
+
 // A device table of the roots c[e[k]] + i s[e[k]] in the form of prec
-// (double2, or float4 split into hi and lo), NULL if the allocation fails.
+// (double2, or float4 split into hi and lo).
 static void *rootTable(const std::vector<double>& c,
                        const std::vector<double>& s,
                        const std::vector<long>& e, int prec)
 {
-  void *d=NULL;
   const size_t n=e.size();
   if(prec == PREC_F64) {
     std::vector<double2> h(n);
     for(size_t k=0; k < n; ++k) h[k]=make_double2(c[e[k]],s[e[k]]);
-    if(devAlloc((void **) &d,n*sizeof(double2)) != cudaSuccess) return NULL;
-    cudaMemcpy(d,h.data(),n*sizeof(double2),cudaMemcpyHostToDevice);
-  } else {
-    std::vector<float4> h(n);
-    for(size_t k=0; k < n; ++k) {
-      const double x=c[e[k]], y=s[e[k]];
-      float hx=(float) x, hy=(float) y;
-      h[k]=make_float4(hx,hy,(float) (x-(double) hx),(float) (y-(double) hy));
-    }
-    if(devAlloc((void **) &d,n*sizeof(float4)) != cudaSuccess) return NULL;
-    cudaMemcpy(d,h.data(),n*sizeof(float4),cudaMemcpyHostToDevice);
+    return upload(h);
   }
-  return d;
+  std::vector<float4> h(n);
+  for(size_t k=0; k < n; ++k) {
+    const double x=c[e[k]], y=s[e[k]];
+    float hx=(float) x, hy=(float) y;
+    h[k]=make_float4(hx,hy,(float) (x-(double) hx),(float) (y-(double) hy));
+  }
+  return upload(h);
 }
 
 const void *twiddles(long n, int prec, long step)
@@ -180,7 +201,7 @@ const void *twiddles(long n, int prec, long step)
   std::vector<long> e;
   for(long t=0; t < n; t += step) e.push_back(t);
   void *d=rootTable(c,s,e,prec);
-  if(d) cache[key]=d;
+  cache[key]=d;
   return d;
 }
 
@@ -249,7 +270,6 @@ static FFTPlanDev fftPlan(long n, int prec, bool oddFirst=false,
     throw std::runtime_error("too many FFT stages");
   }
   p.tw=twiddles(n,prec);
-  if(!p.tw) throw std::runtime_error("twiddle table allocation failed");
   return p;
 }
 
@@ -424,23 +444,19 @@ static void fusedTables(FusedFFT& p, int prec)
     }
     if(eb.empty()) eb.push_back(0);
     if(ej.empty()) ej.push_back(0);
-    Tables t;
-    t.twb=rootTable(c,s,eb,prec);
-    t.twj=rootTable(c,s,ej,prec);
-    t.pairs=t.pos=t.rev=NULL;
     std::vector<int> pos(n);
     for(long b=0; b < n; ++b) pos[rev[b]]=(int) b;
-    const size_t pb=pairs.size()*sizeof(int4), nb=n*sizeof(int);
-    const size_t rb=blocks.size()*sizeof(int);
-    if(!t.twb || !t.twj || devAlloc(&t.pairs,pb) != cudaSuccess ||
-       devAlloc(&t.pos,nb) != cudaSuccess ||
-       devAlloc(&t.rev,rb) != cudaSuccess) {
+    Tables t={};
+    try {
+      t.twb=rootTable(c,s,eb,prec);
+      t.twj=rootTable(c,s,ej,prec);
+      t.pairs=upload(pairs);
+      t.pos=upload(pos);
+      t.rev=upload(blocks);
+    } catch(...) {
       for(void *q : {t.twb,t.twj,t.pairs,t.pos,t.rev}) if(q) cudaFree(q);
-      throw std::runtime_error("twiddle table allocation failed");
+      throw;
     }
-    cudaMemcpy(t.pairs,pairs.data(),pb,cudaMemcpyHostToDevice);
-    cudaMemcpy(t.pos,pos.data(),nb,cudaMemcpyHostToDevice);
-    cudaMemcpy(t.rev,blocks.data(),rb,cudaMemcpyHostToDevice);
     it=cache.emplace(key,t).first;
   }
   p.twb=it->second.twb;
@@ -2101,33 +2117,40 @@ cudaError_t Conv::run(const void *const *in, void *const *out, cudaStream_t s)
     });
 }
 
-// The tables of the fused transforms, made with the plan: its first run may
-// be under stream capture, where nothing can be allocated.
+// The tables of every launch, made with the plan: its first run may be under
+// stream capture, where nothing can be allocated, and a table that cannot be
+// made is an error of the plan's creation.
 void Conv::makeTables()
 {
-  auto make=[&](FusedFFT p) {fusedTables(p,I.prec);};
+  const int prec=I.prec, A=I.A;
+  auto make=[&](FusedFFT p) {fusedTables(p,prec);};
   for(int d=0; d < I.dim-1; ++d) {
     const AxisPlan& a=I.axis[d];
-    if(outerFused(a)) make(outerFFT(a,I.prec,1));
-    else if(a.kind == KIND_REAL) make(realFFT(a.N,a.L,I.prec,1));
+    if(outerFused(a)) make(outerFFT(a,prec,1));
+    else if(a.kind == KIND_REAL) make(realFFT(a.N,a.L,prec,1));
+    else fftPlan(a.m,prec);
+    twiddles(a.N,prec);
   }
   const AxisPlan& a=I.axis[I.dim-1];
-  long nrows=batch;
-  for(int d=0; d < I.dim-1; ++d) nrows *= I.axis[d].rows;
-  const int A=I.A;
+  twiddles(I.longRow ? I.rowM : a.N,prec);
   if(I.longRow) {
-    make(fusedRowPlan(I.rowM,I.prec,A,false,false,1,widest(I.prec)));
+    make(fusedRowPlan(I.rowM,prec,A,false,false,1,widest(prec)));
+    fftPlan(I.rowQ,prec);
+    twiddles(a.N,prec);
+    twiddles(a.N,prec,256);
     return;
   }
   if(a.kind == KIND_HERMITIAN) {
-    make(fusedRowPlan(a.N/2,I.prec,A,true,false,1,widest(I.prec,a.N/2)));
+    make(fusedRowPlan(a.N/2,prec,A,true,false,1,widest(prec,a.N/2)));
     return;
   }
-  const int split=I.mult != MULT_USER ? rowSplit(a.N,nrows,I.prec) : 1;
-  if(split > 1) make(fusedRowPlan(a.N/split,I.prec,A,false,false,1,8));
+  long nrows=batch;
+  for(int d=0; d < I.dim-1; ++d) nrows *= I.axis[d].rows;
+  const int split=I.mult != MULT_USER ? rowSplit(a.N,nrows,prec) : 1;
+  if(split > 1) make(fusedRowPlan(a.N/split,prec,A,false,false,1,8));
   if(rowDirect(a))
-    make(fusedRowPlan(a.m,I.prec,A,false,halfEmpty(a),1,
-                      widest(I.prec,a.m)));
+    make(fusedRowPlan(a.m,prec,A,false,halfEmpty(a),1,widest(prec,a.m)));
+  else fftPlan(a.m,prec);
 }
 
 bool Conv::zeroCopy=true;
@@ -2526,6 +2549,16 @@ cudaError_t Conv::runHost(const void *const *in, void *const *out,
 // ---------------------------------------------------------------------------
 // Standalone padded transform (engine.h).
 
+// Padded transforms and plain FFTs plan on the host alone; with a device
+// their plans make their tables too, as Conv::makeTables.
+static bool deviceReady()
+{
+  int n=0;
+  const bool ok=cudaGetDeviceCount(&n) == cudaSuccess && n > 0;
+  cudaGetLastError();
+  return ok;
+}
+
 PadTransform::PadTransform(int kind, long L, long M, long C, long mForce,
                            int prec) : C(C), prec(prec)
 {
@@ -2563,9 +2596,13 @@ PadTransform::PadTransform(int kind, long L, long M, long C, long mForce,
                                "memory");
     a.tile=pickTile(wide(prec) ? 8 : 16,C,1,sm,wide(prec) ? 2 : 4);
     a.tileB=a.tile;
-    return;
-  }
-  planOuter(a,mForce,prec,C,1,1,1,true);
+  } else planOuter(a,mForce,prec,C,1,1,1,true);
+  if(!deviceReady()) return;
+  if(kind == KIND_REAL || kind == KIND_HERMITIAN) {
+    FusedFFT f=realFFT(a.N,kind == KIND_REAL ? a.L : a.N,prec,1);
+    fusedTables(f,prec);
+  } else fftPlan(a.m,prec);
+  twiddles(a.N,prec);
 }
 
 size_t PadTransform::inElements() const {return (size_t) a.stored*C;}
@@ -2698,6 +2735,12 @@ PlainFFT::PlainFFT(int kind, long n, int sign, long C, long B, long istride,
     };
     tile1=pickTile(maxTile,sign > 0 ? n2 : n1,B,smw(sign > 0 ? n1 : n2));
     tile2=pickTile(maxTile,sign > 0 ? n1 : n2,B,smw(sign > 0 ? n2 : n1));
+    if(deviceReady()) {
+      fftPlan(n1,prec);
+      fftPlan(n2,prec);
+      twiddles(n,prec);
+      twiddles(n,prec,256);
+    }
     if(devAlloc(&scratch,elem(prec)*(size_t) n*(size_t) B) != cudaSuccess) {
       scratch=NULL;
       throw std::runtime_error("device allocation of the scratch array "
@@ -2706,6 +2749,12 @@ PlainFFT::PlainFFT(int kind, long n, int sign, long C, long B, long istride,
     return;
   }
   tile=C > 1 ? pickTile(maxTile,C,B,sm) : 1;
+  if(!deviceReady()) return;
+  if(kind != FFT_C2C) {
+    FusedFFT f=realFFT(n,n,prec,1);
+    fusedTables(f,prec);
+  } else fftPlan(n,prec);
+  twiddles(n,prec);
 }
 
 PlainFFT::~PlainFFT()

@@ -349,7 +349,8 @@ private:
                                               cudaStream_t s);
 };
 
-const void *twiddles(long n, int prec, long step=1);   // every step-th t
+// Every step-th t; throws if the table cannot be made.
+const void *twiddles(long n, int prec, long step=1);
 
 // Every device allocation of the library goes through devAlloc.  Failure
 // injection for tests (host side): failAllocationAfter(n) makes the n-th
