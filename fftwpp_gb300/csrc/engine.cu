@@ -890,6 +890,9 @@ static void planOuter(AxisPlan& a, long mForce, int prec, long C, long nbatch,
     a.N=evenSmooth(mForce > 0 ? std::max(a.M,mForce) : a.M);
     a.m=a.N; a.q=1; a.p=1; a.cshift=0;
     a.rows=a.N/2+1;
+    // The line stays where a two-buffer transform put it.
+    if(FGB_BY_PREC(prec,outerRealSmem,a.L,a.N/2,1) > SMEM_MAX)
+      throw std::runtime_error("outer axis too long for shared memory");
     auto sm=[&](int t) {return realNeed(a,prec,t);};
     a.tile=pickTile(maxTile,C,nbatch*A,sm,minTile);
     a.tileB=pickTile(maxTile,C,nbatch*B,sm,minTile);

@@ -1135,13 +1135,10 @@ cudaError_t launchOuterBwd(const OuterPlan<T>& P, int threads, cudaStream_t s)
   return go(outerBwdKernel<T>);
 }
 
-// The real kernels take what two buffers of one element more per column
-// would hold, as planned.
 template<typename T>
 static cudaError_t launchOuterReal(const OuterPlan<T>& P, bool fwd,
                                    int threads, cudaStream_t s)
 {
-  if(outerRealSmem<T>(P.L,P.N/2,1) > 227*1024) return cudaErrorInvalidValue;
   const size_t sm=fusedOuterSmem<T>(P.L,P.fz.n,P.fz.lg,P.tile,1);
   dim3 grid((P.C+P.tile-1)/P.tile,1,P.nbatch*P.count);
   auto go=[&](auto kernel) {

@@ -51,3 +51,27 @@ def test_padded_tiles_fit(native_lib, kind, C, prec):
             assert max(_needs(v, prec)) <= SMEM_MAX, (L, m, v)
             planned += 1
     assert planned >= 90
+
+
+@pytest.mark.parametrize("prec", [F64, F32])
+def test_real_axis_too_long_is_refused_at_creation(native_lib, prec):
+    """The longest real axis is where two padded buffers of one column fill
+    shared memory; the next length is no plan, rather than one that fails
+    every run."""
+    from fftwpp_gb300 import _native
+    e = 16 if prec == F64 else 8
+    REAL = 3
+    took = refused = 0
+    for L in range(5000, 20000, 250):
+        M = 2 * L - 1
+        N = M + 1
+        while native_lib.fgb_nextfftsize(N // 2) != N // 2:
+            N += 2
+        v = _tiles(native_lib, REAL, L, M, 1, 0, prec)
+        if 2 * e * _padded(N // 2 + 1) <= SMEM_MAX:
+            assert v and v[3] == N, L
+            took += 1
+        else:
+            assert v is None and "too long" in _native.last_error()
+            refused += 1
+    assert took >= 8 and refused >= 8
