@@ -589,6 +589,18 @@ static size_t outerBwdNeed(const AxisPlan& a, int prec, int tile)
   return FGB_BY_PREC(prec,outerBwdSmem,a.L,a.m,tile,(int) a.q);
 }
 
+// Whether the fused outer kernels of an axis take the staged form: float-float
+// with few columns, where fetching the code dominates (39 x 93 convolution 43
+// us fused, 34 staged), not from 1024 on, where the pruned halves count (3D
+// real 256^3, y transforms of 131 584 columns back 558 us staged, 416 before).
+// columns: of all the launch's inputs or outputs and batches, also where a
+// host call makes the launch in column ranges, so that every way gives the
+// same bits.
+static bool stagedColumns(int prec, long long columns)
+{
+  return prec == PREC_FF && columns < 1024;
+}
+
 // CTAs per complex row of padded length n (RowPlan::split): as many of 8, 4
 // or 2 as leave every row its own SMs and every CTA at least 64 points of a
 // length they divide; 1 otherwise.  Measured against one CTA per row (kernel
@@ -1857,6 +1869,7 @@ cudaError_t Conv::runT(const void *const *in, void *const *out, cudaStream_t s)
       O.inRow=strideS[0];
       O.Ltot=LLONG_MAX;
     }
+    O.staged=stagedColumns(I.prec,C*A);
     O.scale=(T) 1;
     O.io64=IN64;
     for(int i=0; i < A; ++i) {O.in[i]=(const Cx *) in[i]; O.out[i]=(Cx *) bufs[i];}
@@ -1886,6 +1899,7 @@ cudaError_t Conv::runT(const void *const *in, void *const *out, cudaStream_t s)
     if(e != cudaSuccess) return e;
     O.count=B;
     retile(O,ax);
+    O.staged=stagedColumns(I.prec,C*B);
     O.scale=(T) scale;
     O.io64=OUT64;
     O.inRow=C;                                  // staging side
@@ -1909,6 +1923,7 @@ cudaError_t Conv::runT(const void *const *in, void *const *out, cudaStream_t s)
   outerPlan(X,ax);
   X.count=A; X.nbatch=1; X.inBatch=X.outBatch=0;
   X.inRow=Cx_; X.outRow=Cx_; X.C=(int) Cx_; X.Ltot=(long long) ax.L*Cx_;
+  X.staged=stagedColumns(I.prec,(long long) Cx_*A);
   X.scale=(T) 1;
   X.io64=IN64;
   if(isStrided) {                   // data side (the caller's arrays)
@@ -1926,6 +1941,7 @@ cudaError_t Conv::runT(const void *const *in, void *const *out, cudaStream_t s)
   Y.count=A; Y.nbatch=(int) ax.rows;
   Y.inBatch=ay.L*nz; Y.outBatch=ay.rows*nz;
   Y.inRow=nz; Y.outRow=nz; Y.C=(int) nz; Y.Ltot=(long long) ay.L*nz;
+  Y.staged=stagedColumns(I.prec,(long long) nz*ax.rows*A);
   Y.scale=(T) 1;
   for(int i=0; i < A; ++i) {Y.in[i]=(const Cx *) bx[i]; Y.out[i]=(Cx *) by[i];}
   e=launchOuterFwd<T>(Y,ay.thr,s);
@@ -1956,6 +1972,7 @@ cudaError_t Conv::runT(const void *const *in, void *const *out, cudaStream_t s)
 
   Y.count=B;
   retile(Y,ay);
+  Y.staged=stagedColumns(I.prec,(long long) nz*ax.rows*B);
   for(int i=0; i < B; ++i) {Y.in[i]=(const Cx *) by[i]; Y.out[i]=(Cx *) bx[i];}
   std::swap(Y.inBatch,Y.outBatch);
   e=launchOuterBwd<T>(Y,ay.thrB,s);
@@ -1964,6 +1981,7 @@ cudaError_t Conv::runT(const void *const *in, void *const *out, cudaStream_t s)
 
   X.count=B;
   retile(X,ax);
+  X.staged=stagedColumns(I.prec,(long long) Cx_*B);
   X.scale=(T) scale;
   X.io64=OUT64;
   X.inRow=Cx_;                                  // staging side

@@ -378,17 +378,6 @@ __device__ __forceinline__ int columnTop(const OuterPlan<T>& P, int col,
   return ((int) P.Ltot-col+(int) row-1)/(int) row;
 }
 
-// Whether a fused outer launch takes the staged form: float-float with few
-// columns, where fetching the code dominates (39 x 93 convolution 43 us fused,
-// 34 staged), not from 1024 on, where the pruned halves count (3D real 256^3,
-// y transforms of 131 584 columns back 558 us staged, 416 before).
-template<typename T>
-__device__ __forceinline__ bool stagedColumns(const OuterPlan<T>& P)
-{
-  return std::is_same<T,ff>::value &&
-    (long long) P.C*P.nbatch*P.count < 1024;
-}
-
 template<typename T, bool WIDE>
 __device__ __forceinline__ void outerFwdFused(const OuterPlan<T>& P, int ctile,
                                               int r, int z,
@@ -418,7 +407,7 @@ __device__ __forceinline__ void outerFwdFused(const OuterPlan<T>& P, int ctile,
       return v;
     };
   };
-  if(stagedColumns(P)) {
+  if(std::is_same<T,ff>::value && P.staged) {
     loadTileFF(x,P.fz,lt,tid,nthr,[&](int cc, int j) {
         int s=j+c;
         if(s >= m) s -= m;
@@ -522,7 +511,7 @@ __device__ __forceinline__ void outerBwdFused(const OuterPlan<T>& P, int ctile,
         storeIO(f+s*P.outRow,v*P.scale,P.io64 & 2,sh);
       };
     };
-    if(stagedColumns(P)) {
+    if(std::is_same<T,ff>::value && P.staged) {
       loadTileFF(x,P.fz,lt,tid,nthr,[&](int cc, int j) {
           return col0+cc < P.C ? swapXY(sr[j*P.inRow+col0+cc]) :
             mk((T) 0,(T) 0);

@@ -140,6 +140,7 @@ struct OuterPlan {
   int fused;               // L <= m and no twX: the fused kernels, with the
                            // rows of a residue block in fz's digit-reversed
                            // order
+  int staged;              // fused, float-float: the staged form (runStages)
   int conj;                // real kernels: conjugate the complex side
                            // (the sign -1 r2c / sign +1 c2r of plain FFTs)
   int cz;                  // data side with strides: column c lies at
