@@ -151,6 +151,8 @@ def load():
     lib.fgb_fft_radices.argtypes = [sz, ctypes.c_int, ctypes.c_int,
                                     ctypes.c_int, P(ctypes.c_int),
                                     ctypes.c_int]
+    lib.fgb_row_split.restype = ctypes.c_int
+    lib.fgb_row_split.argtypes = [ctypes.c_void_p]
     lib.fgb_row_length.restype = ctypes.c_int
     lib.fgb_row_length.argtypes = [ctypes.c_int, sz, sz, sz, ctypes.c_int,
                                    ctypes.c_int, ctypes.c_int, ctypes.c_int,

@@ -748,6 +748,11 @@ int fgb_info(const fgb_conv *c, long *info)
   return 0;
 }
 
+int fgb_row_split(const fgb_conv *c)
+{
+  return c ? c->conv->info().split : -1;
+}
+
 void fgb_set_autotune(int on) {Conv::setAutotune(on != 0);}
 
 size_t fgb_wisdom_export(char *buf, size_t size)

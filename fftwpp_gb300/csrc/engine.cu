@@ -601,6 +601,12 @@ static bool stagedColumns(int prec, long long columns)
   return prec == PREC_FF && columns < 1024;
 }
 
+// The transform of a split row's CTAs.
+static FusedFFT splitPlan(long n, int split, int A, int prec)
+{
+  return fusedRowPlan(n/split,prec,A,false,false,1,8);
+}
+
 // CTAs per complex row of padded length n (RowPlan::split): as many of 8, 4
 // or 2 as leave every row its own SMs and every CTA at least 64 points of a
 // length they divide; 1 otherwise.  Measured against one CTA per row (kernel
@@ -608,12 +614,15 @@ static bool stagedColumns(int prec, long long columns)
 // 27 -> 22 to 25, float-float 43 -> 26 / 30 / 34; from n = 128 down no
 // faster, and FP32, whose rows are bound by latency alone, slower (n = 2048,
 // 76 rows 16 -> 21).
-static int rowSplit(long n, long nrows, int prec)
+static int rowSplit(long n, long nrows, int A, int prec)
 {
   static const int sms=152;
   if(prec == PREC_F32 || n < 512) return 1;
   for(int q : {8,4,2})
-    if(n % q == 0 && n/q >= 64 && smooth(n/q) && nrows*q <= sms) return q;
+    if(n % q == 0 && n/q >= 64 && smooth(n/q) && nrows*q <= sms) {
+      const FusedFFT f=splitPlan(n,q,A,prec);
+      return FGB_BY_PREC(prec,fusedRowSmem,f.n,f.lg,A,1) <= SMEM_MAX ? q : 1;
+    }
   return 1;
 }
 
@@ -950,7 +959,7 @@ static void planOuter(AxisPlan& a, long mForce, int prec, long C, long nbatch,
 
 Conv::Conv(int dim, const int *kinds, const long *L, const long *M,
            const long *mForce, int A, int B, int mult, int prec, long batch,
-           bool tuneSchedule)
+           bool rowForced, bool tuneSchedule)
   : batch(batch), user(NULL), isStrided(false), ffState(NULL), longBuf(0),
     tuning(false), staging(0), hostIn(NULL),
     hostOut(NULL), nlaunch(0),
@@ -1052,6 +1061,9 @@ Conv::Conv(int dim, const int *kinds, const long *L, const long *M,
   // Rows per CTA of the row kernel.
   long nrows=batch;
   for(int d=0; d < dim-1; ++d) nrows *= I.axis[d].rows;
+  I.split=1;
+  if(!I.longRow && in.kind != KIND_HERMITIAN && mult != MULT_USER &&
+     !rowForced) I.split=rowSplit(in.N,nrows,A,prec);
   in.rpc=pickRpc(I.longRow ? I.rowM : in.kind == KIND_HERMITIAN ? in.N/2 :
                  in.m,A,I.longRow ? I.rowQ*nrows : nrows,[&](int r) {
                    return innerNeed(I,in,r,256);});
@@ -1249,8 +1261,10 @@ Conv *Conv::create(int dim, const int *kinds, const long *L, const long *M,
                    const long *mForce, int A, int B, int mult, int prec,
                    long batch)
 {
+  // Whether the caller, not the search or a record, chose the rows' m.
+  const bool rowForced=mForce && dim >= 1 && dim <= 3 && mForce[dim-1] > 0;
   if(!autotune)
-    return new Conv(dim,kinds,L,M,mForce,A,B,mult,prec,batch);
+    return new Conv(dim,kinds,L,M,mForce,A,B,mult,prec,batch,rowForced);
   const std::string key=wisdomKey(dim,kinds,L,M,mForce,A,B,mult,prec,batch,
                                   residueSearch);
   std::string value;
@@ -1269,7 +1283,7 @@ Conv *Conv::create(int dim, const int *kinds, const long *L, const long *M,
     if(ok) {
       try {
         std::unique_ptr<Conv> c(new Conv(dim,kinds,L,M,mw,A,B,mult,prec,batch,
-                                         false));
+                                         rowForced,false));
         // A record may hold another padded length than this plan's, but not
         // where the results depend on it.
         const AxisPlan& a=c->info().axis[dim-1];
@@ -1300,14 +1314,15 @@ Conv *Conv::createSearched(int dim, const int *kinds, const long *L,
                            int mult, int prec, long batch, long *mUsed)
 {
   for(int d=0; d < dim && d < 3; ++d) mUsed[d]=mForce ? mForce[d] : 0;
+  const bool rowForced=dim >= 1 && dim <= 3 && mUsed[dim-1] > 0;
   // A caller's functor is not available at plan time: its plans keep the
   // cost model's residue blocks (the tiles are still timed).
   if(!residueSearch || mult == MULT_USER)
-    return new Conv(dim,kinds,L,M,mForce,A,B,mult,prec,batch);
+    return new Conv(dim,kinds,L,M,mForce,A,B,mult,prec,batch,rowForced);
   long mf[3]={0,0,0};
   for(int d=0; d < dim && d < 3; ++d) mf[d]=mForce ? mForce[d] : 0;
   std::unique_ptr<Conv> base(new Conv(dim,kinds,L,M,mf,A,B,mult,prec,batch,
-                                      false));
+                                      rowForced,false));
   const ConvInfo I0=base->info();
   std::vector<std::vector<long>> cands(dim);
   bool any=false;
@@ -1322,7 +1337,7 @@ Conv *Conv::createSearched(int dim, const int *kinds, const long *L,
   if(!any) {
     base.reset();
     for(int d=0; d < dim; ++d) mUsed[d]=mf[d];
-    return new Conv(dim,kinds,L,M,mf,A,B,mult,prec,batch);
+    return new Conv(dim,kinds,L,M,mf,A,B,mult,prec,batch,rowForced);
   }
 
   // Zero-filled scratch arrays, shared by every candidate (the stored
@@ -1362,7 +1377,7 @@ Conv *Conv::createSearched(int dim, const int *kinds, const long *L,
       long trial[3]={mf[0],mf[1],mf[2]};
       trial[d]=m;
       try {
-        Conv c(dim,kinds,L,M,trial,A,B,mult,prec,batch,false);
+        Conv c(dim,kinds,L,M,trial,A,B,mult,prec,batch,rowForced,false);
         // The residues that go with m may make another length of it.
         const AxisPlan& a=c.info().axis[d];
         if(a.N != I0.axis[d].N && !anyLength(a.kind,a.L,a.M,mult)) continue;
@@ -1379,7 +1394,7 @@ Conv *Conv::createSearched(int dim, const int *kinds, const long *L,
   if(e1) cudaEventDestroy(e1);
   if(s) cudaStreamDestroy(s);
   for(int d=0; d < dim; ++d) mUsed[d]=mf[d];
-  return new Conv(dim,kinds,L,M,mf,A,B,mult,prec,batch);
+  return new Conv(dim,kinds,L,M,mf,A,B,mult,prec,batch,rowForced);
 }
 
 void Conv::tune()
@@ -1702,7 +1717,7 @@ cudaError_t Conv::runT(const void *const *in, void *const *out, cudaStream_t s)
     }
     if(I.longRow) im.longQ=(int) I.rowQ;    // long rows: k = k1 + q k2
   }
-  auto rowPlan=[&](RowPlan<T>& P, const AxisPlan& a, long nrows) {
+  auto rowPlan=[&](RowPlan<T>& P, const AxisPlan& a) {
     P.im=im;
     P.ioShift=guard;
     P.L=(int) a.stored; P.m=(int) a.m; P.q=(int) a.q; P.N=(int) a.N;
@@ -1712,13 +1727,9 @@ cudaError_t Conv::runT(const void *const *in, void *const *out, cudaStream_t s)
     P.io64=0;
     P.direct=rowDirect(a);
     P.nteam=rowTeams(P.rpc,a.thr);
-    P.split=I.mult != MULT_USER ? rowSplit(a.N,nrows,I.prec) : 1;
+    P.split=I.split;
     if(P.split > 1) {
-      P.fz=fusedRowPlan(a.N/P.split,I.prec,A,false,false,1,8);
-      if(FGB_BY_PREC(I.prec,fusedRowSmem,P.fz.n,P.fz.lg,A,1) > SMEM_MAX)
-        P.split=1;
-    }
-    if(P.split > 1) {
+      P.fz=splitPlan(a.N,P.split,A,I.prec);
       fusedTables(P.fz,I.prec);
     } else if(P.direct) {
       P.fz=fusedRowPlan(a.m,I.prec,A,false,halfEmpty(a),P.nteam,
@@ -1843,7 +1854,7 @@ cudaError_t Conv::runT(const void *const *in, void *const *out, cudaStream_t s)
       return e;
     }
     RowPlan<T> P{};
-    rowPlan(P,a,batch);
+    rowPlan(P,a);
     for(int i=0; i < A; ++i) P.in[i]=(const Cx *) in[i];
     for(int i=0; i < B; ++i) P.out[i]=(Cx *) out[i];
     P.rowStride=a.stored; P.nrows=batch; P.scale=(T) scale;
@@ -1889,7 +1900,7 @@ cudaError_t Conv::runT(const void *const *in, void *const *out, cudaStream_t s)
       tick(s);
     } else {
       RowPlan<T> P{};
-      rowPlan(P,ay,ax.rows);
+      rowPlan(P,ay);
       for(int i=0; i < A; ++i) P.in[i]=(const Cx *) bufs[i];
       for(int i=0; i < B; ++i) P.out[i]=(Cx *) bufs[i];
       P.rowStride=C; P.nrows=ax.rows; P.scale=(T) 1;
@@ -1961,7 +1972,7 @@ cudaError_t Conv::runT(const void *const *in, void *const *out, cudaStream_t s)
     tick(s);
   } else {
     RowPlan<T> P{};
-    rowPlan(P,az,nrows);
+    rowPlan(P,az);
     for(int i=0; i < A; ++i) P.in[i]=(const Cx *) by[i];
     for(int i=0; i < B; ++i) P.out[i]=(Cx *) by[i];
     P.rowStride=nz; P.nrows=nrows; P.scale=(T) 1;
@@ -2165,11 +2176,8 @@ void Conv::makeTables()
     make(fusedRowPlan(a.N/2,prec,A,true,false,1,widest(prec,a.N/2)));
     return;
   }
-  long nrows=batch;
-  for(int d=0; d < I.dim-1; ++d) nrows *= I.axis[d].rows;
-  const int split=I.mult != MULT_USER ? rowSplit(a.N,nrows,prec) : 1;
-  if(split > 1) make(fusedRowPlan(a.N/split,prec,A,false,false,1,8));
-  if(rowDirect(a))
+  if(I.split > 1) make(splitPlan(a.N,I.split,A,prec));
+  else if(rowDirect(a))
     make(fusedRowPlan(a.m,prec,A,false,halfEmpty(a),1,widest(prec,a.m)));
   else fftPlan(a.m,prec);
 }

@@ -74,17 +74,19 @@ struct ConvInfo {
   AxisPlan axis[3];
   bool longRow;       // 1D data too long for one CTA: outer/row/outer path
   long rowM, rowQ;    // long path: row length and column DFT length
+  int split;          // complex rows: CTAs (a cluster) per row, or 1
 };
 
 class Conv {
 public:
   // kinds/L/M/mForce: per dimension, outermost first.  mForce[d] = 0 lets
   // the planner choose.  Throws std::runtime_error on invalid input.
-  // tuneSchedule = false skips the timed tile and thread search (the cost
-  // model's schedule stays).
+  // rowForced: the innermost m is the caller's own, to be run as it is (few
+  // rows are not split over CTAs).  tuneSchedule = false skips the timed tile
+  // and thread search (the cost model's schedule stays).
   Conv(int dim, const int *kinds, const long *L, const long *M,
-       const long *mForce, int A, int B, int mult, int prec, long batch=1,
-       bool tuneSchedule=true);
+       const long *mForce, int A, int B, int mult, int prec, long batch,
+       bool rowForced, bool tuneSchedule=true);
   ~Conv();
 
   // A plan whose residue block lengths are chosen by timing (the GPU

@@ -344,6 +344,11 @@ int fgb_batch_task_order(int nlong, const size_t *staging,
 int fgb_fft_radices(size_t n, int precision, int inplace, int wide,
                     int *radix, int max);
 
+/* CTAs that share each complex innermost row: 1, or a cluster of 2, 4 or 8
+ * where there are too few rows for the SMs; then the row runs as that many
+ * residues whatever m and q the plan reports.  A forced m is never split. */
+int fgb_row_split(const fgb_conv *c);
+
 /* The plan of a convolution's innermost axis before any timing (host
  * arithmetic, no GPU): info[0] residue block m, [1] residue count, [2] padded
  * length, [3] whether the results are the same for every padded length >= M
