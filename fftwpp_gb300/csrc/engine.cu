@@ -476,8 +476,12 @@ int rowTeams(int rpc, int threads)
 }
 
 // The widest radix of a fused transform: 16 in FP32, for rows from 640 points
-// on (shorter ones leave most of a team without a radix-16 butterfly: 441
-// rows of 384 points 15 us with 3 16 8, 13 with 3 4 4 8).
+// on; shorter ones leave most of a team without a radix-16 butterfly.  With
+// radix 16 against 8 at most, us: 441 / 4096 rows of 384 points 13.5 / 24.6
+// against 11.2 / 23.7, 512 11.6 / 26.4 against 11.3 / 25.6, 576 13.5 / 40.6
+// against 14.2 / 40.7, 640 13.7 / 34.2 against 13.9 / 42.8, 768 14.7 / 36.3
+// against 13.8 / 46.5; Hermitian rows alike (4096 of 384 29.7 against 26.1, of
+// 512 32.5 against 33.1, of 640 42.4 against 46.8).
 static int widest(int prec, long rowLength=640)
 {
   return prec == PREC_F32 && rowLength >= 640 ? 16 : 8;
@@ -590,15 +594,18 @@ static size_t outerBwdNeed(const AxisPlan& a, int prec, int tile)
 }
 
 // Whether the fused outer kernels of an axis take the staged form: float-float
-// with few columns, where fetching the code dominates (39 x 93 convolution 43
-// us fused, 34 staged), not from 1024 on, where the pruned halves count (3D
-// real 256^3, y transforms of 131 584 columns back 558 us staged, 416 before).
+// with few columns, where fetching the fused form's code dominates; with many,
+// its fewer passes through shared memory and the halves it leaves out count.
+// Forward kernels of ten axes (60 to 1568 points, centred and half empty),
+// fused over staged time, geometric mean: 512 columns 1.10, 1024 1.05, 1536
+// 1.03, 2048 0.99, 3072 0.99, 6144 0.97 (18 us fused against 16 staged for 80
+// points of 1024 columns, 92 against 104 for 1536 points of 2048).
 // columns: of all the launch's inputs or outputs and batches, also where a
 // host call makes the launch in column ranges, so that every way gives the
 // same bits.
 static bool stagedColumns(int prec, long long columns)
 {
-  return prec == PREC_FF && columns < 1024;
+  return prec == PREC_FF && columns < 2048;
 }
 
 // The transform of a split row's CTAs.
@@ -611,9 +618,11 @@ static FusedFFT splitPlan(long n, int split, int A, int prec)
 // or 2 as leave every row its own SMs and every CTA at least 64 points of a
 // length they divide; 1 otherwise.  Measured against one CTA per row (kernel
 // and event, us): FP64 n = 2048, 1 / 38 / 76 rows 66 -> 29 / 45 / 49, n = 512
-// 27 -> 22 to 25, float-float 43 -> 26 / 30 / 34; from n = 128 down no
-// faster, and FP32, whose rows are bound by latency alone, slower (n = 2048,
-// 76 rows 16 -> 21).
+// 27 -> 22 to 25, float-float 43 -> 26 / 30 / 34.  Below 512: n = 128 18 -> 20
+// in FP64 and 18 both ways in float-float, n = 256 21 -> 20 and 20 -> 19, the
+// launch of the cluster eating most of what its shorter rows save (n = 384
+// would gain in FP64, 34 -> 20, and not in float-float, 21 -> 20).  FP32, whose
+// rows are bound by latency alone, gets slower (n = 2048, 76 rows 16 -> 21).
 static int rowSplit(long n, long nrows, int A, int prec)
 {
   static const int sms=152;
