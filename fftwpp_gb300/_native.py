@@ -162,6 +162,12 @@ def load():
                                       ctypes.c_int, ctypes.c_int,
                                       P(ctypes.c_int), ctypes.c_int,
                                       P(ctypes.c_int)]
+    lib.fgb_fused_tables.restype = ctypes.c_int
+    lib.fgb_fused_tables.argtypes = [sz, ctypes.c_int, ctypes.c_int,
+                                     ctypes.c_int, ctypes.c_int,
+                                     P(ctypes.c_long), P(ctypes.c_long),
+                                     P(ctypes.c_int), P(ctypes.c_int),
+                                     P(ctypes.c_int)]
     lib.fgb_index.restype = sz
     lib.fgb_index.argtypes = [ctypes.c_int, sz, sz, sz, sz, sz, sz, sz]
     lib.fgb_hermitian_symmetrize_x_device.restype = ctypes.c_int

@@ -39,6 +39,7 @@ FFTPlanDev fftPlanPublic(long n, int prec, bool oddFirst);   // engine.cu
 FusedFFT fusedRowPlan(long n, int prec, int A, bool herm, bool half,
                       int nteam, int maxR);
 void fusedRowTables(FusedFFT& p, int prec);
+void fusedColumnTables(FusedFFT& p, int prec);
 
 // Shared memory of nteam fused rows of length m at a time.
 static size_t fusedNeedB(int prec, long m, int A, bool half, int nteam)
@@ -380,10 +381,10 @@ void BatchConv::build()
       F.tile=tile;
       F.fused=1;
       F.fz=fusedColumnPlan(qc,prec,2*pc <= qc,tile);
-      fusedRowTables(F.fz,prec);
+      fusedColumnTables(F.fz,prec);
       F.twN=(const Tw *) twiddles(qc,prec);
       F.twX=(const Tw *) twiddles(N,prec); F.NX=N;
-      F.twC=(const Tw *) twiddles(N,prec,256);
+      F.twC=(const Tw *) coarseRoots(N,prec);
       F.count=A; F.nbatch=1; F.inBatch=F.outBatch=0;
       F.inRow=m; F.outRow=m; F.C=(int) m; F.Ltot=L; F.scale=(T) 1;
       for(int a=0; a < A; ++a) F.in[a]=(const cplx<T> *) (offsets[i]*e);

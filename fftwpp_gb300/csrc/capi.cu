@@ -1143,6 +1143,30 @@ int fgb_fused_radices(size_t n, int precision, int inputs, int hermitian,
   return nst;
 }
 
+int fgb_fused_tables(size_t n, int precision, int inputs, int hermitian,
+                     int half, long *block, long *inverse, int *pairs,
+                     int *pos, int *rev)
+{
+  if(!block || !inverse || !pairs || !pos || !rev) return -1;
+  int r[32];
+  const int nst=fgb_fused_radices(n,precision,inputs,hermitian,half,r,32,NULL);
+  if(nst < 0) return -1;
+  FusedFFT p={};
+  p.n=(int) n;
+  p.nst=nst;
+  for(int s=0; s < nst; ++s) p.radix[s]=(unsigned char) r[s];
+  const FusedHost h=fusedHost(p);
+  std::copy(h.block.begin(),h.block.end(),block);
+  std::copy(h.inverse.begin(),h.inverse.end(),inverse);
+  for(size_t i=0; i < h.pairs.size(); ++i) {
+    const int4 q=h.pairs[i];
+    pairs[3*i]=q.x; pairs[3*i+1]=q.y; pairs[3*i+2]=q.z;
+  }
+  std::copy(h.pos.begin(),h.pos.end(),pos);
+  std::copy(h.rev.begin(),h.rev.end(),rev);
+  return (int) h.rev.size();
+}
+
 // Transformed index (fftBase::index, convolve.h:297-326; fftPadReal::index,
 // convolve.h:956-979).  D0 = n mod D (or D), the remainder block of the
 // residue loop (convolve.cc:701-703); overwrite is not modelled.

@@ -109,14 +109,16 @@ cudaError_t devAlloc(void **p, size_t bytes)
 // ---------------------------------------------------------------------------
 // Twiddle tables.
 
-// exp(2 pi i t/n), t < n, from the exact rational angle t/n, reduced to the
-// first octant so that the long double evaluation stays accurate.
-static void unitRoots(long n, std::vector<double>& c, std::vector<double>& s)
+// exp(2 pi i t/n) for every step-th t < n, from the exact rational angle t/n,
+// reduced to the first octant so that the long double evaluation stays
+// accurate.
+static void unitRoots(long n, long step, std::vector<double>& c,
+                      std::vector<double>& s)
 {
-  c.resize(n);
-  s.resize(n);
+  c.reserve((n+step-1)/step);
+  s.reserve((n+step-1)/step);
   const long double pi=3.141592653589793238462643383279502884L;
-  for(long t=0; t < n; ++t) {
+  for(long t=0; t < n; t += step) {
     // angle = 2 pi t/n; fold by symmetry into [0, pi/4].
     long double sign_c=1, sign_s=1;
     long u=t;
@@ -133,8 +135,8 @@ static void unitRoots(long n, std::vector<double>& c, std::vector<double>& s)
     if(a > pi/4) {a=pi/2-a; swap=true;}
     long double cv=cosl(a), sv=sinl(a);
     if(swap) std::swap(cv,sv);
-    c[t]=(double) (sign_c*cv);
-    s[t]=(double) (sign_s*sv);
+    c.push_back((double) (sign_c*cv));
+    s.push_back((double) (sign_s*sv));
   }
 }
 
@@ -197,12 +199,17 @@ const void *twiddles(long n, int prec, long step)
   auto it=cache.find(key);
   if(it != cache.end()) return it->second;
   std::vector<double> c, s;
-  unitRoots(n,c,s);
-  std::vector<long> e;
-  for(long t=0; t < n; t += step) e.push_back(t);
+  unitRoots(n,step,c,s);
+  std::vector<long> e(c.size());
+  for(size_t k=0; k < e.size(); ++k) e[k]=(long) k;
   void *d=rootTable(c,s,e,prec);
   cache[key]=d;
   return d;
+}
+
+const void *coarseRoots(long n, int prec)
+{
+  return prec == PREC_F32 ? twiddles(n,prec,256) : NULL;
 }
 
 // Radices of an n-point transform into radix[] (at most FGB_MAXSTAGES);
@@ -387,83 +394,92 @@ static FusedFFT fusedPlan(long n, int prec, int A, bool herm, bool half,
   return p;
 }
 
-// Twiddle tables of a fused plan (cached for the process): block twiddles
-// W_{R_0..R_s}^{r rev(b)} of the stages s >= 1, inverse twiddles W_{R m}^{r j}
-// of every stage, and the block pairs of real data.
-static void fusedTables(FusedFFT& p, int prec)
+// The tables of a fused plan, on the host: exponents t of W_n^t of the block
+// twiddles W_{R_0..R_s}^{r rev(b)} of the stages s >= 1 and of the inverse
+// twiddles W_{R m}^{r j} of every stage, then FusedFFT's index tables.
+FusedHost fusedHost(const FusedFFT& p)
+{
+  FusedHost h;
+  const long n=p.n;
+  long nblk=p.radix[0];
+  std::vector<long> rev(nblk);
+  for(long b=0; b < nblk; ++b) rev[b]=b;
+  for(int st=1; st < p.nst; ++st) {
+    const int R=p.radix[st];
+    for(int r=1; r < R; ++r)
+      for(long b=0; b < nblk; ++b)
+        h.block.push_back(r*rev[b]*(n/(nblk*R)) % n);
+    if(st == p.nst-1) {
+      h.rev.assign(rev.begin(),rev.end());
+      // Partner blocks of the last stage: rev(b) and nblk - rev(b).
+      std::vector<int> at(nblk);
+      for(long b=0; b < nblk; ++b) at[rev[b]]=(int) b;
+      h.pairs.push_back(make_int4(0,nblk % 2 ? -1 : at[nblk/2],0,0));
+      for(long b=1; b < nblk; ++b) {
+        const long k=rev[b];
+        if(2*k < nblk)
+          h.pairs.push_back(make_int4((int) b,at[nblk-k],(int) k,0));
+      }
+    }
+    std::vector<long> next(nblk*R);
+    for(long b=0; b < nblk; ++b)
+      for(int r=0; r < R; ++r) next[b*R+r]=rev[b]+nblk*r;
+    rev.swap(next);
+    nblk *= R;
+  }
+  long m=1;
+  for(int st=p.nst-1; st >= 0; --st) {
+    const int R=p.radix[st];
+    for(int r=1; r < R; ++r)
+      for(long j=0; j < m; ++j) h.inverse.push_back(r*j*(n/(R*m)) % n);
+    m *= R;
+  }
+  h.pos.resize(n);
+  for(long b=0; b < n; ++b) h.pos[rev[b]]=(int) b;
+  return h;
+}
+
+// A fused plan's twiddle tables on the device, and those of its index tables
+// that its kernels read: the real outer kernels' pairs (float-float: pos),
+// rev where the four-step twiddles are applied.  Cached for the process.
+enum {NEED_PAIRS=1, NEED_POS=2, NEED_REV=4};
+static int realNeeds(int prec) {return prec == PREC_FF ? NEED_POS : NEED_PAIRS;}
+
+static void fusedTables(FusedFFT& p, int prec, int need=0)
 {
   if(prec == PREC_FF) prec=PREC_F32;
   static std::mutex mu;
-  struct Tables {void *twb, *twj, *pairs, *pos, *rev;};
+  struct Tables {char *roots; size_t inverse; void *pairs, *pos, *rev;};
   static std::map<std::tuple<int,int,std::string>,Tables> cache;
   int dev=0;
   cudaGetDevice(&dev);
   const auto key=std::make_tuple(dev,prec,std::string((const char *) p.radix,
                                                       p.nst));
   std::lock_guard<std::mutex> lock(mu);
-  auto it=cache.find(key);
-  if(it == cache.end()) {
-    const long n=p.n;
-    std::vector<double> c, s;
-    unitRoots(n,c,s);
-    std::vector<long> eb, ej;
-    long nblk=p.radix[0];
-    std::vector<long> rev(p.radix[0]);
-    for(long b=0; b < nblk; ++b) rev[b]=b;
-    std::vector<int4> pairs;
-    std::vector<int> blocks;
-    for(int st=1; st < p.nst; ++st) {
-      const int R=p.radix[st];
-      for(int r=1; r < R; ++r)
-        for(long b=0; b < nblk; ++b)
-          eb.push_back(r*rev[b]*(n/(nblk*R)) % n);
-      if(st == p.nst-1) {
-        blocks.assign(rev.begin(),rev.end());
-        // Partner blocks of the last stage: rev(b) and nblk - rev(b).
-        std::vector<int> at(nblk);
-        for(long b=0; b < nblk; ++b) at[rev[b]]=(int) b;
-        pairs.push_back(make_int4(0,nblk % 2 ? -1 : at[nblk/2],0,0));
-        for(long b=1; b < nblk; ++b) {
-          const long k=rev[b];
-          if(2*k < nblk) pairs.push_back(make_int4((int) b,at[nblk-k],(int) k,
-                                                   0));
-        }
-      }
-      std::vector<long> next(nblk*R);
-      for(long b=0; b < nblk; ++b)
-        for(int r=0; r < R; ++r) next[b*R+r]=rev[b]+nblk*r;
-      rev.swap(next);
-      nblk *= R;
+  Tables& t=cache[key];
+  const bool pairs=(need & NEED_PAIRS) && !t.pairs;
+  const bool pos=(need & NEED_POS) && !t.pos, rev=(need & NEED_REV) && !t.rev;
+  if(!t.roots || pairs || pos || rev) {
+    const FusedHost h=fusedHost(p);
+    if(!t.roots) {
+      std::vector<double> c, s;
+      unitRoots(p.n,1,c,s);
+      std::vector<long> e=h.block;
+      e.insert(e.end(),h.inverse.begin(),h.inverse.end());
+      if(e.empty()) e.push_back(0);
+      t.inverse=h.block.size()*(prec == PREC_F64 ? sizeof(double2) :
+                                sizeof(float4));
+      t.roots=(char *) rootTable(c,s,e,prec);
     }
-    long m=1;
-    for(int st=p.nst-1; st >= 0; --st) {
-      const int R=p.radix[st];
-      for(int r=1; r < R; ++r)
-        for(long j=0; j < m; ++j) ej.push_back(r*j*(n/(R*m)) % n);
-      m *= R;
-    }
-    if(eb.empty()) eb.push_back(0);
-    if(ej.empty()) ej.push_back(0);
-    std::vector<int> pos(n);
-    for(long b=0; b < n; ++b) pos[rev[b]]=(int) b;
-    Tables t={};
-    try {
-      t.twb=rootTable(c,s,eb,prec);
-      t.twj=rootTable(c,s,ej,prec);
-      t.pairs=upload(pairs);
-      t.pos=upload(pos);
-      t.rev=upload(blocks);
-    } catch(...) {
-      for(void *q : {t.twb,t.twj,t.pairs,t.pos,t.rev}) if(q) cudaFree(q);
-      throw;
-    }
-    it=cache.emplace(key,t).first;
+    if(pairs) t.pairs=upload(h.pairs);
+    if(pos) t.pos=upload(h.pos);
+    if(rev) t.rev=upload(h.rev);
   }
-  p.twb=it->second.twb;
-  p.twj=it->second.twj;
-  p.pairs=(const int4 *) it->second.pairs;
-  p.pos=(const int *) it->second.pos;
-  p.rev=(const int *) it->second.rev;
+  p.twb=t.roots;
+  p.twj=t.roots+t.inverse;
+  p.pairs=(const int4 *) t.pairs;
+  p.pos=(const int *) t.pos;
+  p.rev=(const int *) t.rev;
 }
 
 // Teams of a fused row launch: one per row where a team keeps at least eight
@@ -494,6 +510,7 @@ FusedFFT fusedRowPlan(long n, int prec, int A, bool herm, bool half,
 }
 
 void fusedRowTables(FusedFFT& p, int prec) {fusedTables(p,prec);}
+void fusedColumnTables(FusedFFT& p, int prec) {fusedTables(p,prec,NEED_REV);}
 
 // The fused column transforms of the batched launch's long problems.
 FusedFFT fusedColumnPlan(long n, int prec, bool half, int tile)
@@ -596,7 +613,7 @@ static size_t outerBwdNeed(const AxisPlan& a, int prec, int tile)
 // Whether the fused outer kernels of an axis take the staged form: float-float
 // with few columns, where fetching the fused form's code dominates; with many,
 // its fewer passes through shared memory and the halves it leaves out count.
-// Forward kernels of ten axes (60 to 1568 points, centred and half empty),
+// Forward kernels of ten axes (80 to 1568 points, centred and half empty),
 // fused over staged time, geometric mean: 512 columns 1.10, 1024 1.05, 1536
 // 1.03, 2048 0.99, 3072 0.99, 6144 0.97 (18 us fused against 16 staged for 80
 // points of 1024 columns, 92 against 104 for 1536 points of 2048).
@@ -699,8 +716,15 @@ static double fusedCost(long n, int prec, int A, int B, bool herm, bool half)
 static std::vector<long> paddedLengths(long M)
 {
   std::vector<long> v;
-  for(long n=M; n <= M+M/3+8; ++n)
-    if(smooth(n)) v.push_back(n);
+  const long top=M+M/3+8;
+  for(long n7=1; n7 <= top; n7 *= 7)
+    for(long n5=n7; n5 <= top; n5 *= 5)
+      for(long n3=n5; n3 <= top; n3 *= 3) {
+        long n=n3;
+        while(n < M) n *= 2;
+        for(; n <= top; n *= 2) v.push_back(n);
+      }
+  std::sort(v.begin(),v.end());
   return v;
 }
 
@@ -1341,7 +1365,16 @@ Conv *Conv::createSearched(int dim, const int *kinds, const long *L,
        (a.kind != KIND_PAD && a.kind != KIND_CENTERED)) continue;
     cands[d]=residueCandidates(a,d < dim-1,prec,A,B,
                                anyLength(a.kind,a.L,a.M,mult));
-    any=any || cands[d].size() > 1;
+    // Split rows run the same kernel whatever their m.
+    if(d == dim-1 && I0.split > 1)
+      cands[d].erase(std::remove_if(cands[d].begin(),cands[d].end(),
+                                    [&](long m) {
+        long mm=0, q=0, N=0;
+        return planRowLength(a.kind,a.L,a.M,m,A,B,mult,prec,&mm,&q,&N) &&
+          N == a.N;
+      }),cands[d].end());
+    // The base plan has the cheapest one, except for the split rows' lengths.
+    any=any || cands[d].size() > (d == dim-1 && I0.split > 1 ? 0 : 1);
   }
   if(!any) {
     base.reset();
@@ -1381,7 +1414,7 @@ Conv *Conv::createSearched(int dim, const int *kinds, const long *L,
   double bestT=ok ? timeOf(*base) : 1e300;
   base.reset();
   for(int d=0; d < dim && ok && bestT < 1e300; ++d) {
-    if(cands[d].size() < 2) continue;
+    if(cands[d].size() < (d == dim-1 && I0.split > 1 ? 1 : 2)) continue;
     for(long m : cands[d]) {
       long trial[3]={mf[0],mf[1],mf[2]};
       trial[d]=m;
@@ -1430,7 +1463,7 @@ void Conv::tune()
     t.launch=I.longRow ? dim : dim-1;
     long avail=I.longRow ? I.rowQ*nrows : nrows;
     for(int r : {1,2,3,4,6,8}) {
-      if(r > avail) break;
+      if(r > avail || (r > 1 && I.split > 1)) break;
       for(int th : thrs)
         if(innerNeed(I,in,r,th) <= SMEM_MAX) t.cands.push_back({r,th});
     }
@@ -1770,7 +1803,7 @@ cudaError_t Conv::runT(const void *const *in, void *const *out, cudaStream_t s)
     if(P.fused || a.kind == KIND_REAL) {
       P.fz=P.fused ? outerFFT(a,I.prec,a.tile) :
         realFFT(a.N,a.L,I.prec,a.tile);
-      fusedTables(P.fz,I.prec);
+      fusedTables(P.fz,I.prec,P.fused ? 0 : realNeeds(I.prec));
     } else P.fp=fftPlan(a.m,I.prec);
     P.twN=(const typename TwT<T>::type *) twiddles(a.N,I.prec);
     P.twX=NULL; P.NX=1;
@@ -2037,7 +2070,7 @@ cudaError_t Conv::runLong(const void *const *in, void *const *out,
   O.fp=fftPlan(q,I.prec);
   O.twN=(const typename TwT<T>::type *) twiddles(q,I.prec);
   O.twX=(const typename TwT<T>::type *) twiddles(N,I.prec);
-  O.twC=(const typename TwT<T>::type *) twiddles(N,I.prec,256);
+  O.twC=(const typename TwT<T>::type *) coarseRoots(N,I.prec);
   O.NX=N;
   O.io64=io64 & 1; O.ioShift=guard;
   O.conj=0;
@@ -2164,11 +2197,11 @@ cudaError_t Conv::run(const void *const *in, void *const *out, cudaStream_t s)
 void Conv::makeTables()
 {
   const int prec=I.prec, A=I.A;
-  auto make=[&](FusedFFT p) {fusedTables(p,prec);};
+  auto make=[&](FusedFFT p, int need=0) {fusedTables(p,prec,need);};
   for(int d=0; d < I.dim-1; ++d) {
     const AxisPlan& a=I.axis[d];
     if(outerFused(a)) make(outerFFT(a,prec,1));
-    else if(a.kind == KIND_REAL) make(realFFT(a.N,a.L,prec,1));
+    else if(a.kind == KIND_REAL) make(realFFT(a.N,a.L,prec,1),realNeeds(prec));
     else fftPlan(a.m,prec);
     twiddles(a.N,prec);
   }
@@ -2178,7 +2211,7 @@ void Conv::makeTables()
     make(fusedRowPlan(I.rowM,prec,A,false,false,1,widest(prec)));
     fftPlan(I.rowQ,prec);
     twiddles(a.N,prec);
-    twiddles(a.N,prec,256);
+    coarseRoots(a.N,prec);
     return;
   }
   if(a.kind == KIND_HERMITIAN) {
@@ -2638,7 +2671,7 @@ PadTransform::PadTransform(int kind, long L, long M, long C, long mForce,
   if(!deviceReady()) return;
   if(kind == KIND_REAL || kind == KIND_HERMITIAN) {
     FusedFFT f=realFFT(a.N,kind == KIND_REAL ? a.L : a.N,prec,1);
-    fusedTables(f,prec);
+    fusedTables(f,prec,realNeeds(prec));
   } else fftPlan(a.m,prec);
   twiddles(a.N,prec);
 }
@@ -2663,7 +2696,7 @@ cudaError_t PadTransform::runT(const void *in, void *out, bool fwd,
   P.cshift=a.cshift; P.tile=fwd ? a.tile : a.tileB;
   if(a.kind == KIND_REAL || a.kind == KIND_HERMITIAN) {
     P.fz=realFFT(a.N,a.kind == KIND_REAL ? a.L : a.N,prec,P.tile);
-    fusedTables(P.fz,prec);
+    fusedTables(P.fz,prec,realNeeds(prec));
   } else P.fp=fftPlan(a.m,prec);
   P.twN=(const typename TwT<T>::type *) twiddles(a.N,prec);
   P.twX=NULL; P.NX=1;
@@ -2777,7 +2810,7 @@ PlainFFT::PlainFFT(int kind, long n, int sign, long C, long B, long istride,
       fftPlan(n1,prec);
       fftPlan(n2,prec);
       twiddles(n,prec);
-      twiddles(n,prec,256);
+      coarseRoots(n,prec);
     }
     if(devAlloc(&scratch,elem(prec)*(size_t) n*(size_t) B) != cudaSuccess) {
       scratch=NULL;
@@ -2790,7 +2823,7 @@ PlainFFT::PlainFFT(int kind, long n, int sign, long C, long B, long istride,
   if(!deviceReady()) return;
   if(kind != FFT_C2C) {
     FusedFFT f=realFFT(n,n,prec,1);
-    fusedTables(f,prec);
+    fusedTables(f,prec,realNeeds(prec));
   } else fftPlan(n,prec);
   twiddles(n,prec);
 }
@@ -2829,7 +2862,7 @@ cudaError_t PlainFFT::runTwoPass(const void *in, void *out, cudaStream_t s)
   if(sign > 0) {
     base(P,n1);
     P.twX=(const typename TwT<T>::type *) twiddles(n,prec); P.NX=n;
-    P.twC=(const typename TwT<T>::type *) twiddles(n,prec,256);
+    P.twC=(const typename TwT<T>::type *) coarseRoots(n,prec);
     P.tile=tile1;
     P.C=(int) n2; P.inRow=n2; P.outRow=n2;
     P.inBatch=ibatch; P.outBatch=n;
@@ -2852,7 +2885,7 @@ cudaError_t PlainFFT::runTwoPass(const void *in, void *out, cudaStream_t s)
   OuterPlan<T> Q{};
   base(Q,n1);
   Q.twX=(const typename TwT<T>::type *) twiddles(n,prec); Q.NX=n;
-  Q.twC=(const typename TwT<T>::type *) twiddles(n,prec,256);
+  Q.twC=(const typename TwT<T>::type *) coarseRoots(n,prec);
   Q.tile=tile2;
   Q.C=(int) n2; Q.inRow=n2; Q.outRow=n2;
   Q.inBatch=n; Q.outBatch=obatch;
@@ -2870,7 +2903,7 @@ cudaError_t PlainFFT::runT(const void *in, void *out, cudaStream_t s)
   P.tile=tile;
   if(real) {
     P.fz=realFFT(n,n,prec,tile);
-    fusedTables(P.fz,prec);
+    fusedTables(P.fz,prec,realNeeds(prec));
   } else P.fp=fftPlan(n,prec);
   P.twN=(const typename TwT<T>::type *) twiddles(n,prec);
   P.twX=NULL; P.NX=1;

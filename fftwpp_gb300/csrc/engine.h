@@ -46,6 +46,9 @@ int fusedRadices(long n, int prec, int A, bool herm, bool half, int maxR,
                  int *radix);
 int fusedPadding(const int *radix, int nst, int level);
 int rowTeams(int rpc, int threads);
+struct FusedFFT;
+struct FusedHost;
+FusedHost fusedHost(const FusedFFT& p);   // its tables (fft_fused.cuh)
 
 // Whether a convolution's results are the same for every padded length
 // N >= M of an axis (engine.cu).
@@ -353,6 +356,9 @@ private:
 
 // Every step-th t; throws if the table cannot be made.
 const void *twiddles(long n, int prec, long step=1);
+// FP32: every 256th, the second factor of the four-step twiddles (fourStep in
+// kernels.cu); NULL where they are read whole.
+const void *coarseRoots(long n, int prec);
 
 // Every device allocation of the library goes through devAlloc.  Failure
 // injection for tests (host side): failAllocationAfter(n) makes the n-th

@@ -35,6 +35,8 @@
 
 #include "fft_smem.cuh"
 
+#include <vector>
+
 namespace fgb {
 
 #define FGB_FUSED_STAGES 12
@@ -59,6 +61,14 @@ struct FusedFFT {
   const int *pos;          // position of natural index k after the last
                            // forward stage
   const int *rev;          // rev(b) of the last stage's blocks
+};
+
+// The same tables on the host (fusedHost in engine.cu), twiddles as exponents
+// of W_n.
+struct FusedHost {
+  std::vector<long> block, inverse;
+  std::vector<int4> pairs;
+  std::vector<int> pos, rev;
 };
 
 // Whether a plan holds a radix-16 stage (its kernels need the WIDE form).

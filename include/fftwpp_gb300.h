@@ -369,6 +369,17 @@ int fgb_row_length(int kind, size_t L, size_t M, size_t m, int A, int B,
 int fgb_fused_radices(size_t n, int precision, int inputs, int hermitian,
                       int half, int *radix, int max, int *padding);
 
+/* The tables those transforms read (host arithmetic, no GPU): exponents t of
+ * W_n^t of the block twiddles (n - R_0 entries: stage s >= 1 with nblk blocks
+ * from nblk - R_0 on, (r-1) nblk + b) and of the inverse ones (n - 1: stage s
+ * of span m from m - 1 on, (r-1) m + j), the last stage's block pairs (b,
+ * partner or -1, index; ceil(nblk/2) of them), the position of each natural
+ * index (n) and the natural index of each last block (nblk).  Every array
+ * holds n entries, pairs 3 n.  Returns nblk, or -1. */
+int fgb_fused_tables(size_t n, int precision, int inputs, int hermitian,
+                     int half, long *block, long *inverse, int *pairs,
+                     int *pos, int *rev);
+
 /* Transformed index of entry i of residue block r (fftBase::index,
  * convolve.h:297-326, and fftPadReal::index, convolve.h:956-979) for the
  * reference's parameters (m,p,q,n,D) of a 1D transform. */
