@@ -79,13 +79,18 @@ class AdvectionJacobian:
         self.lib = _native.load()
         self.shape = self.fwd.shape
         self.dtype = self.fwd.dtype
-        # i kx (a column) and i ky (a row) of the operator's own type, made
-        # once: forming them on every call took 20 us of a 285 us FP32 step
-        # of 1023 x 512 modes.  Complete before any stream can use them.
-        kx, ky = wavenumbers(Lx, Ly, torch.device("cuda"),
-                             self.dtype.to_real())
-        self._ik = (1j * kx[:, :1]).contiguous(), (1j * ky[:1]).contiguous()
-        torch.cuda.current_stream().synchronize()
+        # i kx and i ky of the operator's own type, made once (a column and
+        # a row, as views of the grid): forming them on every call took 20 us
+        # of a 285 us FP32 step of 1023 x 512 modes.  Complete before any
+        # stream can use them, and ordinary tensors, which autograd can save,
+        # wherever the operator is made.
+        with torch.inference_mode(False):
+            kx, ky = wavenumbers(Lx, Ly, torch.device("cuda"),
+                                 self.dtype.to_real())
+            self._ik = ((1j * kx[:, :1]).expand_as(kx),
+                        (1j * ky[:1]).expand_as(ky))
+        self._ik_stream = torch.cuda.current_stream()
+        self._ik_stream.synchronize()
 
     def scale_columns(self, t, s0, s1):
         rows, cols = t.shape
@@ -111,6 +116,13 @@ class AdvectionJacobian:
                                  psi.real.dtype)
             ikx = 1j * kx
             iky = 1j * ky
+        else:
+            # Their memory may outlast the operator only on the stream it
+            # came from; any other has to be known to the allocator.
+            s = torch.cuda.current_stream(ikx.device)
+            if s != self._ik_stream:
+                ikx.record_stream(s)
+                iky.record_stream(s)
         return self.jacobian(ikx * psi, iky * psi, ikx * omega, iky * omega)
 
 
