@@ -120,8 +120,9 @@ BatchConv::BatchConv(int nprob, const long *L, const long *M,
     throw std::runtime_error("batched problems are fftPad or fftPadCentered");
   if(prec != PREC_F64 && prec != PREC_F32)
     throw std::runtime_error("batched problems run in FP64 or FP32");
-  // Per-task shared memory: three CTAs per SM (a larger FP64 budget with
-  // two CTAs per SM measured slower).
+  // Per-task shared memory: room for three CTAs per SM.  The FP64 kernel's
+  // registers allow two (batchBlocks in kernels.cu), but a budget for two
+  // measured slower before it took the fused transforms; not measured since.
   budget=72*1024;
   Ls.assign(L,L+nprob);
   Ms.assign(M,M+nprob);
@@ -394,8 +395,7 @@ void BatchConv::build()
       G.scale=(T) (1.0/(double) N);
       for(int b=0; b < B; ++b) G.out[b]=(cplx<T> *) (offsets[i]*e);
       // Several rows per row task where they fit the budget.
-      // The rows hold one residue of one fold: the direct row variant
-      // (no staging, in-place transforms).
+      // The rows hold one residue of one fold: the fused rows.
       int rpc=1;
       while(2*rpc <= 8 && 2*rpc <= qc &&
             fusedNeedB(prec,m,A,false,2*rpc) <= budget) rpc *= 2;

@@ -2082,7 +2082,7 @@ cudaError_t Conv::runLong(const void *const *in, void *const *out,
   e=launchOuterFwd<T>(O,threads,s);
   tick(s);
   if(e != cudaSuccess) return e;
-  // Rows of length m: one residue, one fold (the direct row variant).
+  // Rows of length m: one residue, one fold: the fused rows.
   RowPlan<T> P{};
   P.im=*im;
   P.L=(int) m; P.m=(int) m; P.q=1; P.N=(int) m; P.cshift=0;

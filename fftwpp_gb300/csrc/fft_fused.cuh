@@ -453,10 +453,10 @@ __device__ __forceinline__ int runFusedMiddle(cplx<T> *x, int cs, int ncol,
 // and stores of column tiles are loops of their own around the stages, and
 // all stages of a radix, forward and inverse, share one piece of code.
 //
-// Float-float takes it everywhere: one of its butterflies is up to 14 KB of
-// instructions and its kernels are bound by fetching them.  With the last
-// forward stage, the product and the first inverse stage fused, a Hermitian
-// row kernel of 768 points stalled on instructions 3.8 times per issue
+// Float-float takes it but for outer axes of many columns (stagedColumns in
+// engine.cu): one of its butterflies is up to 14 KB of instructions and its
+// kernels are bound by fetching them.  With the last forward stage, the
+// product and the first inverse stage fused, a Hermitian row kernel of 768 points stalled on instructions 3.8 times per issue
 // against 0.9 here (89 against 72 us), and a 39 x 93 convolution took 43 us
 // against 34.  Only complex rows keep their first and last stages fused (the
 // half that padding leaves empty is not computed there): 4096 pairs of 1024

@@ -137,9 +137,10 @@ struct OuterPlan {
   int tile;
   int io64;                // as RowPlan::io64
   const int *ioShift;      // as RowPlan::ioShift
-  int fused;               // L <= m and no twX: the fused kernels, with the
-                           // rows of a residue block in fz's digit-reversed
-                           // order
+  int fused;               // L <= m: the fused kernels, with the rows of a
+                           // residue block in fz's digit-reversed order
+                           // (the long-row path's twX launches do not take
+                           // them, the batched launch's do)
   int staged;              // fused, float-float: the staged form (runStages)
   int conj;                // real kernels: conjugate the complex side
                            // (the sign -1 r2c / sign +1 c2r of plain FFTs)
@@ -155,10 +156,12 @@ struct OuterPlan {
                            // real array
   long long flatC;
   T scale;
-  FFTPlanDev fp;           // length-m (complex) or length-N/2 (real) FFT
-  FusedFFT fz;             // the fused kernels' length-m (N/2) FFT
+  FFTPlanDev fp;           // length-m FFT of the natural-order kernels
+  FusedFFT fz;             // length-m FFT of the fused ones, length-N/2 FFT
+                           // of the real ones
   const typename TwT<T>::type *twN;
-  const typename TwT<T>::type *twX;  // optional W_NX^{col*k} (1D long path)
+  const typename TwT<T>::type *twX;  // optional W_NX^{col*k}: long rows, the
+                                     // batch's long problems, two-pass FFTs
   const typename TwT<T>::type *twC;  // FP32: W_NX^{256 i} (fourStep)
   long long NX;
 };
