@@ -443,7 +443,24 @@ FusedHost fusedHost(const FusedFFT& p)
 // that its kernels read: the real outer kernels' pairs (float-float: pos),
 // rev where the four-step twiddles are applied.  Cached for the process.
 enum {NEED_PAIRS=1, NEED_POS=2, NEED_REV=4};
-static int realNeeds(int prec) {return prec == PREC_FF ? NEED_POS : NEED_PAIRS;}
+
+// Whether the real outer kernels of length N on so many columns (all the
+// launch's inputs or outputs and batches) take the staged form.  FP64 always:
+// forward, fused against staged, us, N = 48 of 2592 columns 19.7 / 12.3, N =
+// 64 of 131072 480 / 251, N = 256 of 18180 142 / 132, N = 512 of 131072 1866 /
+// 1858; only N = 180 = 2 (2 5 3 3) is slower, 199 / 203.  FP32 below 2^20
+// points: 10.5 / 8.5 at 124416 (N = 48), 11.0 / 10.4 at 786432 (N = 96), 12.3
+// / 12.9 at 2097152 (N = 256), 174 / 321 at 67108864 (N = 512).
+static bool stagedReal(int prec, long long N, long long columns)
+{
+  return prec != PREC_F32 || N*columns < (1 << 20);
+}
+
+// The index table the kernels of such launches read.
+static int realNeeds(int prec, long long N, long long columns)
+{
+  return stagedReal(prec,N,columns) ? NEED_POS : NEED_PAIRS;
+}
 
 static void fusedTables(FusedFFT& p, int prec, int need=0)
 {
@@ -623,6 +640,12 @@ static size_t outerBwdNeed(const AxisPlan& a, int prec, int tile)
 static bool stagedColumns(int prec, long long columns)
 {
   return prec == PREC_FF && columns < 2048;
+}
+
+static bool stagedOuter(int prec, const AxisPlan& a, long long columns)
+{
+  return a.kind == KIND_REAL ? stagedReal(prec,a.N,columns) :
+    stagedColumns(prec,columns);
 }
 
 // The transform of a split row's CTAs.
@@ -1803,7 +1826,7 @@ cudaError_t Conv::runT(const void *const *in, void *const *out, cudaStream_t s)
     if(P.fused || a.kind == KIND_REAL) {
       P.fz=P.fused ? outerFFT(a,I.prec,a.tile) :
         realFFT(a.N,a.L,I.prec,a.tile);
-      fusedTables(P.fz,I.prec,P.fused ? 0 : realNeeds(I.prec));
+      fusedTables(P.fz,I.prec,P.fused ? 0 : axisNeeds());
     } else P.fp=fftPlan(a.m,I.prec);
     P.twN=(const typename TwT<T>::type *) twiddles(a.N,I.prec);
     P.twX=NULL; P.NX=1;
@@ -1922,7 +1945,7 @@ cudaError_t Conv::runT(const void *const *in, void *const *out, cudaStream_t s)
       O.inRow=strideS[0];
       O.Ltot=LLONG_MAX;
     }
-    O.staged=stagedColumns(I.prec,C*A);
+    O.staged=stagedOuter(I.prec,ax,C*A);
     O.scale=(T) 1;
     O.io64=IN64;
     for(int i=0; i < A; ++i) {O.in[i]=(const Cx *) in[i]; O.out[i]=(Cx *) bufs[i];}
@@ -1952,7 +1975,7 @@ cudaError_t Conv::runT(const void *const *in, void *const *out, cudaStream_t s)
     if(e != cudaSuccess) return e;
     O.count=B;
     retile(O,ax);
-    O.staged=stagedColumns(I.prec,C*B);
+    O.staged=stagedOuter(I.prec,ax,C*B);
     O.scale=(T) scale;
     O.io64=OUT64;
     O.inRow=C;                                  // staging side
@@ -1976,7 +1999,7 @@ cudaError_t Conv::runT(const void *const *in, void *const *out, cudaStream_t s)
   outerPlan(X,ax);
   X.count=A; X.nbatch=1; X.inBatch=X.outBatch=0;
   X.inRow=Cx_; X.outRow=Cx_; X.C=(int) Cx_; X.Ltot=(long long) ax.L*Cx_;
-  X.staged=stagedColumns(I.prec,(long long) Cx_*A);
+  X.staged=stagedOuter(I.prec,ax,(long long) Cx_*A);
   X.scale=(T) 1;
   X.io64=IN64;
   if(isStrided) {                   // data side (the caller's arrays)
@@ -1994,7 +2017,7 @@ cudaError_t Conv::runT(const void *const *in, void *const *out, cudaStream_t s)
   Y.count=A; Y.nbatch=(int) ax.rows;
   Y.inBatch=ay.L*nz; Y.outBatch=ay.rows*nz;
   Y.inRow=nz; Y.outRow=nz; Y.C=(int) nz; Y.Ltot=(long long) ay.L*nz;
-  Y.staged=stagedColumns(I.prec,(long long) nz*ax.rows*A);
+  Y.staged=stagedOuter(I.prec,ay,(long long) nz*ax.rows*A);
   Y.scale=(T) 1;
   for(int i=0; i < A; ++i) {Y.in[i]=(const Cx *) bx[i]; Y.out[i]=(Cx *) by[i];}
   e=launchOuterFwd<T>(Y,ay.thr,s);
@@ -2025,7 +2048,7 @@ cudaError_t Conv::runT(const void *const *in, void *const *out, cudaStream_t s)
 
   Y.count=B;
   retile(Y,ay);
-  Y.staged=stagedColumns(I.prec,(long long) nz*ax.rows*B);
+  Y.staged=stagedOuter(I.prec,ay,(long long) nz*ax.rows*B);
   for(int i=0; i < B; ++i) {Y.in[i]=(const Cx *) by[i]; Y.out[i]=(Cx *) bx[i];}
   std::swap(Y.inBatch,Y.outBatch);
   e=launchOuterBwd<T>(Y,ay.thrB,s);
@@ -2034,7 +2057,7 @@ cudaError_t Conv::runT(const void *const *in, void *const *out, cudaStream_t s)
 
   X.count=B;
   retile(X,ax);
-  X.staged=stagedColumns(I.prec,(long long) Cx_*B);
+  X.staged=stagedOuter(I.prec,ax,(long long) Cx_*B);
   X.scale=(T) scale;
   X.io64=OUT64;
   X.inRow=Cx_;                                  // staging side
@@ -2191,6 +2214,14 @@ cudaError_t Conv::run(const void *const *in, void *const *out, cudaStream_t s)
     });
 }
 
+// Index tables of a real outer axis: of its forward and its backward launch.
+int Conv::axisNeeds() const
+{
+  const AxisPlan& a=I.axis[0];
+  const long long C=(long long) elements()/a.L;
+  return realNeeds(I.prec,a.N,C*I.A) | realNeeds(I.prec,a.N,C*I.B);
+}
+
 // The tables of every launch, made with the plan: its first run may be under
 // stream capture, where nothing can be allocated, and a table that cannot be
 // made is an error of the plan's creation.
@@ -2201,7 +2232,7 @@ void Conv::makeTables()
   for(int d=0; d < I.dim-1; ++d) {
     const AxisPlan& a=I.axis[d];
     if(outerFused(a)) make(outerFFT(a,prec,1));
-    else if(a.kind == KIND_REAL) make(realFFT(a.N,a.L,prec,1),realNeeds(prec));
+    else if(a.kind == KIND_REAL) make(realFFT(a.N,a.L,prec,1),axisNeeds());
     else fftPlan(a.m,prec);
     twiddles(a.N,prec);
   }
@@ -2671,7 +2702,7 @@ PadTransform::PadTransform(int kind, long L, long M, long C, long mForce,
   if(!deviceReady()) return;
   if(kind == KIND_REAL || kind == KIND_HERMITIAN) {
     FusedFFT f=realFFT(a.N,kind == KIND_REAL ? a.L : a.N,prec,1);
-    fusedTables(f,prec,realNeeds(prec));
+    fusedTables(f,prec,realNeeds(prec,a.N,C));
   } else fftPlan(a.m,prec);
   twiddles(a.N,prec);
 }
@@ -2696,7 +2727,8 @@ cudaError_t PadTransform::runT(const void *in, void *out, bool fwd,
   P.cshift=a.cshift; P.tile=fwd ? a.tile : a.tileB;
   if(a.kind == KIND_REAL || a.kind == KIND_HERMITIAN) {
     P.fz=realFFT(a.N,a.kind == KIND_REAL ? a.L : a.N,prec,P.tile);
-    fusedTables(P.fz,prec,realNeeds(prec));
+    fusedTables(P.fz,prec,realNeeds(prec,a.N,C));
+    P.staged=stagedReal(prec,a.N,C);
   } else P.fp=fftPlan(a.m,prec);
   P.twN=(const typename TwT<T>::type *) twiddles(a.N,prec);
   P.twX=NULL; P.NX=1;
@@ -2823,7 +2855,7 @@ PlainFFT::PlainFFT(int kind, long n, int sign, long C, long B, long istride,
   if(!deviceReady()) return;
   if(kind != FFT_C2C) {
     FusedFFT f=realFFT(n,n,prec,1);
-    fusedTables(f,prec,realNeeds(prec));
+    fusedTables(f,prec,realNeeds(prec,n,C*B));
   } else fftPlan(n,prec);
   twiddles(n,prec);
 }
@@ -2903,7 +2935,8 @@ cudaError_t PlainFFT::runT(const void *in, void *out, cudaStream_t s)
   P.tile=tile;
   if(real) {
     P.fz=realFFT(n,n,prec,tile);
-    fusedTables(P.fz,prec,realNeeds(prec));
+    fusedTables(P.fz,prec,realNeeds(prec,n,C*B));
+    P.staged=stagedReal(prec,n,C*B);
   } else P.fp=fftPlan(n,prec);
   P.twN=(const typename TwT<T>::type *) twiddles(n,prec);
   P.twX=NULL; P.NX=1;

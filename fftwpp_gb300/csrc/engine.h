@@ -267,6 +267,7 @@ private:
   cudaError_t planOutputs(cudaStream_t s);
   void allocate();
   void makeTables();
+  int axisNeeds() const;
   void tune();
   bool directSegments() const;
   cudaError_t runZeroCopy(const void *const *hin, const void *const *in,

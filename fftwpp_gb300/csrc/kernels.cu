@@ -297,10 +297,10 @@ outerBwdKernel(const OuterPlan<T> P)
 // row order and the backward undoes it).  The column tile's values cross
 // shared memory once between stages and never before the first or after
 // the last.
-// Float-float (runStages): the tile's inputs into shared memory, and its
+// The staged form (runStages): the tile's inputs into shared memory, and its
 // outputs out of it.  in(cc, j) gives element j of column cc.
 template<typename T, class In>
-__device__ __forceinline__ void loadTileFF(cplx<T> *x, const FusedFFT& p,
+__device__ __forceinline__ void loadTile(cplx<T> *x, const FusedFFT& p,
                                            int lt, int tid, int nthr,
                                            const In& in)
 {
@@ -324,7 +324,7 @@ __device__ __forceinline__ cplx<ff> fromBits(cplx<ff> v, int sh)
 }
 
 template<typename T, class Store>
-__device__ __forceinline__ void storeTileFF(const cplx<T> *x,
+__device__ __forceinline__ void storeTile(const cplx<T> *x,
                                             const FusedFFT& p, int lt, int tid,
                                             int nthr, const Store& store)
 {
@@ -408,7 +408,7 @@ __device__ __forceinline__ void outerFwdFused(const OuterPlan<T>& P, int ctile,
     };
   };
   if(std::is_same<T,ff>::value && P.staged) {
-    loadTileFF(x,P.fz,lt,tid,nthr,[&](int cc, int j) {
+    loadTile(x,P.fz,lt,tid,nthr,[&](int cc, int j) {
         int s=j+c;
         if(s >= m) s -= m;
         cplx<T> v=mk((T) 0,(T) 0);
@@ -512,12 +512,12 @@ __device__ __forceinline__ void outerBwdFused(const OuterPlan<T>& P, int ctile,
       };
     };
     if(std::is_same<T,ff>::value && P.staged) {
-      loadTileFF(x,P.fz,lt,tid,nthr,[&](int cc, int j) {
+      loadTile(x,P.fz,lt,tid,nthr,[&](int cc, int j) {
           return col0+cc < P.C ? swapXY(sr[j*P.inRow+col0+cc]) :
             mk((T) 0,(T) 0);
         });
       runStages<T>(x,0,0,1,P.fz,lt,0,0,tid,nthr,[] {});
-      storeTileFF(x,P.fz,lt,tid,nthr,store);
+      storeTile(x,P.fz,lt,tid,nthr,store);
     } else {
       FGB_FUSED_SWITCH(P.fz.radix[P.fz.nst-1],
                        (outerFirstInv<T,R_,CG>(P,x,sr,col0,tid,nthr)))
@@ -565,7 +565,11 @@ outerBwdFusedKernel16(const OuterPlan<T> P)
 // block of nblk - kappa, so one thread finishes both blocks of a pair
 // (FusedFFT::pairs, blocks in order: b, its partner, kappa; the first entry
 // holds blocks 0 and that of nblk/2, -1 if nblk is odd, which are their own
-// partners).  The inverse packs in the same pairs as it loads.
+// partners).  The inverse packs in the same pairs as it loads.  That is the
+// fused form, which FP32 takes for large launches; in FP64 and float-float,
+// and in small FP32 launches, a pair's two butterflies one after the other
+// leave most threads idle or waiting, and the staged form, one mode pair at a
+// time, is faster (stagedReal in engine.cu).
 
 // F[k] = e + W_N^k o and F[Nh-k] = conj(e - W_N^k o) from Z[k] and
 // Z[Nh-k], e = (Z[k] + conj Z[Nh-k])/2, o = -i (Z[k] - conj Z[Nh-k])/2.
@@ -686,8 +690,8 @@ __device__ __forceinline__ void outerRealFwd(const OuterPlan<T>& P,
       return v;
     };
   };
-  if constexpr(std::is_same<T,ff>::value) {
-    loadTileFF(x,P.fz,lt,tid,nthr,[&](int cc, int j) {
+  if(!std::is_same<T,float>::value || P.staged) {
+    loadTile(x,P.fz,lt,tid,nthr,[&](int cc, int j) {
         const int s=2*j, top=col0+cc < P.C ? L : 0;
         const T *f=src+dataCol(P,col0+cc);
         cplx<T> v=mk((T) 0,(T) 0);
@@ -698,7 +702,7 @@ __device__ __forceinline__ void outerRealFwd(const OuterPlan<T>& P,
         }
         return v;
       });
-    runStages<T>(x,0,1,0,P.fz,lt,0,0,tid,nthr,[] {});
+    runStages<T,WIDE>(x,0,1,0,P.fz,lt,0,0,tid,nthr,[] {});
     const int Nh=P.N/2, top=P.kc > 0 ? P.kc : Nh+1;
 #pragma unroll 2
     for(int idx=tid; idx < (Nh/2+1) << lt; idx += nthr) {
@@ -713,11 +717,13 @@ __device__ __forceinline__ void outerRealFwd(const OuterPlan<T>& P,
     }
     return;
   }
-  runFusedFirst<T,WIDE>(x,0,1,P.fz,lt,tid,nthr,load);
-  runFusedMiddle<T,WIDE>(x,0,1,P.fz,lt,false,0,tid,nthr);
-  __syncthreads();
-  FGB_FUSED_SWITCH(P.fz.radix[P.fz.nst-1],
-                   (realLastFwd<T,R_>(P,x,dst,col0,tid,nthr)))
+  if constexpr(std::is_same<T,float>::value) {
+    runFusedFirst<T,WIDE>(x,0,1,P.fz,lt,tid,nthr,load);
+    runFusedMiddle<T,WIDE>(x,0,1,P.fz,lt,false,0,tid,nthr);
+    __syncthreads();
+    FGB_FUSED_SWITCH(P.fz.radix[P.fz.nst-1],
+                     (realLastFwd<T,R_>(P,x,dst,col0,tid,nthr)))
+  }
 }
 
 template<typename T, int R>
@@ -804,7 +810,7 @@ __device__ __forceinline__ void outerRealBwd(const OuterPlan<T>& P,
       if(s+1 < top) storeIOr(f+(s+1)*P.outRow,v.y,P.io64 & 2,sh);
     };
   };
-  if constexpr(std::is_same<T,ff>::value) {
+  if(!std::is_same<T,float>::value || P.staged) {
     const int Nh=P.N/2, top=P.kc > 0 ? P.kc : Nh+1;
 #pragma unroll 2
     for(int idx=tid; idx < (Nh/2+1) << lt; idx += nthr) {
@@ -825,15 +831,17 @@ __device__ __forceinline__ void outerRealBwd(const OuterPlan<T>& P,
       if(k != 0 && kk != k)
         x[(spl(P.fz.pos[kk],P.fz.lg) << lt)+cc]=swapXY(Yc);
     }
-    runStages<T>(x,0,0,1,P.fz,lt,0,0,tid,nthr,[] {});
-    storeTileFF(x,P.fz,lt,tid,nthr,store);
+    runStages<T,WIDE>(x,0,0,1,P.fz,lt,0,0,tid,nthr,[] {});
+    storeTile(x,P.fz,lt,tid,nthr,store);
     return;
   }
-  FGB_FUSED_SWITCH(P.fz.radix[P.fz.nst-1],
-                   (realFirstInv<T,R_>(P,x,src,col0,tid,nthr)))
-  runFusedMiddle<T,WIDE>(x,0,1,P.fz,lt,true,0,tid,nthr);
-  __syncthreads();
-  runFusedLast<T,WIDE>(x,0,1,P.fz,lt,tid,nthr,store);
+  if constexpr(std::is_same<T,float>::value) {
+    FGB_FUSED_SWITCH(P.fz.radix[P.fz.nst-1],
+                     (realFirstInv<T,R_>(P,x,src,col0,tid,nthr)))
+    runFusedMiddle<T,WIDE>(x,0,1,P.fz,lt,true,0,tid,nthr);
+    __syncthreads();
+    runFusedLast<T,WIDE>(x,0,1,P.fz,lt,tid,nthr,store);
+  }
 }
 
 template<typename T, bool WIDE>

@@ -141,7 +141,8 @@ struct OuterPlan {
                            // residue block in fz's digit-reversed order
                            // (the long-row path's twX launches do not take
                            // them, the batched launch's do)
-  int staged;              // fused, float-float: the staged form (runStages)
+  int staged;              // the staged form (runStages): fused float-float,
+                           // or real FP32, launches
   int conj;                // real kernels: conjugate the complex side
                            // (the sign -1 r2c / sign +1 c2r of plain FFTs)
   int cz;                  // data side with strides: column c lies at
