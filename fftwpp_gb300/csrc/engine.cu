@@ -569,6 +569,21 @@ static size_t fusedRowNeed(int prec, long n, int A, bool herm, bool half,
   return FGB_BY_PREC(prec,fusedRowSmem,p.n,p.lg,A,teams);
 }
 
+// Whether Hermitian rows of half length Nh take the ping-pong kernel: FP64,
+// but for long rows of four inputs or more, whose two buffers leave few CTAs
+// an SM, and which take the staged form.  Ping-pong against staged (and, in
+// brackets, the fused form that FP64 took instead), us, 1536 rows: two
+// inputs, Nh = 27 14.7 / 19.3 (27.0), 48 21.2 / 28.8 (32.5), 96 33.1 / 41.0
+// (42.9), 192 64.6 / 74.6 (74.9), 288 101.8 / 108.9 (109.1), 384 135.1 / 125.3
+// (137.2), 576 206.8 / 210.6 (219.9), 768 250.4 / 253.2 (254.6); four inputs,
+// 192 99.9 / 99.6 (118.9), 384 212.6 / 199.6 (211.6), 768 410.3 / 413.2
+// (423.1); the adjoint's five, 288 265.2 / 271.3 (284.9), 384 374.1 / 349.3
+// (367.8), 768 813.9 / 742.3 (757.3).
+static bool hermPingPong(int prec, long Nh, int A)
+{
+  return prec == PREC_F64 && !(A >= 4 && Nh >= 384);
+}
+
 // Shared memory of the innermost axis' row kernel, as planned.
 static size_t innerNeed(const ConvInfo& I, const AxisPlan& a, int rpc,
                         int threads)
@@ -576,7 +591,9 @@ static size_t innerNeed(const ConvInfo& I, const AxisPlan& a, int rpc,
   if(I.longRow)
     return fusedRowNeed(I.prec,I.rowM,I.A,false,false,rpc,threads);
   if(a.kind == KIND_HERMITIAN)
-    return fusedRowNeed(I.prec,a.N/2,I.A,true,false,rpc,threads);
+    return hermPingPong(I.prec,a.N/2,I.A) ?
+      hermRowSmem<double>(a.N/2,I.A,rpc) :
+      fusedRowNeed(I.prec,a.N/2,I.A,true,false,rpc,threads);
   if(rowDirect(a))
     return fusedRowNeed(I.prec,a.m,I.A,false,halfEmpty(a),rpc,threads);
   return rowNeed(I.prec,a.stored,a.m,I.A,I.B,rpc);
@@ -865,16 +882,24 @@ static bool planRowHermitian(AxisPlan& a, long mForce, int A, int B, int prec,
     M=std::max<long>(M,mForce*q);
   }
   a.N=evenSmooth(M);
-  // Another even length a third longer at most where its stages cost less.
-  if(longer && mForce <= 0 && hermNeed(prec,a.N/2,A) <= SMEM_MAX) {
-    double best=fusedCost(a.N/2,prec,A,B,true,false);
-    for(long n : paddedLengths(a.N/2)) {
-      const double cost=fusedCost(n,prec,A,B,true,false);
-      if(cost < best && hermNeed(prec,n,A) <= SMEM_MAX) {
-        best=cost;
+  // Another even length a third longer at most where its stages cost less;
+  // for the ping-pong kernel, at least 7 % less, and rows of 120 points or
+  // more: shorter ones, and small savings, are eaten by the longer row's own
+  // loads and threads (1536 FP64 rows, us: 27 -> 32 points 14.7 -> 17.2, 75 ->
+  // 80 32.7 -> 32.9, 375 of 135 -> 144 20.1 -> 23.1; but 240 -> 256 92 -> 80,
+  // 450 -> 512 209 -> 159).
+  const bool pingpong=hermPingPong(prec,a.N/2,A);
+  if(longer && mForce <= 0 && hermNeed(prec,a.N/2,A) <= SMEM_MAX &&
+     !(pingpong && a.N/2 < 120)) {
+    auto cost=[&](long n) {
+      return pingpong ? fftInstr(n) : fusedCost(n,prec,A,B,true,false);
+    };
+    double best=(pingpong ? 0.93 : 1.0)*cost(a.N/2);
+    for(long n : paddedLengths(a.N/2))
+      if(cost(n) < best && hermNeed(prec,n,A) <= SMEM_MAX) {
+        best=cost(n);
         a.N=2*n;
       }
-    }
   }
   a.m=a.N; a.q=1; a.p=1;
   a.cshift=0;
@@ -1811,9 +1836,13 @@ cudaError_t Conv::runT(const void *const *in, void *const *out, cudaStream_t s)
     P.rpc=a.rpc;
     P.nteam=rowTeams(P.rpc,a.thr);
     P.io64=0;
-    P.fz=fusedRowPlan(a.N/2,I.prec,A,true,false,P.nteam,
-                      widest(I.prec,a.N/2));
-    fusedTables(P.fz,I.prec);
+    P.pingpong=hermPingPong(I.prec,a.N/2,A);
+    if(P.pingpong) P.fp=fftPlan(a.N/2,I.prec);
+    else {
+      P.fz=fusedRowPlan(a.N/2,I.prec,A,true,false,P.nteam,
+                        widest(I.prec,a.N/2));
+      fusedTables(P.fz,I.prec);
+    }
     P.twN=(const typename TwT<T>::type *) twiddles(a.N,I.prec);
   };
   auto outerPlan=[&](OuterPlan<T>& P, const AxisPlan& a) {
@@ -2246,7 +2275,8 @@ void Conv::makeTables()
     return;
   }
   if(a.kind == KIND_HERMITIAN) {
-    make(fusedRowPlan(a.N/2,prec,A,true,false,1,widest(prec,a.N/2)));
+    if(hermPingPong(prec,a.N/2,A)) fftPlan(a.N/2,prec);
+    else make(fusedRowPlan(a.N/2,prec,A,true,false,1,widest(prec,a.N/2)));
     return;
   }
   if(I.split > 1) make(splitPlan(a.N,I.split,A,prec));

@@ -462,9 +462,10 @@ __device__ __forceinline__ int runFusedMiddle(cplx<T> *x, int cs, int ncol,
 // half that padding leaves empty is not computed there): 4096 pairs of 1024
 // points, 454 against 497 us.
 //
-// The other precisions take it for rows whose fused first stage would leave
-// threads of the team without a butterfly: 320 Hermitian FP64 rows of 160
-// points took 32 us fused, with 32 butterfly pairs for 128 threads.
+// FP64 takes it for real outer axes and for those Hermitian rows that do not
+// take the ping-pong transform (stagedReal and hermPingPong in engine.cu), FP32
+// for small real outer launches, and both for rows whose fused first stage
+// would leave threads of the team without a butterfly.
 //
 // The forward stages from `first` on for A columns at x (cs apart, each of
 // 2^lt interleaved ones), mid(), the inverse stages down to `first` for B

@@ -114,8 +114,10 @@ struct HermRowPlan {
   int nteam;               // as RowPlan::nteam
   int io64;                // as RowPlan::io64
   const int *ioShift;      // as RowPlan::ioShift
+  int pingpong;            // FP64: hermRowPingPongKernel, transformed by fp
   T scale;
   FusedFFT fz;             // length-Nh complex FFT
+  FFTPlanDev fp;           // the same for the ping-pong kernel
   const typename TwT<T>::type *twN;   // W_N^t, t < N
   IndexMap im;             // slot positions (position-dependent multipliers)
 };
@@ -291,6 +293,11 @@ template<typename T> size_t outerFwdSmem(int L, int m, int tile);
 // sizes for any residue count.
 template<typename T> size_t outerBwdSmem(int L, int m, int tile, int q=0);
 template<typename T> size_t outerRealSmem(int L, int Nh, int tile);
+// Two buffers of the ping-pong Hermitian rows.
+template<typename T> size_t hermRowSmem(int Nh, int A, int rpc)
+{
+  return sizeof(cplx<T>)*2*(size_t) padded(Nh*A*rpc);
+}
 // Fused kernels: nteam rows of A columns; a tile of columns (and, backward
 // with several residues, its accumulator).
 template<typename T> size_t fusedRowSmem(int n, int lg, int A, int nteam)

@@ -28,10 +28,8 @@
 //  * sizes whose staging does not fit in the array are rejected with an
 //    error before anything is launched.
 //
-// It reuses the engine's kernels unchanged (outerFwdKernel, hermRowKernel,
-// outerBwdKernel) with explicit padding on both axes.  The x transform is
-// the natural-order one, whose single table is the smallest; the rows'
-// fused transform takes two tables of its length and half of the W_N one.
+// It reuses the engine's kernels unchanged (outerFwdKernel,
+// hermRowPingPongKernel, outerBwdKernel) with explicit padding on both axes.
 #include "engine.h"
 #include "kernels.cuh"
 
@@ -67,58 +65,14 @@ cudaError_t scratchPointer(void **ptr)
   return cudaSuccess;
 }
 
-// W_n^t = exp(2 pi i t/n), t < count, written into the scratch array.
-__global__ void fillTwiddles(double2 *tw, int n, int count)
+// W_n^t = exp(2 pi i t/n), t < n, written into the scratch array.
+__global__ void fillTwiddles(double2 *tw, int n)
 {
   int t=blockIdx.x*blockDim.x+threadIdx.x;
-  if(t >= count) return;
+  if(t >= n) return;
   double s, c;
   sincospi(2.0*(double) t/(double) n,&s,&c);
   tw[t]=make_double2(c,s);
-}
-
-// The block and input twiddle tables of a fused FP64 transform
-// (fft_fused.cuh), one entry per thread.
-__global__ void fillFused(double2 *twb, double2 *twj, const fgb::FusedFFT p)
-{
-  const int i=blockIdx.x*blockDim.x+threadIdx.x;
-  if(i >= p.n) return;
-  const int R0=p.radix[0];
-  int nblk=R0;
-  for(int s=1; s < p.nst; ++s) {
-    const int R=p.radix[s], at=i-(nblk-R0);
-    if(at < 0) break;
-    if(at < (R-1)*nblk) {
-      const int r=at/nblk+1, b=at-(r-1)*nblk;
-      // natural index of block b's digits
-      int k=0, mul=1, w=nblk, q=b;
-      for(int z=0; z < s; ++z) {
-        w /= p.radix[z];
-        const int d=q/w;
-        q -= d*w;
-        k += d*mul;
-        mul *= p.radix[z];
-      }
-      double sn, cn;
-      sincospi(2.0*(double) (r*k)/(double) (nblk*R),&sn,&cn);
-      twb[i]=make_double2(cn,sn);
-      break;
-    }
-    nblk *= R;
-  }
-  int m=1;
-  for(int s=p.nst-1; s >= 0; --s) {
-    const int R=p.radix[s], at=i-(m-1);
-    if(at < 0) break;
-    if(at < (R-1)*m) {
-      const int r=at/m+1, j=at-(r-1)*m;
-      double sn, cn;
-      sincospi(2.0*(double) (r*j)/(double) (R*m),&sn,&cn);
-      twj[i]=make_double2(cn,sn);
-      break;
-    }
-    m *= R;
-  }
 }
 
 long evenSmoothLen(long M)
@@ -155,11 +109,6 @@ int fail(const std::string& what)
 
 } // namespace
 
-namespace fgb {
-FusedFFT fusedRowPlan(long n, int prec, int A, bool herm, bool half,
-                      int nteam, int maxR);   // engine.cu
-}
-
 extern "C" int fgb_hconv2d_convolve_noalloc(const void *f, const void *g,
                                             void *h, size_t Lx, size_t Ly,
                                             void *stream)
@@ -177,20 +126,19 @@ extern "C" int fgb_hconv2d_convolve_noalloc(const void *f, const void *g,
   const long Ny=evenSmoothLen(std::max<long>(My,(long) Ly));
   const long Nyh=Ny/2;
 
-  // Scratch layout: 2 staging arrays [Nx][Hy], then W_Nx (x transform) and
-  // three tables of Ny/2 entries for the rows: W_Ny up to Ny/2 (Hermitian
-  // packing), the row transform's block and input twiddles.
+  // Scratch layout: 2 staging arrays [Nx][Hy], then the three tables
+  // W_Nx (x transform), W_Ny (Hermitian packing), W_{Ny/2} (row FFT).
   const size_t stageBytes=sizeof(Cx)*(size_t) Nx*(size_t) Hy;
   const size_t twx=align256(2*stageBytes);
   const size_t twy=twx+align256(sizeof(double2)*(size_t) Nx);
-  const size_t need=twy+align256(sizeof(double2)*(size_t) Ny)+
-    align256(sizeof(double2)*(size_t) Nyh);
+  const size_t twyh=twy+align256(sizeof(double2)*(size_t) Ny);
+  const size_t need=twyh+align256(sizeof(double2)*(size_t) Nyh);
   if(need > FGB_NOALLOC_SCRATCH_BYTES)
     return fail("Lx="+std::to_string(Lx)+", Ly="+std::to_string(Ly)+
                 " needs "+std::to_string(need)+" scratch bytes; the maximum "
                 "is "+std::to_string(FGB_NOALLOC_SCRATCH_BYTES));
   const size_t smx=outerBwdSmem<double>((int) Lx,(int) Nx,1);
-  if(smx > 227*1024 || 2*sizeof(Cx)*(size_t) padded((int) (2*Nyh)) > 227*1024)
+  if(smx > 227*1024 || hermRowSmem<double>((int) Nyh,2,1) > 227*1024)
     return fail("rows too long for shared memory");
 
   void *base=NULL;
@@ -202,14 +150,11 @@ extern "C" int fgb_hconv2d_convolve_noalloc(const void *f, const void *g,
   Cx *stage1=(Cx *) (sc+stageBytes);
   double2 *tx=(double2 *) (sc+twx);
   double2 *ty=(double2 *) (sc+twy);
-  double2 *tyb=ty+Nyh, *tyj=tyb+Nyh;
-  FusedFFT fz=fusedRowPlan(Nyh,PREC_F64,2,true,false,1,8);
-  fz.twb=tyb;
-  fz.twj=tyj;
+  double2 *tyh=(double2 *) (sc+twyh);
 
-  fillTwiddles<<<(unsigned) ((Nx+255)/256),256,0,s>>>(tx,(int) Nx,(int) Nx);
-  fillTwiddles<<<(unsigned) ((Nyh+255)/256),256,0,s>>>(ty,(int) Ny,(int) Nyh);
-  fillFused<<<(unsigned) ((Nyh+255)/256),256,0,s>>>(tyb,tyj,fz);
+  fillTwiddles<<<(unsigned) ((Nx+255)/256),256,0,s>>>(tx,(int) Nx);
+  fillTwiddles<<<(unsigned) ((Ny+255)/256),256,0,s>>>(ty,(int) Ny);
+  fillTwiddles<<<(unsigned) ((Nyh+255)/256),256,0,s>>>(tyh,(int) Nyh);
   e=cudaGetLastError();
   if(e != cudaSuccess) return fail(cudaGetErrorString(e));
 
@@ -241,8 +186,9 @@ extern "C" int fgb_hconv2d_convolve_noalloc(const void *f, const void *g,
   HermRowPlan<double> P{};
   P.io64=0;
   P.H=(int) Hy; P.N=(int) Ny; P.Nh=(int) Nyh;
-  P.A=2; P.B=1; P.mult=MULT_REALBINARY; P.rpc=1; P.nteam=1;
-  P.fz=fz;
+  P.A=2; P.B=1; P.mult=MULT_REALBINARY; P.rpc=1;
+  P.pingpong=1;
+  P.fp=radixPlan(Nyh,tyh);
   P.twN=ty;
   P.in[0]=stage0; P.in[1]=stage1; P.out[0]=stage0;
   P.rowStride=Hy; P.nrows=Nx; P.scale=1.0;

@@ -1255,6 +1255,91 @@ __device__ __forceinline__ void hermRowStaged(const HermRowPlan<T>& P,
   }
 }
 
+// One slot t of a Hermitian row (real grid points 2t and 2t+1) in shared
+// memory: the A values at X[sp(base+a*stride)] in, the B results back.
+template<class Mul, typename T>
+__device__ __forceinline__ void mulHermSlot(const Mul& mul,
+                                            const HermRowPlan<T>& P,
+                                            cplx<T> *X, int base, int stride,
+                                            long long row, int t)
+{
+  if constexpr(Mul::positional) {
+    constexpr int A=MulArity<Mul>::A, B=MulArity<Mul>::B;
+    cplx<T> v[A];
+#pragma unroll
+    for(int a=0; a < A; ++a) v[a]=nrm(X[sp(base+a*stride)]);
+    mul.slotReal(v,outerIndices(P.im,row),2*t);
+#pragma unroll
+    for(int b=0; b < B; ++b) X[sp(base+b*stride)]=v[b];
+  } else mul(X,base,stride,P.A,P.B,P.mult);
+}
+
+// FP64 rows through the self-sorting transform (hermPingPong in engine.cu):
+// the P.rpc rows of a group as interleaved columns col = a rpc + rho of two
+// buffers, all threads on all of them, natural order throughout.  Every read
+// of a group precedes its writes, so in = out is safe.
+template<typename T, class Mul>
+__global__ void __launch_bounds__(256)
+hermRowPingPongKernel(const HermRowPlan<T> P, const Mul mul)
+{
+  extern __shared__ __align__(16) unsigned char smemRaw[];
+  const int H=P.H, Nh=P.Nh, R=P.rpc, ld=P.A*R, lb=P.B*R;
+  cplx<T> *x=(cplx<T> *) smemRaw, *y=x+padded(Nh*ld);
+  const int tid=threadIdx.x, nthr=blockDim.x;
+  const UDiv dH(H), dLd(ld), dR(R);
+  const int np=Nh/2+1;                 // k = 0 .. floor(Nh/2)
+  const long long groups=(P.nrows+R-1)/R;
+  for(long long g=blockIdx.x; g < groups; g += gridDim.x) {
+    const long long row0=g*R;
+    for(int i0=tid; i0 < np*ld; i0 += FGB_LOADS*nthr) {
+      cplx<T> zk[FGB_LOADS], zc[FGB_LOADS];
+#pragma unroll
+      for(int u=0; u < FGB_LOADS; ++u) {
+        const int i=i0+u*nthr, k=dLd(i), col=i-k*ld, a=dR(col), kk=Nh-k;
+        const long long row=row0+col-a*R;
+        const bool live=i < np*ld && row < P.nrows;
+        zk[u]=zc[u]=mk((T) 0,(T) 0);
+        if(live && k < H) zk[u]=P.in[a][row*P.rowStride+k];
+        if(live && kk < H) zc[u]=P.in[a][row*P.rowStride+kk];
+      }
+#pragma unroll
+      for(int u=0; u < FGB_LOADS; ++u) {
+        const int i=i0+u*nthr;
+        if(i >= np*ld) break;
+        const int k=dLd(i), col=i-k*ld;
+        cplx<T> Y, Yc;
+        if(k == 0) zk[u].y=(T) 0;
+        hermPack(zk[u],zc[u],ldtw(P.twN+k),Y,Yc);
+        x[sp(i)]=Y;
+        if(k != 0 && 2*k != Nh) x[sp((Nh-k)*ld+col)]=Yc;
+      }
+    }
+    __syncthreads();
+    cplx<T> *X=fftSmem<T,1>(x,y,P.fp,ld,ld,tid,nthr);
+    cplx<T> *Y=X == x ? y : x;
+    for(int i=tid; i < Nh*R; i += nthr) {
+      const int t=dR(i), rho=i-t*R;
+      mulHermSlot(mul,P,X,t*ld+rho,R,row0+rho,t);
+    }
+    __syncthreads();
+    const cplx<T> *Z=fftSmem<T,-1>(X,Y,P.fp,lb,ld,tid,nthr);
+    // When both k and Nh-k are stored modes the lower one writes both.
+    const T hs=(T) 0.5*P.scale;
+    for(int i=tid; i < lb*H; i += nthr) {
+      const int col=dH(i), k=i-col*H, b=dR(col), kk=k == 0 ? 0 : Nh-k;
+      const long long row=row0+col-b*R;
+      const bool pair=k != 0 && kk < H && kk != k;
+      if(row >= P.nrows || (pair && kk < k)) continue;
+      cplx<T> V, Vc;
+      hermUnpack(Z[sp(k*ld+col)],Z[sp(kk*ld+col)],hs,ldtw(P.twN+k),V,Vc);
+      cplx<T> *o=P.out[b]+row*P.rowStride;
+      o[k]=V;
+      if(pair) o[kk]=Vc;
+    }
+    __syncthreads();
+  }
+}
+
 // First radices of fused Hermitian rows (the two butterflies of a pair are
 // in registers together).
 #define FGB_HERM_SWITCH(R,CALL) \
@@ -1280,13 +1365,14 @@ __device__ __forceinline__ void hermRows(const HermRowPlan<T>& P,
   const int cs=fusedSpan(P.Nh,P.fz.lg);
   cplx<T> *x=(cplx<T> *) smemRaw+team*P.A*cs;
   const int R0=P.fz.radix[0];
-  const bool staged=std::is_same<T,ff>::value || P.A*((P.Nh/R0+1)/2) < nt;
+  const bool staged=!std::is_same<T,float>::value ||
+    P.A*((P.Nh/R0+1)/2) < nt;
   const long long groups=(P.nrows+P.rpc-1)/P.rpc;
   for(long long g=blockIdx.x; g < groups; g += gridDim.x)
     for(int rho=team; rho < P.rpc; rho += P.nteam) {
       const long long row=g*P.rpc+rho;
       if(staged) hermRowStaged<T,WIDE>(P,mul,x,cs,row,team,t,nt);
-      else if constexpr(!std::is_same<T,ff>::value) {
+      else if constexpr(std::is_same<T,float>::value) {
         FGB_HERM_SWITCH(R0,(hermFirst<T,R_>(P,x,cs,row,t,nt)))
         fusedRowInner<T,WIDE>(P,mul,x,cs,row,team,t,nt);
         FGB_HERM_SWITCH(R0,(hermLast<T,R_>(P,x,cs,row,t,nt)))
@@ -1356,7 +1442,8 @@ template<typename T, class Mul>
 cudaError_t launchHermRowWith(const HermRowPlan<T>& P, const Mul& mul,
                               int threads, long long grid, cudaStream_t s)
 {
-  const size_t sm=fusedRowSmem<T>(P.fz.n,P.fz.lg,P.A,P.nteam);
+  const size_t sm=P.pingpong ? hermRowSmem<T>(P.Nh,P.A,P.rpc) :
+    fusedRowSmem<T>(P.fz.n,P.fz.lg,P.A,P.nteam);
   const long long groups=(P.nrows+P.rpc-1)/P.rpc;
   grid=std::min(std::min(grid,groups),(long long) INT_MAX);
   if(grid < 1) return cudaSuccess;
@@ -1368,6 +1455,8 @@ cudaError_t launchHermRowWith(const HermRowPlan<T>& P, const Mul& mul,
   };
   if constexpr(std::is_same<T,float>::value)
     if(wideFused(P.fz)) return go(hermRowKernel16<T,Mul>);
+  if constexpr(std::is_same<T,double>::value)
+    if(P.pingpong) return go(hermRowPingPongKernel<T,Mul>);
   return go(hermRowKernel<T,Mul>);
 }
 
