@@ -464,8 +464,7 @@ __device__ __forceinline__ int runFusedMiddle(cplx<T> *x, int cs, int ncol,
 //
 // FP64 takes it for real outer axes and for those Hermitian rows that do not
 // take the ping-pong transform (stagedReal and hermPingPong in engine.cu), FP32
-// for small real outer launches, and both for rows whose fused first stage
-// would leave threads of the team without a butterfly.
+// for small real outer launches, and complex rows as fusedRow says.
 //
 // The forward stages from `first` on for A columns at x (cs apart, each of
 // 2^lt interleaved ones), mid(), the inverse stages down to `first` for B

@@ -876,7 +876,16 @@ __device__ __forceinline__ void fusedRow(const RowPlan<T>& P, const Mul& mul,
       else storeIO(f+s,v*P.scale,P.io64 & 2,sh);
     };
   };
-  if(P.A*(m/P.fz.radix[0]) < nt) {
+  // The staged form where the fused first stage would leave threads of the
+  // team without a butterfly, and for FP64 rows of up to 128 points (512 rows
+  // of 80 points 26 us fused, 19 staged; 6000 of 128 104 / 100; 512 of 160 25.9
+  // / 26.1, 1536 of 192 60 / 65).  FP32 rows are faster fused throughout (441
+  // of 80 points 9 us, 12 staged; 1536 of 360 13 / 19), but for the batched
+  // launch, whose short problems have a whole CTA for one row.
+  bool staged=P.A*(m/P.fz.radix[0]) < nt;
+  if constexpr(std::is_same<T,double>::value) staged=staged || m <= 128;
+  if constexpr(std::is_same<T,float>::value && !CG) staged=false;
+  if(staged) {
     const ColumnMap cols(m);             // the staged form (runStages)
 #pragma unroll 2
     for(int i=t; i < P.A*m; i += nt) {
@@ -1215,7 +1224,7 @@ __device__ __forceinline__ void hermLast(const HermRowPlan<T>& P,
 
 // The staged form (runStages) of a Hermitian row: the packing and unpacking
 // one pair at a time.
-template<typename T, bool WIDE, class Mul>
+template<typename T, class Mul>
 __device__ __forceinline__ void hermRowStaged(const HermRowPlan<T>& P,
                                               const Mul& mul, cplx<T> *x,
                                               int cs, long long row, int team,
@@ -1237,7 +1246,7 @@ __device__ __forceinline__ void hermRowStaged(const HermRowPlan<T>& P,
     x[c*cs+spl(k,p.lg)]=Y;
     if(k != 0 && 2*k != Nh) x[c*cs+spl(kk,p.lg)]=Yc;
   }
-  runStages<T,WIDE>(x,cs,P.A,P.B,p,0,0,team,t,nt,[&] {
+  runStages<T>(x,cs,P.A,P.B,p,0,0,team,t,nt,[&] {
       fusedMulSlots(P,mul,x,cs,row,t,nt);
     });
   const T hs=(T) 0.5*P.scale;
@@ -1365,14 +1374,13 @@ __device__ __forceinline__ void hermRows(const HermRowPlan<T>& P,
   const int cs=fusedSpan(P.Nh,P.fz.lg);
   cplx<T> *x=(cplx<T> *) smemRaw+team*P.A*cs;
   const int R0=P.fz.radix[0];
-  const bool staged=!std::is_same<T,float>::value ||
-    P.A*((P.Nh/R0+1)/2) < nt;
   const long long groups=(P.nrows+P.rpc-1)/P.rpc;
   for(long long g=blockIdx.x; g < groups; g += gridDim.x)
     for(int rho=team; rho < P.rpc; rho += P.nteam) {
       const long long row=g*P.rpc+rho;
-      if(staged) hermRowStaged<T,WIDE>(P,mul,x,cs,row,team,t,nt);
-      else if constexpr(std::is_same<T,float>::value) {
+      if constexpr(!std::is_same<T,float>::value)
+        hermRowStaged<T>(P,mul,x,cs,row,team,t,nt);
+      else {
         FGB_HERM_SWITCH(R0,(hermFirst<T,R_>(P,x,cs,row,t,nt)))
         fusedRowInner<T,WIDE>(P,mul,x,cs,row,team,t,nt);
         FGB_HERM_SWITCH(R0,(hermLast<T,R_>(P,x,cs,row,t,nt)))
