@@ -584,6 +584,13 @@ static bool hermPingPong(int prec, long Nh, int A)
   return prec == PREC_F64 && !(A >= 4 && Nh >= 384);
 }
 
+// Whether FP32 Hermitian rows, `points` of all inputs, take the staged form:
+// small launches, as the outer kernels' (stagedColumns).  2D convolutions back
+// to back, us fused / staged: 81 x 35 modes (7000 points) 22.7 / 20.7, 143 x 81
+// (27216) 23.3 / 21.4, 95 x 433 (96768) 26.8 / 24.8, 255 x 255 (147456) 26.8 /
+// 26.8, 131 x 829 (250880) 29.8 / 32.9, 255 x 1023 (589824) 31.9 / 36.0.
+static bool stagedHerm(long long points) {return points < (1 << 17);}
+
 // Shared memory of the innermost axis' row kernel, as planned.
 static size_t innerNeed(const ConvInfo& I, const AxisPlan& a, int rpc,
                         int threads)
@@ -644,25 +651,32 @@ static size_t outerBwdNeed(const AxisPlan& a, int prec, int tile)
   return FGB_BY_PREC(prec,outerBwdSmem,a.L,a.m,tile,(int) a.q);
 }
 
-// Whether the fused outer kernels of an axis take the staged form: float-float
-// with few columns, where fetching the fused form's code dominates; with many,
-// its fewer passes through shared memory and the halves it leaves out count.
-// Forward kernels of ten axes (80 to 1568 points, centred and half empty),
-// fused over staged time, geometric mean: 512 columns 1.10, 1024 1.05, 1536
-// 1.03, 2048 0.99, 3072 0.99, 6144 0.97 (18 us fused against 16 staged for 80
-// points of 1024 columns, 92 against 104 for 1536 points of 2048).
+// Whether the fused outer kernels of an axis of length N take the staged form:
+// small float-float and FP32 launches, where fetching the fused form's code
+// dominates; in large ones its fewer passes through shared memory and the
+// halves it leaves out count.
+// Float-float, forward kernels of ten axes (80 to 1568 points, centred and
+// half empty), fused over staged time, geometric mean: 512 columns 1.10, 1024
+// 1.05, 1536 1.03, 2048 0.99, 3072 0.99, 6144 0.97 (18 us fused against 16
+// staged for 80 points of 1024 columns, 92 against 104 for 1536 points of
+// 2048).
+// FP32, 2D convolutions back to back, us fused / staged: 63 x 63 modes (6144
+// points a launch) 22.6 / 20.6, 127 x 127 (24576) 26.2 / 24.4, 584 x 97 (228144)
+// 32.1 / 29.2, 131 x 829 (162680) 29.2 / 29.8, 511 x 511 (393216) 31.2 / 32.6.
+// FP64 gains 2 us at 121 x 123 and loses 3 at 255 x 255; it stays fused.
 // columns: of all the launch's inputs or outputs and batches, also where a
 // host call makes the launch in column ranges, so that every way gives the
 // same bits.
-static bool stagedColumns(int prec, long long columns)
+static bool stagedColumns(int prec, long long N, long long columns)
 {
-  return prec == PREC_FF && columns < 2048;
+  return prec == PREC_FF ? columns < 2048 :
+    prec == PREC_F32 && N*columns < (1 << 18);
 }
 
 static bool stagedOuter(int prec, const AxisPlan& a, long long columns)
 {
   return a.kind == KIND_REAL ? stagedReal(prec,a.N,columns) :
-    stagedColumns(prec,columns);
+    stagedColumns(prec,a.m,columns);
 }
 
 // The transform of a split row's CTAs.
@@ -785,8 +799,12 @@ static double rowCost(const AxisPlan& a, long m, long q, int A, int B,
   if(q == 1 && a.L <= m)
     return fusedCost(m,prec,A,B,false,a.kind != KIND_CENTERED && 2*a.L <= m);
   // The fused rows run an instruction's worth in 0.55 (FP32) to 0.9 of the
-  // time (4096 rows of 1024: FP32 175 -> 83 us, FP64 1728 -> 1425).
-  const double slower=prec == PREC_F32 ? 1.8 : 1.1;
+  // time (4096 rows of 1024: FP32 175 -> 83 us, FP64 1728 -> 1425).  In FP64
+  // a little more, which decides near ties: 80 points as two residues of 40
+  // are 0.8 % cheaper at 1.1, but a 25 x 40 convolution of them takes 47 us
+  // against 37 with one (the timed search still takes two where many rows make
+  // them faster).
+  const double slower=prec == PREC_F32 ? 1.8 : 1.15;
   return slower*(stagedRowCost(a,m,q,A,B)+2.0*(A+B)*(double) (q*m));
 }
 
@@ -1828,7 +1846,7 @@ cudaError_t Conv::runT(const void *const *in, void *const *out, cudaStream_t s)
     } else P.fp=fftPlan(a.m,I.prec,inplaceFFT<T>(),true);
     P.twN=(const typename TwT<T>::type *) twiddles(a.N,I.prec);
   };
-  auto hermPlan=[&](HermRowPlan<T>& P, const AxisPlan& a) {
+  auto hermPlan=[&](HermRowPlan<T>& P, const AxisPlan& a, long nrows) {
     P.im=im;
     P.ioShift=guard;
     P.H=(int) a.stored; P.N=(int) a.N; P.Nh=(int) (a.N/2);
@@ -1837,6 +1855,7 @@ cudaError_t Conv::runT(const void *const *in, void *const *out, cudaStream_t s)
     P.nteam=rowTeams(P.rpc,a.thr);
     P.io64=0;
     P.pingpong=hermPingPong(I.prec,a.N/2,A);
+    P.staged=stagedHerm(a.N/2*A*nrows);
     if(P.pingpong) P.fp=fftPlan(a.N/2,I.prec);
     else {
       P.fz=fusedRowPlan(a.N/2,I.prec,A,true,false,P.nteam,
@@ -1938,7 +1957,7 @@ cudaError_t Conv::runT(const void *const *in, void *const *out, cudaStream_t s)
     const AxisPlan& a=I.axis[0];
     if(a.kind == KIND_HERMITIAN) {
       HermRowPlan<T> P{};
-      hermPlan(P,a);
+      hermPlan(P,a,batch);
       for(int i=0; i < A; ++i) P.in[i]=(const Cx *) in[i];
       for(int i=0; i < B; ++i) P.out[i]=(Cx *) out[i];
       P.rowStride=a.stored; P.nrows=batch; P.scale=(T) scale;
@@ -1986,7 +2005,7 @@ cudaError_t Conv::runT(const void *const *in, void *const *out, cudaStream_t s)
                    NULL,&im,1.0,s);
     } else if(ay.kind == KIND_HERMITIAN) {
       HermRowPlan<T> P{};
-      hermPlan(P,ay);
+      hermPlan(P,ay,ax.rows);
       for(int i=0; i < A; ++i) P.in[i]=(const Cx *) bufs[i];
       for(int i=0; i < B; ++i) P.out[i]=(Cx *) bufs[i];
       P.rowStride=C; P.nrows=ax.rows; P.scale=(T) 1;
@@ -2058,7 +2077,7 @@ cudaError_t Conv::runT(const void *const *in, void *const *out, cudaStream_t s)
     e=runLong<T>((const void *const *) by,by,nrows,nz,0,NULL,&im,1.0,s);
   } else if(az.kind == KIND_HERMITIAN) {
     HermRowPlan<T> P{};
-    hermPlan(P,az);
+    hermPlan(P,az,nrows);
     for(int i=0; i < A; ++i) P.in[i]=(const Cx *) by[i];
     for(int i=0; i < B; ++i) P.out[i]=(Cx *) by[i];
     P.rowStride=nz; P.nrows=nrows; P.scale=(T) 1;

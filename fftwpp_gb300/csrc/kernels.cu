@@ -378,7 +378,8 @@ __device__ __forceinline__ int columnTop(const OuterPlan<T>& P, int col,
   return ((int) P.Ltot-col+(int) row-1)/(int) row;
 }
 
-template<typename T, bool WIDE>
+// STAGED: whether the kernel holds the staged form (OuterPlan::staged).
+template<typename T, bool WIDE, bool STAGED>
 __device__ __forceinline__ void outerFwdFused(const OuterPlan<T>& P, int ctile,
                                               int r, int z,
                                               unsigned char *smemRaw)
@@ -407,7 +408,7 @@ __device__ __forceinline__ void outerFwdFused(const OuterPlan<T>& P, int ctile,
       return v;
     };
   };
-  if(std::is_same<T,ff>::value && P.staged) {
+  if(STAGED && P.staged) {
     loadTile(x,P.fz,lt,tid,nthr,[&](int cc, int j) {
         int s=j+c;
         if(s >= m) s -= m;
@@ -419,7 +420,7 @@ __device__ __forceinline__ void outerFwdFused(const OuterPlan<T>& P, int ctile,
         }
         return v;
       });
-    runStages<T>(x,0,1,0,P.fz,lt,0,0,tid,nthr,[] {});
+    runStages<T,WIDE>(x,0,1,0,P.fz,lt,0,0,tid,nthr,[] {});
 #pragma unroll 4
     for(int idx=tid; idx < m << lt; idx += nthr) {
       const int j=idx >> lt, cc=idx & (tile-1);
@@ -435,12 +436,20 @@ __device__ __forceinline__ void outerFwdFused(const OuterPlan<T>& P, int ctile,
                    (outerLastFwd<T,R_>(P,x,dst,col0,nblk,tid,nthr)))
 }
 
+// Precisions whose outer launches may take the staged form (stagedColumns in
+// engine.cu).
+template<typename T> __host__ __device__ constexpr bool stagedOuterForm()
+{
+  return !std::is_same<T,double>::value;
+}
+
 template<typename T>
 __global__ void __launch_bounds__(256)
 outerFwdFusedKernel(const OuterPlan<T> P)
 {
   extern __shared__ __align__(16) unsigned char smemRaw[];
-  outerFwdFused<T,false>(P,blockIdx.x,blockIdx.y,blockIdx.z,smemRaw);
+  outerFwdFused<T,false,stagedOuterForm<T>()>(P,blockIdx.x,blockIdx.y,
+                                              blockIdx.z,smemRaw);
 }
 
 // The first inverse stage: staging rows into shared memory.
@@ -476,7 +485,7 @@ __device__ __forceinline__ void outerFirstInv(const OuterPlan<T>& P,
 
 // All residues of a column tile; with several, a thread adds the outputs it
 // computes into its own entries of an accumulator behind the tile.
-template<typename T, bool WIDE, bool CG>
+template<typename T, bool WIDE, bool CG, bool STAGED>
 __device__ __forceinline__ void outerBwdFused(const OuterPlan<T>& P, int ctile,
                                               int z, unsigned char *smemRaw)
 {
@@ -511,12 +520,12 @@ __device__ __forceinline__ void outerBwdFused(const OuterPlan<T>& P, int ctile,
         storeIO(f+s*P.outRow,v*P.scale,P.io64 & 2,sh);
       };
     };
-    if(std::is_same<T,ff>::value && P.staged) {
+    if(STAGED && P.staged) {
       loadTile(x,P.fz,lt,tid,nthr,[&](int cc, int j) {
           return col0+cc < P.C ? swapXY(sr[j*P.inRow+col0+cc]) :
             mk((T) 0,(T) 0);
         });
-      runStages<T>(x,0,0,1,P.fz,lt,0,0,tid,nthr,[] {});
+      runStages<T,WIDE>(x,0,0,1,P.fz,lt,0,0,tid,nthr,[] {});
       storeTile(x,P.fz,lt,tid,nthr,store);
     } else {
       FGB_FUSED_SWITCH(P.fz.radix[P.fz.nst-1],
@@ -534,7 +543,8 @@ __global__ void __launch_bounds__(256)
 outerBwdFusedKernel(const OuterPlan<T> P)
 {
   extern __shared__ __align__(16) unsigned char smemRaw[];
-  outerBwdFused<T,false,false>(P,blockIdx.x,blockIdx.z,smemRaw);
+  outerBwdFused<T,false,false,stagedOuterForm<T>()>(P,blockIdx.x,blockIdx.z,
+                                                    smemRaw);
 }
 
 // FP32 plans with a radix-16 stage: their own instantiations, capped at 85
@@ -545,7 +555,7 @@ __global__ void __launch_bounds__(256,3)
 outerFwdFusedKernel16(const OuterPlan<T> P)
 {
   extern __shared__ __align__(16) unsigned char smemRaw[];
-  outerFwdFused<T,true>(P,blockIdx.x,blockIdx.y,blockIdx.z,smemRaw);
+  outerFwdFused<T,true,true>(P,blockIdx.x,blockIdx.y,blockIdx.z,smemRaw);
 }
 
 template<typename T>
@@ -553,7 +563,7 @@ __global__ void __launch_bounds__(256,3)
 outerBwdFusedKernel16(const OuterPlan<T> P)
 {
   extern __shared__ __align__(16) unsigned char smemRaw[];
-  outerBwdFused<T,true,false>(P,blockIdx.x,blockIdx.z,smemRaw);
+  outerBwdFused<T,true,false,true>(P,blockIdx.x,blockIdx.z,smemRaw);
 }
 
 // ---------------------------------------------------------------------------
@@ -961,8 +971,8 @@ batchKernel(const BatchArgs<T> P)
         rebase(O,O.count,fwd && (rel & 4),!fwd && (rel & 8),P.inBase,
                P.outBase);
       __syncthreads();
-      if(fwd) outerFwdFused<T,false>(O,tk.i,0,tk.j,smemRaw);
-      else outerBwdFused<T,false,true>(O,tk.i,tk.j,smemRaw);
+      if(fwd) outerFwdFused<T,false,false>(O,tk.i,0,tk.j,smemRaw);
+      else outerBwdFused<T,false,true,false>(O,tk.i,tk.j,smemRaw);
       __syncthreads();
     }
     if(tk.type == TASK_COLFWD || tk.type == TASK_ROW) {

@@ -115,6 +115,7 @@ struct HermRowPlan {
   int io64;                // as RowPlan::io64
   const int *ioShift;      // as RowPlan::ioShift
   int pingpong;            // FP64: hermRowPingPongKernel, transformed by fp
+  int staged;              // FP32: the staged form (runStages)
   T scale;
   FusedFFT fz;             // length-Nh complex FFT
   FFTPlanDev fp;           // the same for the ping-pong kernel
@@ -143,8 +144,8 @@ struct OuterPlan {
                            // residue block in fz's digit-reversed order
                            // (the long-row path's twX launches do not take
                            // them, the batched launch's do)
-  int staged;              // the staged form (runStages): fused float-float,
-                           // or real FP32, launches
+  int staged;              // the staged form (runStages): fused float-float
+                           // and FP32 launches, real FP32 ones
   int conj;                // real kernels: conjugate the complex side
                            // (the sign -1 r2c / sign +1 c2r of plain FFTs)
   int cz;                  // data side with strides: column c lies at

@@ -1224,7 +1224,7 @@ __device__ __forceinline__ void hermLast(const HermRowPlan<T>& P,
 
 // The staged form (runStages) of a Hermitian row: the packing and unpacking
 // one pair at a time.
-template<typename T, class Mul>
+template<typename T, bool WIDE, class Mul>
 __device__ __forceinline__ void hermRowStaged(const HermRowPlan<T>& P,
                                               const Mul& mul, cplx<T> *x,
                                               int cs, long long row, int team,
@@ -1246,7 +1246,7 @@ __device__ __forceinline__ void hermRowStaged(const HermRowPlan<T>& P,
     x[c*cs+spl(k,p.lg)]=Y;
     if(k != 0 && 2*k != Nh) x[c*cs+spl(kk,p.lg)]=Yc;
   }
-  runStages<T>(x,cs,P.A,P.B,p,0,0,team,t,nt,[&] {
+  runStages<T,WIDE>(x,cs,P.A,P.B,p,0,0,team,t,nt,[&] {
       fusedMulSlots(P,mul,x,cs,row,t,nt);
     });
   const T hs=(T) 0.5*P.scale;
@@ -1378,9 +1378,9 @@ __device__ __forceinline__ void hermRows(const HermRowPlan<T>& P,
   for(long long g=blockIdx.x; g < groups; g += gridDim.x)
     for(int rho=team; rho < P.rpc; rho += P.nteam) {
       const long long row=g*P.rpc+rho;
-      if constexpr(!std::is_same<T,float>::value)
-        hermRowStaged<T>(P,mul,x,cs,row,team,t,nt);
-      else {
+      if(!std::is_same<T,float>::value || P.staged)
+        hermRowStaged<T,WIDE>(P,mul,x,cs,row,team,t,nt);
+      else if constexpr(std::is_same<T,float>::value) {
         FGB_HERM_SWITCH(R0,(hermFirst<T,R_>(P,x,cs,row,t,nt)))
         fusedRowInner<T,WIDE>(P,mul,x,cs,row,team,t,nt);
         FGB_HERM_SWITCH(R0,(hermLast<T,R_>(P,x,cs,row,t,nt)))

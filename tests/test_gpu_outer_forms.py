@@ -65,3 +65,31 @@ def test_real_ffts(native_lib, n, M, precision):
     B = fft.mcrfft1d(n, M, precision=precision)
     y = B.fft(X.reshape(B.in_shape)).double().reshape(M, n) / n
     assert rel_l2(y.cpu().numpy(), x.cpu().numpy()) <= TOL[precision]
+
+
+@pytest.mark.parametrize("precision", ["f64", "ff", "f32"])
+@pytest.mark.parametrize("kinds,L", [
+    ([H.CENTERED, H.CENTERED], (170, 511)), ([H.CENTERED, H.CENTERED],
+                                             (171, 513)),
+    ([H.PAD, H.PAD], (128, 511)), ([H.PAD, H.PAD], (128, 512)),
+    ([H.PAD, H.PAD], (128, 513)), ([H.PAD, H.PAD, H.PAD], (9, 21, 48)),
+    ([H.PAD, H.PAD], (25, 40)), ([H.CENTERED, H.PAD], (7, 3))])
+def test_complex_convolution(native_lib, kinds, L, precision):
+    """Complex outer axes around the lines between the forms of their FP32
+    (2^18 points a launch) and float-float (2048 columns) kernels."""
+    import torch
+    from fftwpp_gb300.gpu import HybridConvolution
+    conv = HybridConvolution(kinds, L, precision=precision)
+    g = torch.Generator(device="cuda").manual_seed(sum(L))
+    f = [torch.randn(L, generator=g, device="cuda", dtype=torch.complex128)
+         for _ in range(2)]
+    got = conv.convolve(*[t.to(conv.dtype) for t in f])[0]
+    s = [2 * n for n in L]
+    F = [torch.fft.fftn(t, s) for t in f]
+    full = torch.fft.ifftn(F[0] * F[1])
+    # Centred axes: index i stands for i - L//2, so the product starts at
+    # L//2 of the full linear convolution.
+    cut = tuple(slice(n // 2, n // 2 + n) if k == H.CENTERED else slice(n)
+                for k, n in zip(kinds, L))
+    assert rel_l2(got.cpu().numpy().astype(np.complex128),
+                  full[cut].cpu().numpy()) <= TOL[precision]
