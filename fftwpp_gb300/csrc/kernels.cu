@@ -297,6 +297,12 @@ outerBwdKernel(const OuterPlan<T> P)
 // row order and the backward undoes it).  The column tile's values cross
 // shared memory once between stages and never before the first or after
 // the last.
+// CTAs of 256 threads per SM of the staged kernels (radix 16 in FP32).
+template<typename T> __host__ __device__ constexpr int stagedBlocks()
+{
+  return std::is_same<T,float>::value ? 3 : 1;
+}
+
 // The staged form (runStages): the tile's inputs into shared memory, and its
 // outputs out of it.  in(cc, j) gives element j of column cc.
 template<typename T, class In>
@@ -378,8 +384,8 @@ __device__ __forceinline__ int columnTop(const OuterPlan<T>& P, int col,
   return ((int) P.Ltot-col+(int) row-1)/(int) row;
 }
 
-// STAGED: whether the kernel holds the staged form (OuterPlan::staged).
-template<typename T, bool WIDE, bool STAGED>
+// STAGED: the staged form (OuterPlan::staged), in kernels of its own.
+template<typename T, bool WIDE, bool STAGED=false>
 __device__ __forceinline__ void outerFwdFused(const OuterPlan<T>& P, int ctile,
                                               int r, int z,
                                               unsigned char *smemRaw)
@@ -394,21 +400,7 @@ __device__ __forceinline__ void outerFwdFused(const OuterPlan<T>& P, int ctile,
   cplx<T> *dst=P.out[a]+batch*P.outBatch+(long long) r*m*P.outRow;
   const int lt=log2of(tile);
   const int sh=ioShift<T>(P.ioShift,a);
-  const auto load=[&](int, int cc) {
-    const int top=columnTop(P,col0+cc,P.inRow);
-    const cplx<T> *f=src+dataCol(P,col0+cc);
-    return [=,&P](int j) {
-      int s=j+c;
-      if(s >= m) s -= m;
-      cplx<T> v=mk((T) 0,(T) 0);
-      if(s < top) {
-        v=loadIO(f+s*P.inRow,P.io64 & 1,sh);
-        if(r != 0) v=twmul<1>(v,P.twN[twExp(s,c,r,N)]);
-      }
-      return v;
-    };
-  };
-  if(STAGED && P.staged) {
+  if constexpr(STAGED) {
     loadTile(x,P.fz,lt,tid,nthr,[&](int cc, int j) {
         int s=j+c;
         if(s >= m) s -= m;
@@ -427,20 +419,27 @@ __device__ __forceinline__ void outerFwdFused(const OuterPlan<T>& P, int ctile,
       if(col0+cc < P.C)
         dst[j*P.outRow+col0+cc]=x[(spl(j,P.fz.lg) << lt)+cc];
     }
-    return;
+  } else {
+    const auto load=[&](int, int cc) {
+      const int top=columnTop(P,col0+cc,P.inRow);
+      const cplx<T> *f=src+dataCol(P,col0+cc);
+      return [=,&P](int j) {
+        int s=j+c;
+        if(s >= m) s -= m;
+        cplx<T> v=mk((T) 0,(T) 0);
+        if(s < top) {
+          v=loadIO(f+s*P.inRow,P.io64 & 1,sh);
+          if(r != 0) v=twmul<1>(v,P.twN[twExp(s,c,r,N)]);
+        }
+        return v;
+      };
+    };
+    runFusedFirst<T,WIDE>(x,0,1,P.fz,lt,tid,nthr,load);
+    const int nblk=runFusedMiddle<T,WIDE>(x,0,1,P.fz,lt,false,0,tid,nthr);
+    __syncthreads();
+    FGB_FUSED_SWITCH(P.fz.radix[P.fz.nst-1],
+                     (outerLastFwd<T,R_>(P,x,dst,col0,nblk,tid,nthr)))
   }
-  runFusedFirst<T,WIDE>(x,0,1,P.fz,lt,tid,nthr,load);
-  const int nblk=runFusedMiddle<T,WIDE>(x,0,1,P.fz,lt,false,0,tid,nthr);
-  __syncthreads();
-  FGB_FUSED_SWITCH(P.fz.radix[P.fz.nst-1],
-                   (outerLastFwd<T,R_>(P,x,dst,col0,nblk,tid,nthr)))
-}
-
-// Precisions whose outer launches may take the staged form (stagedColumns in
-// engine.cu).
-template<typename T> __host__ __device__ constexpr bool stagedOuterForm()
-{
-  return !std::is_same<T,double>::value;
 }
 
 template<typename T>
@@ -448,8 +447,7 @@ __global__ void __launch_bounds__(256)
 outerFwdFusedKernel(const OuterPlan<T> P)
 {
   extern __shared__ __align__(16) unsigned char smemRaw[];
-  outerFwdFused<T,false,stagedOuterForm<T>()>(P,blockIdx.x,blockIdx.y,
-                                              blockIdx.z,smemRaw);
+  outerFwdFused<T,false>(P,blockIdx.x,blockIdx.y,blockIdx.z,smemRaw);
 }
 
 // The first inverse stage: staging rows into shared memory.
@@ -485,7 +483,7 @@ __device__ __forceinline__ void outerFirstInv(const OuterPlan<T>& P,
 
 // All residues of a column tile; with several, a thread adds the outputs it
 // computes into its own entries of an accumulator behind the tile.
-template<typename T, bool WIDE, bool CG, bool STAGED>
+template<typename T, bool WIDE, bool CG, bool STAGED=false>
 __device__ __forceinline__ void outerBwdFused(const OuterPlan<T>& P, int ctile,
                                               int z, unsigned char *smemRaw)
 {
@@ -520,7 +518,7 @@ __device__ __forceinline__ void outerBwdFused(const OuterPlan<T>& P, int ctile,
         storeIO(f+s*P.outRow,v*P.scale,P.io64 & 2,sh);
       };
     };
-    if(STAGED && P.staged) {
+    if constexpr(STAGED) {
       loadTile(x,P.fz,lt,tid,nthr,[&](int cc, int j) {
           return col0+cc < P.C ? swapXY(sr[j*P.inRow+col0+cc]) :
             mk((T) 0,(T) 0);
@@ -543,8 +541,7 @@ __global__ void __launch_bounds__(256)
 outerBwdFusedKernel(const OuterPlan<T> P)
 {
   extern __shared__ __align__(16) unsigned char smemRaw[];
-  outerBwdFused<T,false,false,stagedOuterForm<T>()>(P,blockIdx.x,blockIdx.z,
-                                                    smemRaw);
+  outerBwdFused<T,false,false>(P,blockIdx.x,blockIdx.z,smemRaw);
 }
 
 // FP32 plans with a radix-16 stage: their own instantiations, capped at 85
@@ -555,7 +552,7 @@ __global__ void __launch_bounds__(256,3)
 outerFwdFusedKernel16(const OuterPlan<T> P)
 {
   extern __shared__ __align__(16) unsigned char smemRaw[];
-  outerFwdFused<T,true,true>(P,blockIdx.x,blockIdx.y,blockIdx.z,smemRaw);
+  outerFwdFused<T,true>(P,blockIdx.x,blockIdx.y,blockIdx.z,smemRaw);
 }
 
 template<typename T>
@@ -563,7 +560,29 @@ __global__ void __launch_bounds__(256,3)
 outerBwdFusedKernel16(const OuterPlan<T> P)
 {
   extern __shared__ __align__(16) unsigned char smemRaw[];
-  outerBwdFused<T,true,false,true>(P,blockIdx.x,blockIdx.z,smemRaw);
+  outerBwdFused<T,true,false>(P,blockIdx.x,blockIdx.z,smemRaw);
+}
+
+// The staged form (FP32: with radix 16), for small launches (stagedColumns in
+// engine.cu).  Kernels of their own: as a branch of the fused FP32 ones their
+// code cost those 4 to 10 % (2D 1023 x 512 modes, forward 22.8 -> 24.2 us,
+// backward 14.9 -> 16.7).
+template<typename T>
+__global__ void __launch_bounds__(256,stagedBlocks<T>())
+outerFwdStagedKernel(const OuterPlan<T> P)
+{
+  extern __shared__ __align__(16) unsigned char smemRaw[];
+  outerFwdFused<T,std::is_same<T,float>::value,true>(P,blockIdx.x,blockIdx.y,
+                                                     blockIdx.z,smemRaw);
+}
+
+template<typename T>
+__global__ void __launch_bounds__(256,stagedBlocks<T>())
+outerBwdStagedKernel(const OuterPlan<T> P)
+{
+  extern __shared__ __align__(16) unsigned char smemRaw[];
+  outerBwdFused<T,std::is_same<T,float>::value,false,true>(P,blockIdx.x,
+                                                           blockIdx.z,smemRaw);
 }
 
 // ---------------------------------------------------------------------------
@@ -675,7 +694,7 @@ __device__ __forceinline__ void realLastFwd(const OuterPlan<T>& P,
   }
 }
 
-template<typename T, bool WIDE>
+template<typename T, bool WIDE, bool STAGED>
 __device__ __forceinline__ void outerRealFwd(const OuterPlan<T>& P,
                                              unsigned char *smemRaw)
 {
@@ -689,18 +708,7 @@ __device__ __forceinline__ void outerRealFwd(const OuterPlan<T>& P,
   cplx<T> *dst=P.out[a]+batch*P.outBatch;
   const int lt=log2of(tile);
   const int sh=ioShift<T>(P.ioShift,a);
-  const auto load=[&](int, int cc) {
-    const int top=col0+cc < P.C ? L : 0;
-    const T *f=src+dataCol(P,col0+cc);
-    return [=,&P](int j) {
-      const int s=2*j;
-      cplx<T> v=mk((T) 0,(T) 0);
-      if(s < top) v.x=loadIOr(f+s*P.inRow,P.io64 & 1,sh);
-      if(s+1 < top) v.y=loadIOr(f+(s+1)*P.inRow,P.io64 & 1,sh);
-      return v;
-    };
-  };
-  if(!std::is_same<T,float>::value || P.staged) {
+  if constexpr(STAGED) {
     loadTile(x,P.fz,lt,tid,nthr,[&](int cc, int j) {
         const int s=2*j, top=col0+cc < P.C ? L : 0;
         const T *f=src+dataCol(P,col0+cc);
@@ -727,7 +735,18 @@ __device__ __forceinline__ void outerRealFwd(const OuterPlan<T>& P,
     }
     return;
   }
-  if constexpr(std::is_same<T,float>::value) {
+  if constexpr(!STAGED) {
+    const auto load=[&](int, int cc) {
+      const int top=col0+cc < P.C ? L : 0;
+      const T *f=src+dataCol(P,col0+cc);
+      return [=,&P](int j) {
+        const int s=2*j;
+        cplx<T> v=mk((T) 0,(T) 0);
+        if(s < top) v.x=loadIOr(f+s*P.inRow,P.io64 & 1,sh);
+        if(s+1 < top) v.y=loadIOr(f+(s+1)*P.inRow,P.io64 & 1,sh);
+        return v;
+      };
+    };
     runFusedFirst<T,WIDE>(x,0,1,P.fz,lt,tid,nthr,load);
     runFusedMiddle<T,WIDE>(x,0,1,P.fz,lt,false,0,tid,nthr);
     __syncthreads();
@@ -796,7 +815,7 @@ __device__ __forceinline__ void realFirstInv(const OuterPlan<T>& P,
   }
 }
 
-template<typename T, bool WIDE>
+template<typename T, bool WIDE, bool STAGED>
 __device__ __forceinline__ void outerRealBwd(const OuterPlan<T>& P,
                                              unsigned char *smemRaw)
 {
@@ -820,7 +839,7 @@ __device__ __forceinline__ void outerRealBwd(const OuterPlan<T>& P,
       if(s+1 < top) storeIOr(f+(s+1)*P.outRow,v.y,P.io64 & 2,sh);
     };
   };
-  if(!std::is_same<T,float>::value || P.staged) {
+  if constexpr(STAGED) {
     const int Nh=P.N/2, top=P.kc > 0 ? P.kc : Nh+1;
 #pragma unroll 2
     for(int idx=tid; idx < (Nh/2+1) << lt; idx += nthr) {
@@ -845,7 +864,7 @@ __device__ __forceinline__ void outerRealBwd(const OuterPlan<T>& P,
     storeTile(x,P.fz,lt,tid,nthr,store);
     return;
   }
-  if constexpr(std::is_same<T,float>::value) {
+  if constexpr(!STAGED) {
     FGB_FUSED_SWITCH(P.fz.radix[P.fz.nst-1],
                      (realFirstInv<T,R_>(P,x,src,col0,tid,nthr)))
     runFusedMiddle<T,WIDE>(x,0,1,P.fz,lt,true,0,tid,nthr);
@@ -854,20 +873,20 @@ __device__ __forceinline__ void outerRealBwd(const OuterPlan<T>& P,
   }
 }
 
-template<typename T, bool WIDE>
+template<typename T, bool WIDE, bool STAGED>
 __global__ void __launch_bounds__(256,2)
 outerRealFwdKernel(const OuterPlan<T> P)
 {
   extern __shared__ __align__(16) unsigned char smemRaw[];
-  outerRealFwd<T,WIDE>(P,smemRaw);
+  outerRealFwd<T,WIDE,STAGED>(P,smemRaw);
 }
 
-template<typename T, bool WIDE>
+template<typename T, bool WIDE, bool STAGED>
 __global__ void __launch_bounds__(256,2)
 outerRealBwdKernel(const OuterPlan<T> P)
 {
   extern __shared__ __align__(16) unsigned char smemRaw[];
-  outerRealBwd<T,WIDE>(P,smemRaw);
+  outerRealBwd<T,WIDE,STAGED>(P,smemRaw);
 }
 
 // ---------------------------------------------------------------------------
@@ -971,8 +990,8 @@ batchKernel(const BatchArgs<T> P)
         rebase(O,O.count,fwd && (rel & 4),!fwd && (rel & 8),P.inBase,
                P.outBase);
       __syncthreads();
-      if(fwd) outerFwdFused<T,false,false>(O,tk.i,0,tk.j,smemRaw);
-      else outerBwdFused<T,false,true,false>(O,tk.i,tk.j,smemRaw);
+      if(fwd) outerFwdFused<T,false>(O,tk.i,0,tk.j,smemRaw);
+      else outerBwdFused<T,false,true>(O,tk.i,tk.j,smemRaw);
       __syncthreads();
     }
     if(tk.type == TASK_COLFWD || tk.type == TASK_ROW) {
@@ -1115,6 +1134,8 @@ cudaError_t launchOuterFwd(const OuterPlan<T>& P, int threads, cudaStream_t s)
     return cudaGetLastError();
   };
   if(P.fused) {
+    if constexpr(!std::is_same<T,double>::value)
+      if(P.staged) return go(outerFwdStagedKernel<T>);
     if constexpr(std::is_same<T,float>::value)
       if(wideFused(P.fz)) return go(outerFwdFusedKernel16<T>);
     return go(outerFwdFusedKernel<T>);
@@ -1135,6 +1156,8 @@ cudaError_t launchOuterBwd(const OuterPlan<T>& P, int threads, cudaStream_t s)
     return cudaGetLastError();
   };
   if(P.fused) {
+    if constexpr(!std::is_same<T,double>::value)
+      if(P.staged) return go(outerBwdStagedKernel<T>);
     if constexpr(std::is_same<T,float>::value)
       if(wideFused(P.fz)) return go(outerBwdFusedKernel16<T>);
     return go(outerBwdFusedKernel<T>);
@@ -1155,11 +1178,16 @@ static cudaError_t launchOuterReal(const OuterPlan<T>& P, bool fwd,
     return cudaGetLastError();
   };
   if constexpr(std::is_same<T,float>::value)
-    if(wideFused(P.fz))
-      return fwd ? go(outerRealFwdKernel<T,true>) :
-        go(outerRealBwdKernel<T,true>);
-  return fwd ? go(outerRealFwdKernel<T,false>) :
-    go(outerRealBwdKernel<T,false>);
+    if(!P.staged) {
+      if(wideFused(P.fz))
+        return fwd ? go(outerRealFwdKernel<T,true,false>) :
+          go(outerRealBwdKernel<T,true,false>);
+      return fwd ? go(outerRealFwdKernel<T,false,false>) :
+        go(outerRealBwdKernel<T,false,false>);
+    }
+  constexpr bool wide=std::is_same<T,float>::value;
+  return fwd ? go(outerRealFwdKernel<T,wide,true>) :
+    go(outerRealBwdKernel<T,wide,true>);
 }
 
 template<typename T>

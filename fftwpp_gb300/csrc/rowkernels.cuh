@@ -1364,7 +1364,7 @@ hermRowPingPongKernel(const HermRowPlan<T> P, const Mul mul)
     default: break; \
   }
 
-template<typename T, class Mul, bool WIDE>
+template<typename T, class Mul, bool WIDE, bool STAGED>
 __device__ __forceinline__ void hermRows(const HermRowPlan<T>& P,
                                          const Mul& mul,
                                          unsigned char *smemRaw)
@@ -1373,14 +1373,13 @@ __device__ __forceinline__ void hermRows(const HermRowPlan<T>& P,
   const int team=threadIdx.x/nt, t=threadIdx.x-team*nt;
   const int cs=fusedSpan(P.Nh,P.fz.lg);
   cplx<T> *x=(cplx<T> *) smemRaw+team*P.A*cs;
-  const int R0=P.fz.radix[0];
   const long long groups=(P.nrows+P.rpc-1)/P.rpc;
   for(long long g=blockIdx.x; g < groups; g += gridDim.x)
     for(int rho=team; rho < P.rpc; rho += P.nteam) {
       const long long row=g*P.rpc+rho;
-      if(!std::is_same<T,float>::value || P.staged)
-        hermRowStaged<T,WIDE>(P,mul,x,cs,row,team,t,nt);
-      else if constexpr(std::is_same<T,float>::value) {
+      if constexpr(STAGED) hermRowStaged<T,WIDE>(P,mul,x,cs,row,team,t,nt);
+      else {
+        const int R0=P.fz.radix[0];
         FGB_HERM_SWITCH(R0,(hermFirst<T,R_>(P,x,cs,row,t,nt)))
         fusedRowInner<T,WIDE>(P,mul,x,cs,row,team,t,nt);
         FGB_HERM_SWITCH(R0,(hermLast<T,R_>(P,x,cs,row,t,nt)))
@@ -1391,19 +1390,19 @@ __device__ __forceinline__ void hermRows(const HermRowPlan<T>& P,
 
 template<typename T, class Mul>
 __global__ void __launch_bounds__(256,fusedBlocks<T>())
-hermRowKernel(const HermRowPlan<T> P, const Mul mul)
+hermRowStagedKernel(const HermRowPlan<T> P, const Mul mul)
 {
   extern __shared__ __align__(16) unsigned char smemRaw[];
-  hermRows<T,Mul,false>(P,mul,smemRaw);
+  hermRows<T,Mul,std::is_same<T,float>::value,true>(P,mul,smemRaw);
 }
 
-// FP32 plans with a radix-16 stage.
-template<typename T, class Mul>
+// FP32, fused; WIDE: plans with a radix-16 stage.
+template<typename T, class Mul, bool WIDE>
 __global__ void __launch_bounds__(256,fusedBlocks<T>())
-hermRowKernel16(const HermRowPlan<T> P, const Mul mul)
+hermRowFusedKernel(const HermRowPlan<T> P, const Mul mul)
 {
   extern __shared__ __align__(16) unsigned char smemRaw[];
-  hermRows<T,Mul,true>(P,mul,smemRaw);
+  hermRows<T,Mul,WIDE,false>(P,mul,smemRaw);
 }
 
 // ---------------------------------------------------------------------------
@@ -1461,11 +1460,13 @@ cudaError_t launchHermRowWith(const HermRowPlan<T>& P, const Mul& mul,
     kernel<<<(unsigned) grid,threads,sm,s>>>(P,mul);
     return cudaGetLastError();
   };
-  if constexpr(std::is_same<T,float>::value)
-    if(wideFused(P.fz)) return go(hermRowKernel16<T,Mul>);
   if constexpr(std::is_same<T,double>::value)
     if(P.pingpong) return go(hermRowPingPongKernel<T,Mul>);
-  return go(hermRowKernel<T,Mul>);
+  if constexpr(std::is_same<T,float>::value)
+    if(!P.staged)
+      return wideFused(P.fz) ? go(hermRowFusedKernel<T,Mul,true>) :
+        go(hermRowFusedKernel<T,Mul,false>);
+  return go(hermRowStagedKernel<T,Mul>);
 }
 
 } // namespace fgb
