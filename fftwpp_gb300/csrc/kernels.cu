@@ -297,12 +297,6 @@ outerBwdKernel(const OuterPlan<T> P)
 // row order and the backward undoes it).  The column tile's values cross
 // shared memory once between stages and never before the first or after
 // the last.
-// CTAs of 256 threads per SM of the staged kernels (radix 16 in FP32).
-template<typename T> __host__ __device__ constexpr int stagedBlocks()
-{
-  return std::is_same<T,float>::value ? 3 : 1;
-}
-
 // The staged form (runStages): the tile's inputs into shared memory, and its
 // outputs out of it.  in(cc, j) gives element j of column cc.
 template<typename T, class In>
@@ -568,7 +562,7 @@ outerBwdFusedKernel16(const OuterPlan<T> P)
 // code cost those 4 to 10 % (2D 1023 x 512 modes, forward 22.8 -> 24.2 us,
 // backward 14.9 -> 16.7).
 template<typename T>
-__global__ void __launch_bounds__(256,stagedBlocks<T>())
+__global__ void __launch_bounds__(256,3)
 outerFwdStagedKernel(const OuterPlan<T> P)
 {
   extern __shared__ __align__(16) unsigned char smemRaw[];
@@ -577,7 +571,7 @@ outerFwdStagedKernel(const OuterPlan<T> P)
 }
 
 template<typename T>
-__global__ void __launch_bounds__(256,stagedBlocks<T>())
+__global__ void __launch_bounds__(256,3)
 outerBwdStagedKernel(const OuterPlan<T> P)
 {
   extern __shared__ __align__(16) unsigned char smemRaw[];
